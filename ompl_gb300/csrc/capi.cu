@@ -271,6 +271,7 @@ struct gbo_nn
     int F = 0;
     double *pts64 = nullptr;
     float *feat32 = nullptr;
+    float4 *feat4 = nullptr;
     unsigned char *alive = nullptr;
     float eps32 = 0.f;
     NNBoxCells cells;
@@ -291,6 +292,8 @@ struct gbo_nn
             cudaFree(pts64);
         if (feat32)
             cudaFree(feat32);
+        if (feat4)
+            cudaFree(feat4);
         if (alive)
             cudaFree(alive);
     }
@@ -1554,6 +1557,7 @@ gbo_status gbo_nn_create(const gbo_space *space, int64_t capacity, gbo_nn **out)
     nn->eps32 = space->sp.kind == GBO_SPACE_KINEMATIC_CHAIN ? chain_knn_eps(space->sp) : box_knn_eps(space->sp);
     if (cudaMalloc(&nn->pts64, sizeof(double) * space->sp.dim * capacity) != cudaSuccess ||
         cudaMalloc(&nn->feat32, sizeof(float) * nn->F * capacity) != cudaSuccess ||
+        cudaMalloc(&nn->feat4, sizeof(float4) * ((nn->F + 3) / 4) * capacity) != cudaSuccess ||
         cudaMalloc(&nn->alive, capacity) != cudaSuccess || nn->ctr.init() != GBO_OK)
     {
         delete nn;
@@ -1598,7 +1602,7 @@ gbo_status gbo_nn_add(gbo_nn *nn, const double *states, int64_t n, int64_t ld, i
     StatesView v = make_view(states, ld, layout);
     launch_store_points(lc, v, n, nn->sp.dim, nn->pts64, nn->cap, nn->size, nn->alive);
     // features of the new elements, written at column offset `size` of the [F][cap] array
-    launch_features(lc, nn->sp, v, n, nn->feat32 + nn->size, nn->cap);
+    launch_features(lc, nn->sp, v, n, nn->feat32 + nn->size, nn->cap, nn->feat4 + nn->size);
     CHECK_LAUNCH();
     nn->size += n;
     nn->alive_count += n;
@@ -1657,6 +1661,7 @@ static NNArgs nn_args(const gbo_nn *nn)
     NNArgs a;
     a.pts64 = nn->pts64;
     a.feat32 = nn->feat32;
+    a.feat4 = nn->feat4;
     a.alive = nn->alive;
     a.cap = nn->cap;
     a.size = nn->size;
@@ -1729,24 +1734,46 @@ gbo_status gbo_nn_nearest_k(gbo_nn *nn, const double *q, int64_t nq, int64_t ld,
     nn->queries += nq;
     if (nn->precision == GBO_PRECISION_FP32_GUARDED && k <= knn_fp32_max_k(nn->sp))
     {
-        if (auto st = nn->qfeat.reserve(sizeof(float) * nn->F * nq, lc.stream))
-            return st;
         if (auto st = nn->fb_list.reserve(sizeof(unsigned long long) * nq, lc.stream))
             return st;
         unsigned long long *fb_n = &ctr->queue;
+        // The cell searches take batches large enough to win over reading every element: their fixed cost
+        // (query order, one search per warp) is 0.2 to 0.6 ms. Measured (cells / group kernel): planar,
+        // 200,000 elements, 1,000 queries 184 / 152 us, 4,096 queries 264 / 490 us; wrapped 7-D, 200,000
+        // elements, 1,000 queries 651 / 432 us, 4,096 queries 646 / 1,586 us; 1M elements, 500 queries
+        // 795 / 952 us; chain, 200,000 elements, 4,096 queries 2.37 / 2.58 ms.
+        const bool chain = nn->sp.kind == GBO_SPACE_KINEMATIC_CHAIN;
+        const bool cells = nn->size >= 65536 && nn->size < (1ll << 31) && nq >= (chain ? 1024 : 256) &&
+                           nq * nn->size >= (chain ? 800000000ll : 400000000ll) && !(chain && prefix);
+        // a huge batch over a tiny index: thread per query (100 elements, 20,000 queries: 148 us against
+        // 186 us wrapped, 0.62 ms against 0.91 ms on the chain)
+        const bool tiny = nq >= 16384 && nn->size <= 256;
+        if (!cells && !tiny)
+        {
+            NNArgs g = a;
+            if (nn->alive_count == nn->size)
+                g.alive = nullptr;
+            if (launch_knn_group(lc, g, nn->sp, qv, nq, k, prefix, idx, dist, (unsigned long long *)nn->fb_list.p,
+                                 fb_n, ctr))
+            {
+                launch_knn_exact(lc, a, nn->sp, qv, nq, k, prefix, idx, dist,
+                                 (const unsigned long long *)nn->fb_list.p, fb_n, std::min<int64_t>(nq, 4096));
+                CHECK_LAUNCH();
+                return GBO_OK;
+            }
+        }
+        if (auto st = nn->qfeat.reserve(sizeof(float) * nn->F * nq, lc.stream))
+            return st;
         const int P = knn_chunks(lc, nq, nn->size);
         const int keep = knn_keep(k);
         const size_t pl = (size_t)P * nq * keep;
-        if (auto st = nn->part.reserve(pl * (sizeof(float) + sizeof(int64_t)) + (size_t)nq * sizeof(unsigned) + 64,
-                                       lc.stream))
+        if (auto st = nn->part.reserve(pl * (sizeof(float) + sizeof(int64_t)) + 64, lc.stream))
             return st;
         int64_t *part_k = (int64_t *)nn->part.p;
         float *part_d = (float *)(part_k + pl);
-        unsigned *thr = (unsigned *)(part_d + pl);  // per-query bound shared by the chunks of the FP32 scan
         launch_features(lc, nn->sp, qv, nq, (float *)nn->qfeat.p, nq);
         // large batches over a large RealVector / wrapped index: cell index (PRM's prefix kNN)
-        if ((nn->sp.kind == GBO_SPACE_WRAP_L2 || nn->sp.kind == GBO_SPACE_REAL_VECTOR) && nn->sp.dim <= 8 &&
-            nn->size >= 65536 && nn->size < (1ll << 31) && nq >= 256)
+        if (cells && (nn->sp.kind == GBO_SPACE_WRAP_L2 || nn->sp.kind == GBO_SPACE_REAL_VECTOR) && nn->sp.dim <= 8)
         {
             if (auto st = ensure_box_cells(nn, lc))
                 return st;
@@ -1774,10 +1801,8 @@ gbo_status gbo_nn_nearest_k(gbo_nn *nn, const double *q, int64_t nq, int64_t ld,
                 return GBO_OK;
             }
         }
-        // large batches without prefix limits run in spatial order (the lanes of a warp then prune the
-        // same elements); with PRM prefix limits the given order keeps each CTA's scan range short
-        const int64_t *order = nullptr;
-        if (!prefix && nq >= 1024)
+        // a large chain index: the cell search, one warp per query (the query order's keys are the cells)
+        if (cells && chain && nn->sp.dim <= 10 && k <= 20)
         {
             const size_t wb = ((size_t)3 * kQueryKeys + nq) * sizeof(int);
             if (auto st = nn->qorder.reserve(wb + (size_t)nq * sizeof(int64_t) + 16, lc.stream))
@@ -1785,31 +1810,23 @@ gbo_status gbo_nn_nearest_k(gbo_nn *nn, const double *q, int64_t nq, int64_t ld,
             int *work = (int *)nn->qorder.p;
             int64_t *ord = (int64_t *)((char *)nn->qorder.p + pad16(wb));
             launch_query_order(lc, nn->sp, (const float *)nn->qfeat.p, nq, work, ord);
-            order = ord;
-            // a large chain index: the cell search, one warp per query (the query order's keys are the
-            // cells)
-            if (nn->sp.kind == GBO_SPACE_KINEMATIC_CHAIN && nn->sp.dim <= 10 && k <= 20 && nn->size >= 65536 &&
-                nn->size < (1ll << 31))
+            if (auto st = ensure_chain_cells(nn, lc))
+                return st;
+            NNChainCells &c = nn->ccells;
+            const ChainCellArgs ci{(const int *)c.start.p,  (const int *)c.count.p, (const int64_t *)c.skey.p,
+                                   (const float4 *)c.sfeat.p, nn->size,  (const uint4 *)c.box.p,
+                                   (const int *)c.cstart.p,   (const uint4 *)c.cbox.p};
+            if (launch_knn_ccell(lc, a, ci, nn->sp, qv, (const float *)nn->qfeat.p, nq, ord, work + 3 * kQueryKeys, k,
+                                 idx, dist, (unsigned long long *)nn->fb_list.p, fb_n, ctr, part_d, part_k))
             {
-                if (auto st = ensure_chain_cells(nn, lc))
-                    return st;
-                NNChainCells &c = nn->ccells;
-                const ChainCellArgs ci{(const int *)c.start.p,  (const int *)c.count.p, (const int64_t *)c.skey.p,
-                                       (const float4 *)c.sfeat.p, nn->size,  (const uint4 *)c.box.p,
-                                       (const int *)c.cstart.p,   (const uint4 *)c.cbox.p};
-                if (launch_knn_ccell(lc, a, ci, nn->sp, qv, (const float *)nn->qfeat.p, nq, ord,
-                                     work + 3 * kQueryKeys, k, idx, dist, (unsigned long long *)nn->fb_list.p, fb_n,
-                                     ctr, part_d, part_k))
-                {
-                    launch_knn_exact(lc, a, nn->sp, qv, nq, k, prefix, idx, dist,
-                                     (const unsigned long long *)nn->fb_list.p, fb_n, std::min<int64_t>(nq, 4096));
-                    CHECK_LAUNCH();
-                    return GBO_OK;
-                }
+                launch_knn_exact(lc, a, nn->sp, qv, nq, k, prefix, idx, dist,
+                                 (const unsigned long long *)nn->fb_list.p, fb_n, std::min<int64_t>(nq, 4096));
+                CHECK_LAUNCH();
+                return GBO_OK;
             }
         }
         if (launch_knn_fp32(lc, a, nn->sp, qv, (const float *)nn->qfeat.p, nq, k, prefix, idx, dist,
-                            (unsigned long long *)nn->fb_list.p, fb_n, ctr, part_d, part_k, P, order, thr))
+                            (unsigned long long *)nn->fb_list.p, fb_n, ctr, part_d, part_k, P))
         {
             // queries whose FP32 band overflowed: exact FP64 scan (count read on the device)
             launch_knn_exact(lc, a, nn->sp, qv, nq, k, prefix, idx, dist, (const unsigned long long *)nn->fb_list.p,

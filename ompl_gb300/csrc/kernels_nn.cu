@@ -22,26 +22,10 @@
 
 #include <cuda_fp16.h>
 
-#include "kernels_nn.cuh"
+#include "nn_device.cuh"
 
 namespace gbo
 {
-
-template <int MAXD>
-__device__ __forceinline__ void load_point(const double *pts, int64_t cap, int dim, int64_t key, double *x)
-{
-#pragma unroll
-    for (int d = 0; d < MAXD; ++d)
-        x[d] = d < dim ? pts[(int64_t)d * cap + key] : 0.0;
-}
-
-template <int MAXD>
-__device__ __forceinline__ void load_query(const StatesView &v, int64_t i, int dim, double *x)
-{
-#pragma unroll
-    for (int d = 0; d < MAXD; ++d)
-        x[d] = d < dim ? v(i, d) : 0.0;
-}
 
 // Insert (d, key) into an ascending register list; equal distances keep the earlier entry first.
 template <int K, class T, class I>
@@ -63,11 +47,6 @@ __device__ __forceinline__ void topk_insert(T *dk, I *ik, T d, I key)
             ik[j] = key;
         }
     }
-}
-
-__device__ __forceinline__ bool less_dk(double a, int64_t ka, double b, int64_t kb)
-{
-    return a < b || (a == b && ka < kb);
 }
 
 template <int K, int MAXD>
@@ -154,28 +133,6 @@ __global__ void __launch_bounds__(256) knn_exact_kernel(NNArgs nn, SpaceParams s
 
 // ---------------------------------------------------------------- FP32 scan
 
-// Element features: REAL_VECTOR / WRAP_L2 / SO2: the coordinates (F = dim); KINEMATIC_CHAIN: the
-// cumulative link-direction sums interleaved (X_1, Y_1, ..., X_n, Y_n), F = 2 dim, so that
-// distance = L * sum_i |(X_i(a) - X_i(b), Y_i(a) - Y_i(b))|. All indices below are compile-time.
-template <int KIND, int MAXF>
-__device__ __forceinline__ float box_dist2(const float *a, const float *b, int dim)
-{
-    float s = 0.f;
-#pragma unroll
-    for (int i = 0; i < MAXF; ++i)
-        if (i < dim)
-        {
-            float d = a[i] - b[i];
-            if constexpr (KIND == GBO_SPACE_WRAP_L2 || KIND == GBO_SPACE_SO2)
-            {
-                d = fabsf(d);
-                d = fminf(d, 6.28318530717958647692f - d);
-            }
-            s = fmaf(d, d, s);
-        }
-    return s;
-}
-
 // Partial L1 lower bound over links [i0, i1): sum (|dx_i| + |dy_i|) <= sqrt(2) * sum |(dx_i, dy_i)|.
 template <int MAXF>
 __device__ __forceinline__ float chain_l1(const float *a, const float *b, int dim, int i0, int i1)
@@ -188,43 +145,17 @@ __device__ __forceinline__ float chain_l1(const float *a, const float *b, int di
     return l1;
 }
 
-__device__ __forceinline__ float sqrt_approx(float x)
-{
-    float r;
-    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
-}
-
-template <int MAXF>
-__device__ __forceinline__ float chain_dist32(const float *a, const float *b, int dim)
-{
-    float s = 0.f;
-#pragma unroll
-    for (int i = 0; i < MAXF / 2; ++i)
-        if (i < dim)
-        {
-            const float dx = a[2 * i] - b[2 * i], dy = a[2 * i + 1] - b[2 * i + 1];
-            s += sqrt_approx(fmaf(dx, dx, dy * dy));
-        }
-    return s;
-}
-
 // Partial scan: CTA (x = block of 128 queries, y = chunk of elements). Each thread keeps the K_KEEP
 // smallest FP32 distances (squared for box/wrapped kinds) of its query within the chunk. qorder
 // (nullable): thread qs takes query qorder[qs] (queries in spatial order, so that the lanes of a warp
 // prune the same elements); its list is kept at position qs.
 // qkey (nullable): only the queries with qkey < key_limit are this launch's (the others' lists are
 // written by the cell kernel).
-// thr (nullable): per query position, the smallest K_KEEP-th distance any chunk has reached so far
-// (float bits; non-negative floats order like their bits). Every chunk's list is an upper bound on the
-// query's K_KEEP-th smallest distance, so each CTA prunes against the smallest one published, reading
-// and publishing it once per tile. An element dropped that way is beyond the merged list's last entry,
-// which the finish kernel's overflow test already treats as possibly dropped.
 template <int KIND, int MAXF, int K_KEEP>
 __global__ void __launch_bounds__(128) knn_scan_kernel(NNArgs nn, SpaceParams sp, const float *qf, int64_t nq,
                                                        const int64_t *prefix, int64_t chunk, float *part_d,
                                                        int64_t *part_k, const int64_t *qorder, const int *qkey,
-                                                       int key_limit, unsigned *thr)
+                                                       int key_limit)
 {
     constexpr int TILE = 128;
     constexpr int FP = (MAXF + 3) / 4 * 4;
@@ -261,7 +192,6 @@ __global__ void __launch_bounds__(128) knn_scan_kernel(NNArgs nn, SpaceParams sp
         ik[j] = -1;
     }
     const float lscale = KIND == GBO_SPACE_KINEMATIC_CHAIN ? 0.70710678f * (1.0f - 1e-5f) * (float)sp.link : 1.0f;
-    float g = __int_as_float(0x7f800000);  // the shared bound last read
     for (int64_t base = c0; base < block_end; base += TILE)
     {
         __syncthreads();
@@ -276,9 +206,7 @@ __global__ void __launch_bounds__(128) knn_scan_kernel(NNArgs nn, SpaceParams sp
         __syncthreads();
         if (!active)
             continue;
-        if (thr)
-            g = __uint_as_float(__ldcg(thr + qs));
-        float cut = fminf(dk[K_KEEP - 1], g);
+        float cut = dk[K_KEEP - 1];
         const int tn = (int)max((int64_t)0, min((int64_t)TILE, limit - base));
         for (int t = 0; t < tn; ++t)
         {
@@ -312,11 +240,9 @@ __global__ void __launch_bounds__(128) knn_scan_kernel(NNArgs nn, SpaceParams sp
             if (d < cut)
             {
                 topk_insert<K_KEEP>(dk, ik, d, (int)(base + t));
-                cut = fminf(cut, dk[K_KEEP - 1]);
+                cut = dk[K_KEEP - 1];
             }
         }
-        if (thr && dk[K_KEEP - 1] < g)
-            atomicMin(thr + qs, __float_as_uint(dk[K_KEEP - 1]));
     }
     if (!active)
         return;
@@ -441,11 +367,22 @@ __global__ void __launch_bounds__(128) knn_finish_kernel(NNArgs nn, SpaceParams 
 
 // ---------------------------------------------------------------- features
 template <int MAXD>
-__global__ void features_kernel(SpaceParams sp, StatesView v, int64_t n, float *out, int64_t ld_out)
+__global__ void features_kernel(SpaceParams sp, StatesView v, int64_t n, float *out, int64_t ld_out, float4 *out4)
 {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n)
         return;
+    float4 w = make_float4(0.f, 0.f, 0.f, 0.f);  // the plane being filled
+    int f = 0;
+    auto put = [&](float x) {
+        out[(int64_t)f * ld_out + i] = x;
+        (&w.x)[f & 3] = x;
+        if ((++f & 3) == 0 && out4)
+        {
+            out4[(int64_t)(f / 4 - 1) * ld_out + i] = w;
+            w = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    };
     if (sp.kind == GBO_SPACE_KINEMATIC_CHAIN)
     {
         double theta = 0.;
@@ -457,15 +394,17 @@ __global__ void features_kernel(SpaceParams sp, StatesView v, int64_t n, float *
             dir32(theta, c, s);
             X += c;
             Y += s;
-            out[(int64_t)(2 * d) * ld_out + i] = X;
-            out[(int64_t)(2 * d + 1) * ld_out + i] = Y;
+            put(X);
+            put(Y);
         }
     }
     else
     {
         for (int d = 0; d < sp.dim; ++d)
-            out[(int64_t)d * ld_out + i] = (float)v(i, d);
+            put((float)v(i, d));
     }
+    if ((f & 3) && out4)
+        out4[(int64_t)(f / 4) * ld_out + i] = w;
 }
 
 template <int MAXD>
@@ -659,16 +598,13 @@ template <int KIND, int MAXD, int MAXF, int K_KEEP>
 static void launch_fp32_t(const LaunchCfg &lc, const NNArgs &nn, const SpaceParams &sp, StatesView qv, const float *qf,
                           int64_t nq, int k, const int64_t *prefix, int64_t *idx, double *dist,
                           unsigned long long *fb_list, unsigned long long *fb_n, RunCounters *ctr, float *part_d,
-                          int64_t *part_k, int P, int64_t chunk, const int64_t *qorder, unsigned *thr)
+                          int64_t *part_k, int P, int64_t chunk)
 {
     const int qb = (int)((nq + 127) / 128);
-    if (thr && P > 1)
-        cudaMemsetAsync(thr, 0x7f, (size_t)nq * sizeof(unsigned), lc.stream);  // 3.4e38: no bound yet
     knn_scan_kernel<KIND, MAXF, K_KEEP><<<dim3(qb, P), 128, 0, lc.stream>>>(nn, sp, qf, nq, prefix, chunk, part_d,
-                                                                           part_k, qorder, nullptr, 0,
-                                                                           P > 1 ? thr : nullptr);
+                                                                           part_k, nullptr, nullptr, 0);
     knn_finish_kernel<KIND, MAXD, K_KEEP><<<qb, 128, 0, lc.stream>>>(nn, sp, qv, nq, k, P, part_d, part_k, idx, dist,
-                                                                    fb_list, fb_n, ctr, qorder);
+                                                                    fb_list, fb_n, ctr, nullptr);
     note_launch();
     note_launch();
 }
@@ -693,15 +629,14 @@ int knn_chunks(const LaunchCfg &lc, int64_t nq, int64_t size)
 
 bool launch_knn_fp32(const LaunchCfg &lc, const NNArgs &nn, const SpaceParams &sp, StatesView qv, const float *qf,
                      int64_t nq, int k, const int64_t *prefix, int64_t *idx, double *dist, unsigned long long *fb_list,
-                     unsigned long long *fb_n, RunCounters *ctr, float *part_d, int64_t *part_k, int P,
-                     const int64_t *qorder, unsigned *thr)
+                     unsigned long long *fb_n, RunCounters *ctr, float *part_d, int64_t *part_k, int P)
 {
     if (nq == 0 || k > knn_fp32_max_k(sp))
         return false;
     const int64_t chunk = (nn.size + P - 1) / P;
 #define GBO_FP32(KIND, MAXD, MAXF, KK)                                                                                 \
     launch_fp32_t<KIND, MAXD, MAXF, KK>(lc, nn, sp, qv, qf, nq, k, prefix, idx, dist, fb_list, fb_n, ctr, part_d,     \
-                                        part_k, P, chunk, qorder, thr)
+                                        part_k, P, chunk)
 #define GBO_FP32_K(KIND, MAXD, MAXF)                                                                                   \
     do                                                                                                                \
     {                                                                                                                 \
@@ -732,11 +667,12 @@ bool launch_knn_fp32(const LaunchCfg &lc, const NNArgs &nn, const SpaceParams &s
     return true;
 }
 
-void launch_features(const LaunchCfg &lc, const SpaceParams &sp, StatesView v, int64_t n, float *out, int64_t ld_out)
+void launch_features(const LaunchCfg &lc, const SpaceParams &sp, StatesView v, int64_t n, float *out, int64_t ld_out,
+                     float4 *out4)
 {
     if (n == 0)
         return;
-    features_kernel<GBO_MAXD><<<(int)((n + 255) / 256), 256, 0, lc.stream>>>(sp, v, n, out, ld_out);
+    features_kernel<GBO_MAXD><<<(int)((n + 255) / 256), 256, 0, lc.stream>>>(sp, v, n, out, ld_out, out4);
     note_launch();
 }
 
@@ -1321,7 +1257,7 @@ static void launch_bcell_t(const LaunchCfg &lc, const NNArgs &nn, const BoxCellA
         // band 0 (limits below a quarter of the index) through the prefix scan, same P lists
         knn_scan_kernel<KIND, 8, K_KEEP><<<dim3(qb, P), 128, 0, lc.stream>>>(nn, sp, qf, nq, prefix,
                                                                             (nn.size + P - 1) / P, part_d, part_k,
-                                                                            qorder, qcell, ci.C, nullptr);
+                                                                            qorder, qcell, ci.C);
         note_launch();
     }
     knn_finish_kernel<KIND, 8, K_KEEP><<<qb, 128, 0, lc.stream>>>(nn, sp, qv, nq, k, P, part_d, part_k, idx, dist,

@@ -9,6 +9,7 @@ struct NNArgs
 {
     const double *pts64;        // SoA FP64 elements [dim][cap]
     const float *feat32;        // SoA FP32 features [F][cap]
+    const float4 *feat4;        // the same features, four to a float4: planes [(F + 3) / 4][cap], unused ones 0
     const unsigned char *alive; // 1 = present, 0 = removed (tombstone)
     int64_t cap;
     int64_t size;               // keys handed out so far (removed ones included)
@@ -23,8 +24,12 @@ void launch_knn_exact(const LaunchCfg &lc, const NNArgs &nn, const SpaceParams &
                       const unsigned long long *list_n, int64_t max_items);
 bool launch_knn_fp32(const LaunchCfg &lc, const NNArgs &nn, const SpaceParams &sp, StatesView qv, const float *qf,
                      int64_t nq, int k, const int64_t *prefix, int64_t *idx, double *dist, unsigned long long *fb_list,
-                     unsigned long long *fb_n, RunCounters *ctr, float *part_d, int64_t *part_k, int P,
-                     const int64_t *qorder, unsigned *thr);
+                     unsigned long long *fb_n, RunCounters *ctr, float *part_d, int64_t *part_k, int P);
+// nearestK in one launch (kernels_nn_group.cu): no query features, partial lists or order; nn.alive may be
+// null (every element present). False when the space or k has no FP32 form.
+bool launch_knn_group(const LaunchCfg &lc, const NNArgs &nn, const SpaceParams &sp, StatesView qv, int64_t nq, int k,
+                      const int64_t *prefix, int64_t *idx, double *dist, unsigned long long *fb_list,
+                      unsigned long long *fb_n, RunCounters *ctr);
 // Cell index of a RealVector / wrapped nearest-neighbour index (large batches, PRM prefix kNN).
 struct BoxCellArgs
 {
@@ -79,7 +84,9 @@ int knn_chunks(const LaunchCfg &lc, int64_t nq, int64_t size);
 // and other kinds use the FP64 scan) and the list length they keep per query and chunk
 int knn_fp32_max_k(const SpaceParams &sp);
 int knn_keep(int k);
-void launch_features(const LaunchCfg &lc, const SpaceParams &sp, StatesView v, int64_t n, float *out, int64_t ld_out);
+// features of n states into out[F][ld_out] and, where out4 is given, its float4 planes (same row stride)
+void launch_features(const LaunchCfg &lc, const SpaceParams &sp, StatesView v, int64_t n, float *out, int64_t ld_out,
+                     float4 *out4 = nullptr);
 void launch_store_points(const LaunchCfg &lc, StatesView v, int64_t n, int dim, double *pts, int64_t cap,
                          int64_t first, unsigned char *alive);
 void launch_remove(const LaunchCfg &lc, const int64_t *keys, int64_t n, int64_t size, unsigned char *alive);
