@@ -272,6 +272,7 @@ struct gbo_nn
     double *pts64 = nullptr;
     float *feat32 = nullptr;
     float4 *feat4 = nullptr;
+    int *outside = nullptr;  // device flag: an element lies outside the bounds eps32 was derived for
     unsigned char *alive = nullptr;
     float eps32 = 0.f;
     NNBoxCells cells;
@@ -294,6 +295,8 @@ struct gbo_nn
             cudaFree(feat32);
         if (feat4)
             cudaFree(feat4);
+        if (outside)
+            cudaFree(outside);
         if (alive)
             cudaFree(alive);
     }
@@ -1558,12 +1561,14 @@ gbo_status gbo_nn_create(const gbo_space *space, int64_t capacity, gbo_nn **out)
     if (cudaMalloc(&nn->pts64, sizeof(double) * space->sp.dim * capacity) != cudaSuccess ||
         cudaMalloc(&nn->feat32, sizeof(float) * nn->F * capacity) != cudaSuccess ||
         cudaMalloc(&nn->feat4, sizeof(float4) * ((nn->F + 3) / 4) * capacity) != cudaSuccess ||
+        cudaMalloc(&nn->outside, sizeof(int)) != cudaSuccess ||
         cudaMalloc(&nn->alive, capacity) != cudaSuccess || nn->ctr.init() != GBO_OK)
     {
         delete nn;
         return fail(GBO_ERR_OUT_OF_MEMORY, "nearest-neighbour index allocation failed");
     }
     cudaMemset(nn->alive, 0, capacity);
+    cudaMemset(nn->outside, 0, sizeof(int));
     if (cudaStreamCreateWithFlags(&nn->host_stream, cudaStreamNonBlocking) != cudaSuccess)
     {
         delete nn;
@@ -1600,7 +1605,7 @@ gbo_status gbo_nn_add(gbo_nn *nn, const double *states, int64_t n, int64_t ld, i
         *first_key = nn->size;
     LaunchCfg lc = lcfg(stream);
     StatesView v = make_view(states, ld, layout);
-    launch_store_points(lc, v, n, nn->sp.dim, nn->pts64, nn->cap, nn->size, nn->alive);
+    launch_store_points(lc, nn->sp, v, n, nn->pts64, nn->cap, nn->size, nn->alive, nn->outside);
     // features of the new elements, written at column offset `size` of the [F][cap] array
     launch_features(lc, nn->sp, v, n, nn->feat32 + nn->size, nn->cap, nn->feat4 + nn->size);
     CHECK_LAUNCH();
@@ -1629,6 +1634,7 @@ gbo_status gbo_nn_clear(gbo_nn *nn)
         return fail(GBO_ERR_INVALID_ARGUMENT, "nn is NULL");
     CUDA_TRY(cudaDeviceSynchronize());
     CUDA_TRY(cudaMemset(nn->alive, 0, nn->cap));
+    CUDA_TRY(cudaMemset(nn->outside, 0, sizeof(int)));
     nn->size = 0;
     nn->alive_count = 0;
     nn->cells.valid = false;
@@ -1840,13 +1846,25 @@ gbo_status gbo_nn_nearest_k(gbo_nn *nn, const double *q, int64_t nq, int64_t ld,
     return GBO_OK;
 }
 
+// counts, or with offsets the filled and sorted segments
+static void radius_call(gbo_nn *nn, StatesView qv, int64_t nq, double r, int64_t *counts, const int64_t *offsets,
+                        int64_t *idx, double *dist, gbo_stream stream)
+{
+    NNArgs a = nn_args(nn);
+    if (nn->alive_count == nn->size)
+        a.alive = nullptr;
+    if (nn->precision == GBO_PRECISION_FP32_GUARDED &&
+        launch_radius_group(lcfg(stream), a, nn->sp, qv, nq, r, nn->outside, counts, offsets, idx, dist))
+        return;
+    launch_radius(lcfg(stream), nn_args(nn), nn->sp, qv, nq, r, counts, offsets, idx, dist);
+}
+
 gbo_status gbo_nn_nearest_r_count(gbo_nn *nn, const double *q, int64_t nq, int64_t ld, int layout, double r,
                                   int64_t *counts, gbo_stream stream)
 {
     if (!nn || nq < 0 || (nq > 0 && (!q || !counts)) || !valid_layout(layout, nq, ld, nn->sp.dim))
         return fail(GBO_ERR_INVALID_ARGUMENT, "bad nearestR arguments");
-    launch_radius(lcfg(stream), nn_args(nn), nn->sp, make_view(q, ld, layout), nq, r, counts, nullptr, nullptr,
-                  nullptr);
+    radius_call(nn, make_view(q, ld, layout), nq, r, counts, nullptr, nullptr, nullptr, stream);
     CHECK_LAUNCH();
     return GBO_OK;
 }
@@ -1856,7 +1874,7 @@ gbo_status gbo_nn_nearest_r_fill(gbo_nn *nn, const double *q, int64_t nq, int64_
 {
     if (!nn || nq < 0 || (nq > 0 && (!q || !offsets || !idx || !dist)) || !valid_layout(layout, nq, ld, nn->sp.dim))
         return fail(GBO_ERR_INVALID_ARGUMENT, "bad nearestR arguments");
-    launch_radius(lcfg(stream), nn_args(nn), nn->sp, make_view(q, ld, layout), nq, r, nullptr, offsets, idx, dist);
+    radius_call(nn, make_view(q, ld, layout), nq, r, nullptr, offsets, idx, dist, stream);
     CHECK_LAUNCH();
     return GBO_OK;
 }

@@ -408,14 +408,21 @@ __global__ void features_kernel(SpaceParams sp, StatesView v, int64_t n, float *
 }
 
 template <int MAXD>
-__global__ void store_points_kernel(StatesView v, int64_t n, int dim, double *pts, int64_t cap, int64_t first,
-                                    unsigned char *alive)
+__global__ void store_points_kernel(SpaceParams sp, StatesView v, int64_t n, double *pts, int64_t cap, int64_t first,
+                                    unsigned char *alive, int *outside)
 {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n)
         return;
-    for (int d = 0; d < dim; ++d)
-        pts[(int64_t)d * cap + first + i] = v(i, d);
+    bool in = true;
+    for (int d = 0; d < sp.dim; ++d)
+    {
+        const double x = v(i, d);
+        pts[(int64_t)d * cap + first + i] = x;
+        in &= x >= sp.low[d] && x <= sp.high[d];
+    }
+    if (!in)
+        *outside = 1;
     alive[first + i] = 1;
 }
 
@@ -676,12 +683,13 @@ void launch_features(const LaunchCfg &lc, const SpaceParams &sp, StatesView v, i
     note_launch();
 }
 
-void launch_store_points(const LaunchCfg &lc, StatesView v, int64_t n, int dim, double *pts, int64_t cap,
-                         int64_t first, unsigned char *alive)
+void launch_store_points(const LaunchCfg &lc, const SpaceParams &sp, StatesView v, int64_t n, double *pts, int64_t cap,
+                         int64_t first, unsigned char *alive, int *outside)
 {
     if (n == 0)
         return;
-    store_points_kernel<GBO_MAXD><<<(int)((n + 255) / 256), 256, 0, lc.stream>>>(v, n, dim, pts, cap, first, alive);
+    store_points_kernel<GBO_MAXD><<<(int)((n + 255) / 256), 256, 0, lc.stream>>>(sp, v, n, pts, cap, first, alive,
+                                                                                        outside);
     note_launch();
 }
 

@@ -87,9 +87,15 @@ int knn_keep(int k);
 // features of n states into out[F][ld_out] and, where out4 is given, its float4 planes (same row stride)
 void launch_features(const LaunchCfg &lc, const SpaceParams &sp, StatesView v, int64_t n, float *out, int64_t ld_out,
                      float4 *out4 = nullptr);
-void launch_store_points(const LaunchCfg &lc, StatesView v, int64_t n, int dim, double *pts, int64_t cap,
-                         int64_t first, unsigned char *alive);
+// *outside is raised when a stored coordinate lies outside the space's bounds (or is NaN)
+void launch_store_points(const LaunchCfg &lc, const SpaceParams &sp, StatesView v, int64_t n, double *pts, int64_t cap,
+                         int64_t first, unsigned char *alive, int *outside);
 void launch_remove(const LaunchCfg &lc, const int64_t *keys, int64_t n, int64_t size, unsigned char *alive);
+// nearestR with FP32 distances and FP64 decisions near the radius (kernels_nn_group.cu): counts, or with
+// offsets the sorted segments; nn.alive may be null. False when the space has no FP32 form.
+bool launch_radius_group(const LaunchCfg &lc, const NNArgs &nn, const SpaceParams &sp, StatesView qv, int64_t nq,
+                         double r, const int *outside, int64_t *counts, const int64_t *offsets, int64_t *idx,
+                         double *dist);
 void launch_radius(const LaunchCfg &lc, const NNArgs &nn, const SpaceParams &sp, StatesView qv, int64_t nq, double r,
                    int64_t *counts, const int64_t *offsets, int64_t *idx, double *dist);
 
