@@ -201,6 +201,8 @@ struct gbo_checker
     void *d64 = nullptr, *d32 = nullptr;
     int *cell_start = nullptr, *cell_items = nullptr;
     float *cell_items4 = nullptr;
+    __half *clr = nullptr;
+    ArmTail *tail = nullptr;  // one list per counter slot
     unsigned *test_order = nullptr;
     CounterRing ctr;
     int tuned_schedule = -1;
@@ -220,6 +222,10 @@ struct gbo_checker
             cudaFree(cell_items);
         if (cell_items4)
             cudaFree(cell_items4);
+        if (clr)
+            cudaFree(clr);
+        if (tail)
+            cudaFree(tail);
         if (test_order)
             cudaFree(test_order);
         if (host_stream)
@@ -872,7 +878,10 @@ gbo_status gbo_checker_create(const gbo_space *space, int kind, const double *wo
             arm.sa[i] = code == 0 ? 0.f : (float)code;
             arm.af[i] = (float)arm.a[i];
             arm.dfl[i] = (float)arm.d[i];
+            arm.len[i] = (float)(1.000001 * std::sqrt(arm.a[i] * arm.a[i] + arm.d[i] * arm.d[i]));
         }
+        arm.rsf = (float)sphere_radius;
+        arm.inv_spl = 1.0f / (float)spheres_per_link;
         // FP32 obstacles (rows as given)
         std::vector<float> s32(stride * n_world);
         double rmax = 0.0;
@@ -1029,6 +1038,38 @@ gbo_status gbo_checker_create(const gbo_space *space, int kind, const double *wo
         wa.cell_start = c->cell_start;
         wa.cell_items = c->cell_items;
         wa.grid_n = G;
+        // Clearance grid over the same box. Its distances hold for finite obstacles whose reach |rs + r| is
+        // not larger than rs + r (the box and its margins follow r); otherwise nothing is proven free.
+        {
+            const int CG = 128;  // a multiple of 8
+            bool ok = true;
+            double scale = reach;
+            for (int64_t i = 0; i < stride * n_world; ++i)
+                ok &= std::isfinite(world[i]);
+            for (int64_t i = 0; i < n_world && !boxes; ++i)
+                ok &= world[4 * i + 3] >= -sphere_radius;
+            for (int64_t i = 0; i < n_world && boxes; ++i)
+                for (int r = 3; r < 6; ++r)
+                    ok &= world[6 * i + r] >= 0.0;
+            for (int r = 0; r < 3; ++r)
+                scale = std::max(scale, std::max(std::fabs(lo[r]), std::fabs(hi[r])) + (hi[r] - lo[r]));
+            ok &= scale < 1e3;
+            wa.clr_n = CG;
+            for (int r = 0; r < 3; ++r)
+            {
+                wa.clr_lo[r] = (float)lo[r];
+                wa.clr_cell[r] = (float)((hi[r] - lo[r]) / CG);
+                wa.clr_inv[r] = (float)(CG / (hi[r] - lo[r]));
+            }
+            wa.clr_margin = ok ? (float)(2.0 * dc + 4e-6 * scale + 1e-6) : 1e6f;
+            wa.clr_out = ok ? (float)sphere_radius - wa.clr_margin : -1e6f;
+            if (cudaMalloc(&c->clr, sizeof(__half) * CG * CG * CG) != cudaSuccess ||
+                cudaMalloc(&c->tail, sizeof(ArmTail) * kArmTailRoom * CounterRing::kSlots) != cudaSuccess)
+                return cleanup(fail(GBO_ERR_OUT_OF_MEMORY, "clearance grid allocation failed"));
+            wa.clr = c->clr;
+            launch_arm_clearance(lcfg(nullptr), wa, c->clr);
+            cudaStreamSynchronize(nullptr);
+        }
     }
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess)
@@ -1108,7 +1149,7 @@ static gbo_status motion_impl(gbo_checker *c, const double *s1, const double *s2
     LaunchCfg lc = lcfg(stream);
     RunCounters *ctr = c->ctr.take(lc.stream);
     launch_motion(lc, c->precision, schedule, c->sp, c->wa, make_view(s1, ld, layout), make_view(s2, ld, layout), n,
-                  ok, first_j, nd, ctr);
+                  ok, first_j, nd, ctr, c->tail ? c->tail + (ctr - c->ctr.dev) * kArmTailRoom : nullptr);
     CHECK_LAUNCH();
     return GBO_OK;
 }
@@ -1122,6 +1163,8 @@ gbo_status gbo_check_motion(gbo_checker *c, const double *s1, const double *s2, 
         return fail(GBO_ERR_INVALID_ARGUMENT, "bad checkMotion arguments");
     if (n == 0)
         return GBO_OK;
+    if (schedule == GBO_SCHEDULE_AUTO && c->wa.kind == GBO_CHECK_DH_SPHERES)
+        schedule = GBO_SCHEDULE_WARP;  // one form for every schedule
     if (schedule == GBO_SCHEDULE_AUTO)
     {
         std::lock_guard<std::mutex> lk(c->tune_mu);

@@ -1,6 +1,8 @@
 // Kernel-side argument structures and the launcher interface between the C ABI (capi.cu) and the
 // kernel translation units.
 #pragma once
+#include <cuda_fp16.h>
+
 #include "common.cuh"
 #include "checkers.cuh"
 
@@ -18,7 +20,17 @@ struct RunCounters
     unsigned int max_err_bits;     // kNN: largest |FP32 - FP64| distance of a re-checked candidate (float bits)
     unsigned int timeout;          // a bounded wait ran out
     unsigned int error;
+    unsigned int deferred;         // edges the arm's motion kernel left to its chunk kernel
 };
+
+// An edge whose states many warps share (kernels_arm.cu): first unchecked state, smallest colliding one found
+// (INT_MAX: none)
+struct ArmTail
+{
+    long long e;
+    int next, first;
+};
+constexpr int kArmTailRoom = 2048;
 
 struct DHArm
 {
@@ -28,6 +40,8 @@ struct DHArm
     double a[8], d[8];
     float ca[8], sa[8];  // cos/sin of alpha (exactly 0 or +-1)
     float af[8], dfl[8];
+    float len[8];        // link lengths sqrt(a^2 + d^2), rounded up
+    float rsf, inv_spl;  // rs and 1 / spl
 };
 
 struct WorldArgs
@@ -59,6 +73,12 @@ struct WorldArgs
     // centre (Euclidean) can move when every sine and cosine of the forward kinematics moves by one ulp
     double hz_pos;
     double hz_dh;
+    // clearance grid of the DH arm's world (arm_device.cuh): clr_n^3 cells over the box of the obstacle grid
+    const __half *clr;
+    int clr_n;
+    float clr_lo[3], clr_inv[3], clr_cell[3];
+    float clr_margin;  // taken off the stored distances: FP32 error of both sides and of the positions
+    float clr_out;     // a point outside the box is clear by its distance to the box plus this
     const unsigned *test_order;  // kinematic chain: segment-test order (likely intersections first)
 };
 
@@ -75,13 +95,18 @@ void note_launch();
 void launch_validity(const LaunchCfg &lc, int precision, const SpaceParams &sp, const WorldArgs &wa, StatesView v,
                      int64_t n, uint8_t *out, RunCounters *ctr);
 void launch_motion(const LaunchCfg &lc, int precision, int schedule, const SpaceParams &sp, const WorldArgs &wa,
-                   StatesView v1, StatesView v2, int64_t n, uint8_t *ok, int32_t *fj, int32_t *nd, RunCounters *ctr);
+                   StatesView v1, StatesView v2, int64_t n, uint8_t *ok, int32_t *fj, int32_t *nd, RunCounters *ctr,
+                   ArmTail *tail);
 void launch_states_chain(const LaunchCfg &lc, const SpaceParams &sp, const WorldArgs &wa, StatesView v, int64_t n,
                          unsigned long long *first, RunCounters *ctr);
 void launch_last_valid(const LaunchCfg &lc, const SpaceParams &sp, StatesView v1, StatesView v2, const int32_t *fj,
                        const int32_t *nd, int64_t n, double *last_t, MutStatesView out);
 void launch_chain_hits(cudaStream_t s, const SpaceParams &sp, const WorldArgs &wa, const double *states, int n,
                        unsigned *bits, int words);
+void launch_arm_clearance(const LaunchCfg &lc, const WorldArgs &wa, __half *out);
+void launch_arm_motion(const LaunchCfg &lc, int precision, const SpaceParams &sp, const WorldArgs &wa, StatesView v1,
+                       StatesView v2, int64_t n, ArmTail *tail, uint8_t *ok, int32_t *fj, int32_t *nd,
+                       RunCounters *ctr);
 bool launch_chain_validity_warp(const LaunchCfg &lc, const SpaceParams &sp, const WorldArgs &wa, StatesView v,
                                 int64_t n, uint8_t *out, RunCounters *ctr);
 bool launch_chain_motion_warp(const LaunchCfg &lc, const SpaceParams &sp, const WorldArgs &wa, StatesView v1,
@@ -207,23 +232,23 @@ __device__ bool dh_valid64(const DHArm &arm, const double *q, const double *w, c
 }
 
 // FP64 form of one state, warp-cooperative (warp-uniform call; q and pos in shared memory, q holding the
-// state): every lane runs the forward kinematics above (identical values, so one warp instruction per
-// step), lane 0 records the joint positions in pos[0..joints], and the spheres are spread over the
-// lanes, each centre and each pair test in the operation order of dh_valid64. Same boolean as
+// state): lane r runs row r of the forward kinematics above, the joint positions go to pos[0..joints], and
+// the spheres are spread over the lanes, each centre and each pair test in the operation order of dh_valid64. Same boolean as
 // dh_valid64 on the same state. Out of line: the callers' FP32 loops keep their registers.
 static __device__ __noinline__ bool dh_valid64_warp(const DHArm &arm, const double *q, const double *w,
                                                     const WorldArgs &wa, double (*pos)[3], int lane,
                                                     unsigned long long *hz)
 {
-    double R[3][3] = {{1, 0, 0}, {0, 1, 0}, {0, 0, 1}};
-    double p[3] = {0, 0, 0};
     const int G = wa.grid_n;
-    if (lane == 0)
-        pos[0][0] = pos[0][1] = pos[0][2] = 0.0;
-    // the joints' sines and cosines, one joint per lane (the FK below is the same in every lane)
+    // row r of the rotation and coordinate r of the position in lane r (the rows of R A do not mix)
+    const int row = lane < 3 ? lane : 0;
+    double R0 = row == 0 ? 1.0 : 0.0, R1 = row == 1 ? 1.0 : 0.0, R2 = row == 2 ? 1.0 : 0.0, p = 0.0;
+    if (lane < 3)
+        pos[0][lane] = 0.0;
+    // the joints' sines and cosines, one joint per lane
     double cq_l = 1.0, sq_l = 0.0;
     if (lane < arm.joints)
-        sincos(q[lane], &sq_l, &cq_l);
+        sincos_cr(q[lane], &sq_l, &cq_l);
 #pragma unroll 1
     for (int i = 0; i < arm.joints; ++i)
     {
@@ -231,26 +256,15 @@ static __device__ __noinline__ bool dh_valid64_warp(const DHArm &arm, const doub
         const double ca = (double)arm.ca[i], sa = (double)arm.sa[i];
         const double A[3][3] = {{cq, dmul(-sq, ca), dmul(sq, sa)}, {sq, dmul(cq, ca), dmul(-cq, sa)}, {0.0, sa, ca}};
         const double pA[3] = {dmul(arm.a[i], cq), dmul(arm.a[i], sq), arm.d[i]};
-        double Rn[3][3], pn[3];
-#pragma unroll
-        for (int r = 0; r < 3; ++r)
-        {
-#pragma unroll
-            for (int k = 0; k < 3; ++k)
-                Rn[r][k] = dadd(dadd(dmul(R[r][0], A[0][k]), dmul(R[r][1], A[1][k])), dmul(R[r][2], A[2][k]));
-            pn[r] = dadd(dadd(dadd(dmul(R[r][0], pA[0]), dmul(R[r][1], pA[1])), dmul(R[r][2], pA[2])), p[r]);
-        }
-        if (lane == 0)
-            for (int r = 0; r < 3; ++r)
-                pos[i + 1][r] = pn[r];
-#pragma unroll
-        for (int r = 0; r < 3; ++r)
-        {
-            p[r] = pn[r];
-#pragma unroll
-            for (int k = 0; k < 3; ++k)
-                R[r][k] = Rn[r][k];
-        }
+        const double n0 = dadd(dadd(dmul(R0, A[0][0]), dmul(R1, A[1][0])), dmul(R2, A[2][0]));
+        const double n1 = dadd(dadd(dmul(R0, A[0][1]), dmul(R1, A[1][1])), dmul(R2, A[2][1]));
+        const double n2 = dadd(dadd(dmul(R0, A[0][2]), dmul(R1, A[1][2])), dmul(R2, A[2][2]));
+        p = dadd(dadd(dadd(dmul(R0, pA[0]), dmul(R1, pA[1])), dmul(R2, pA[2])), p);
+        R0 = n0;
+        R1 = n1;
+        R2 = n2;
+        if (lane < 3)
+            pos[i + 1][lane] = p;
     }
     __syncwarp();
     bool hit = false;
