@@ -560,6 +560,89 @@ static gbo_status order_chain_tests(gbo_checker *c)
     return GBO_OK;
 }
 
+// Uniform grid over the circles' bounding box: as many cells a side (at most 256) as keep the lists below 16
+// entries a circle (plus a floor for small worlds). None for a world with a value that is not finite.
+static gbo_status build_circle_grid(gbo_checker *c, const double *world, int64_t n)
+{
+    CircleGrid &g = c->wa.circles;
+    double lo[2] = {1e300, 1e300}, hi[2] = {-1e300, -1e300};
+    for (int64_t i = 0; i < n; ++i)
+        for (int d = 0; d < 2; ++d)
+        {
+            const double x = world[3 * i + d], r = std::fabs(world[3 * i + 2]);
+            if (!(std::fabs(x) < 1e100 && r < 1e100))
+                return GBO_OK;
+            lo[d] = std::min(lo[d], x - r);
+            hi[d] = std::max(hi[d], x + r);
+        }
+    if (n == 0 || !(hi[0] - lo[0] > 0.0) || !(hi[1] - lo[1] > 0.0))
+        return GBO_OK;
+    for (int d = 0; d < 2; ++d)
+    {
+        const double pad = 1e-6 * (hi[d] - lo[d]) + 1e-12 * std::max(std::fabs(lo[d]), std::fabs(hi[d]));
+        lo[d] -= pad;
+        hi[d] += pad;
+    }
+    std::vector<int> start, items;
+    for (int G = 256; G >= 2; G /= 2)
+    {
+        const double cell[2] = {(hi[0] - lo[0]) / G, (hi[1] - lo[1]) / G};
+        auto visit = [&](int64_t i, auto &&emit) {
+            const double x[2] = {world[3 * i], world[3 * i + 1]}, r = std::fabs(world[3 * i + 2]);
+            int a[2], b[2];
+            for (int d = 0; d < 2; ++d)
+            {
+                a[d] = std::max(0, (int)std::floor((x[d] - r - lo[d]) / cell[d]) - 1);
+                b[d] = std::min(G - 1, (int)std::floor((x[d] + r - lo[d]) / cell[d]) + 1);
+            }
+            for (int p = a[0]; p <= b[0]; ++p)
+                for (int q = a[1]; q <= b[1]; ++q)
+                {
+                    double d2 = 0.0;
+                    const int k[2] = {p, q};
+                    for (int d = 0; d < 2; ++d)
+                    {
+                        const double b0 = lo[d] + (k[d] - 1e-3) * cell[d], b1 = lo[d] + (k[d] + 1.0 + 1e-3) * cell[d];
+                        const double gap = x[d] < b0 ? b0 - x[d] : (x[d] > b1 ? x[d] - b1 : 0.0);
+                        d2 += gap * gap;
+                    }
+                    if (d2 <= r * r * (1.0 + 1e-9))
+                        emit(p * G + q);
+                }
+        };
+        const size_t most = 4096 + 16 * (size_t)n;
+        size_t total = 0;
+        start.assign((size_t)G * G + 1, 0);
+        for (int64_t i = 0; i < n && total <= most; ++i)
+            visit(i, [&](int k) {
+                ++start[k + 1];
+                ++total;
+            });
+        if (total > most)
+            continue;
+        for (size_t k = 0; k < (size_t)G * G; ++k)
+            start[k + 1] += start[k];
+        std::vector<int> fill(start.begin(), start.end() - 1);
+        items.assign(std::max<size_t>(total, 1), 0);
+        for (int64_t i = 0; i < n; ++i)
+            visit(i, [&](int k) { items[fill[k]++] = (int)i; });
+        CUDA_TRY(cudaMalloc(&c->cell_start, start.size() * sizeof(int)));
+        CUDA_TRY(cudaMalloc(&c->cell_items, items.size() * sizeof(int)));
+        CUDA_TRY(cudaMemcpy(c->cell_start, start.data(), start.size() * sizeof(int), cudaMemcpyHostToDevice));
+        CUDA_TRY(cudaMemcpy(c->cell_items, items.data(), items.size() * sizeof(int), cudaMemcpyHostToDevice));
+        g.n = G;
+        for (int d = 0; d < 2; ++d)
+        {
+            g.lo[d] = lo[d];
+            g.inv[d] = G / (hi[d] - lo[d]);
+        }
+        g.start = c->cell_start;
+        g.items = c->cell_items;
+        return GBO_OK;
+    }
+    return GBO_OK;
+}
+
 extern "C" {
 
 const char *gbo_status_string(gbo_status s)
@@ -831,7 +914,10 @@ gbo_status gbo_checker_create(const gbo_space *space, int kind, const double *wo
     }
     wa.data64 = c->d64;
     wa.bytes64 = (unsigned)b64;
-    wa.stage64 = (b64 > 0 && b64 <= 96 * 1024 && wa.kind != GBO_CHECK_DH_SPHERES) ? 1 : 0;
+    if (kind == GBO_CHECK_CIRCLES)
+        if (auto st = build_circle_grid(c, world, n_world))
+            return cleanup(st);
+    wa.stage64 = (b64 > 0 && !wa.circles.n && b64 <= 96 * 1024 && wa.kind != GBO_CHECK_DH_SPHERES) ? 1 : 0;
     if (kind == GBO_CHECK_CHAIN_SEGMENTS)
     {
         std::vector<ChainSegF32> segs;

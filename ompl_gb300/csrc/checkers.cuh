@@ -39,6 +39,35 @@ __device__ __forceinline__ bool circles_valid64(const double *w, int n, double x
     return true;
 }
 
+// The same verdict from the circles listed in the point's cell of a uniform grid (n x n cells over the circles'
+// bounding box; a cell lists the circles within a thousandth of a cell of it, which covers the rounding of
+// the cell index). No circle holds a point outside the box, or one that is not a number. The loop over all
+// circles is 5 FP64 operations each on a pipe that takes 16 cycles a warp instruction: 10,000 edges among 100
+// circles 454 us, with the lists (about one circle a point) 36 us; 10,000 states 46 us, 4 us.
+struct CircleGrid
+{
+    int n;  // 0: none
+    double lo[2], inv[2];
+    const int *start, *items;
+};
+__device__ __forceinline__ bool circles_valid64(const double *w, const CircleGrid &g, double x, double y)
+{
+    const float gx = (float)dmul(dsub(x, g.lo[0]), g.inv[0]), gy = (float)dmul(dsub(y, g.lo[1]), g.inv[1]);
+    const float m = (float)g.n;
+    if (!(gx >= 0.f && gx < m && gy >= 0.f && gy < m))
+        return true;
+    const int c = (int)gx * g.n + (int)gy;
+    const int b = __ldg(g.start + c), e = __ldg(g.start + c + 1);
+    for (int k = b; k < e; ++k)
+    {
+        const double *o = w + 3 * (int64_t)__ldg(g.items + k);
+        const double dx = dsub(o[0], x), dy = dsub(o[1], y);
+        if (dadd(dmul(dx, dx), dmul(dy, dy)) < o[2])
+            return false;
+    }
+    return true;
+}
+
 // ---------------------------------------------------------------- kinematic chain (FP64)
 // Segment intersection of demos/KinematicChain.h:251-276.
 __device__ __forceinline__ bool seg_intersect64(double ax0, double ay0, double ax1, double ay1, double bx0, double by0,

@@ -73,6 +73,7 @@ struct WorldArgs
     // centre (Euclidean) can move when every sine and cosine of the forward kinematics moves by one ulp
     double hz_pos;
     double hz_dh;
+    CircleGrid circles;
     // clearance grid of the DH arm's world (arm_device.cuh): clr_n^3 cells over the box of the obstacle grid
     const __half *clr;
     int clr_n;

@@ -48,7 +48,8 @@ struct Eval
     __device__ bool valid64(const SpaceParams &s, const double *q) const
     {
         if constexpr (CK == GBO_CHECK_CIRCLES)
-            return circles_valid64(w64, nw, q[0], q[1]);
+            return wa->circles.n ? circles_valid64(w64, wa->circles, q[0], q[1])
+                                 : circles_valid64(w64, nw, q[0], q[1]);
         else if constexpr (CK == GBO_CHECK_CHAIN_SEGMENTS)
             return chain_valid64<MAXD>(s, q, w64, nw, wa->hz_pos, hz);
         else if constexpr (CK == GBO_CHECK_DH_SPHERES)
@@ -220,10 +221,12 @@ __device__ int segment_count(const SpaceParams &sp, const WorldArgs &wa, const d
     return segment_count_from_distance(sp, distance64<MAXD>(sp, a, b));
 }
 
+// A warp takes `per` consecutive edges at a time: lane i computes the segment count of edge i (FP64, so a warp
+// instruction costs the same for one edge as for 32), then the warp checks the edges one after another.
 template <int CK, int MAXD>
 __global__ void __launch_bounds__(256) motion_plain_kernel(SpaceParams sp, WorldArgs wa, StatesView v1,
-                                                           StatesView v2, int64_t n, uint8_t *ok, int32_t *first_j,
-                                                           int32_t *nd_out, RunCounters *ctr)
+                                                           StatesView v2, int64_t n, int per, uint8_t *ok,
+                                                           int32_t *first_j, int32_t *nd_out, RunCounters *ctr)
 {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ uint64_t bar;
@@ -234,40 +237,53 @@ __global__ void __launch_bounds__(256) motion_plain_kernel(SpaceParams sp, World
     const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     unsigned evaluated = 0, rechecks = 0;
-    for (int64_t e = warp; e < n; e += nwarps)
+    for (int64_t e0 = warp * per; e0 < n; e0 += nwarps * per)
     {
         double a[MAXD], b[MAXD];
-        load_state<MAXD>(v1, e, sp.dim, a);
-        load_state<MAXD>(v2, e, sp.dim, b);
-        const int nd = segment_count_from_distance(sp, distance64<MAXD>(sp, a, b));
-        const int top = nd > 1 ? nd : 1;
-        int first = -1;
-        for (int base = 1; base <= top; base += 32)
+        const int64_t mine = e0 + lane;
+        int nds = 0, result = -1;
+        if (lane < per && mine < n)
         {
-            const int j = base + lane;
-            bool bad = false;
-            if (j <= top)
-            {
-                double q[MAXD];
-                state_at<MAXD>(sp, a, b, j, nd, top, q);
-                bad = !ev.valid64(sp, q);
-                ++evaluated;
-            }
-            const unsigned m = __ballot_sync(0xffffffffu, bad);
-            if (m)
-            {
-                const int jj = base + __ffs(m) - 1;
-                first = jj == top ? nd : jj;
-                break;
-            }
+            load_state<MAXD>(v1, mine, sp.dim, a);
+            load_state<MAXD>(v2, mine, sp.dim, b);
+            nds = segment_count_from_distance(sp, distance64<MAXD>(sp, a, b));
         }
-        if (lane == 0)
+        __syncwarp();
+        for (int i = 0; i < per && e0 + i < n; ++i)
         {
-            ok[e] = first < 0 ? 1 : 0;
+            const int nd = __shfl_sync(0xffffffffu, nds, i), top = nd > 1 ? nd : 1;
+            load_state<MAXD>(v1, e0 + i, sp.dim, a);
+            load_state<MAXD>(v2, e0 + i, sp.dim, b);
+            int first = -1;
+            for (int base = 1; base <= top; base += 32)
+            {
+                const int j = base + lane;
+                bool bad = false;
+                if (j <= top)
+                {
+                    double q[MAXD];
+                    state_at<MAXD>(sp, a, b, j, nd, top, q);
+                    bad = !ev.valid64(sp, q);
+                    ++evaluated;
+                }
+                const unsigned m = __ballot_sync(0xffffffffu, bad);
+                if (m)
+                {
+                    const int jj = base + __ffs(m) - 1;
+                    first = jj == top ? nd : jj;
+                    break;
+                }
+            }
+            if (lane == i)
+                result = first;
+        }
+        if (lane < per && mine < n)
+        {
+            ok[mine] = result < 0 ? 1 : 0;
             if (first_j)
-                first_j[e] = first;
+                first_j[mine] = result;
             if (nd_out)
-                nd_out[e] = nd;
+                nd_out[mine] = nds;
         }
     }
     flush_counts(ctr, evaluated, rechecks);
@@ -580,8 +596,10 @@ static void launch_motion_t(const LaunchCfg &lc, int schedule, const SpaceParams
     {
         auto k = motion_plain_kernel<CK, MAXD>;
         const unsigned sm = world_smem_bytes(wa, GBO_PRECISION_FP64);
-        const int grid = persistent_grid((const void *)k, 256, sm, lc, (n * 32 + 255) / 256);
-        k<<<grid, 256, sm, lc.stream>>>(sp, wa, v1, v2, n, ok, fj, nd, ctr);
+        // 16 warps an SM already keep the FP64 pipe busy: beyond that, edges per warp
+        const int per = (int)std::max<int64_t>(1, std::min<int64_t>(32, n / ((int64_t)lc.sm_count * 16)));
+        const int grid = persistent_grid((const void *)k, 256, sm, lc, ((n + per - 1) / per * 32 + 255) / 256);
+        k<<<grid, 256, sm, lc.stream>>>(sp, wa, v1, v2, n, per, ok, fj, nd, ctr);
     }
     else if (schedule == GBO_SCHEDULE_WARP)
     {
