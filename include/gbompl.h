@@ -162,7 +162,11 @@ gbo_status gbo_last_valid(const gbo_space *s, const double *s1, const double *s2
 gbo_status gbo_check_motion_states(gbo_checker *c, const double *states, int64_t count, int64_t ld, int layout,
                                    uint8_t *ok, int64_t *first_invalid, gbo_stream stream);
 
-/* Host-memory drop-ins (AoS rows like OMPL states); staging buffers are owned by the checker. */
+/* Host-memory drop-ins (AoS rows like OMPL states); staging buffers are owned by the checker. The *_rows
+ * calls run on the caller's stream, after the work it already holds, and return after it. */
+gbo_status gbo_is_valid_rows(gbo_checker *c, const double *states, int64_t n, uint8_t *out, gbo_stream stream);
+gbo_status gbo_check_motion_rows(gbo_checker *c, const double *s1, const double *s2, int64_t n, int schedule,
+                                 uint8_t *ok, int32_t *first_j, int32_t *nd, gbo_stream stream);
 gbo_status gbo_is_valid_host(gbo_checker *c, const double *states, int64_t n, uint8_t *out);
 gbo_status gbo_check_motion_host(gbo_checker *c, const double *s1, const double *s2, int64_t n, uint8_t *ok,
                                  double *last_t, double *last_state);
@@ -250,6 +254,8 @@ gbo_status gbo_nn_nearest_k_noalloc(gbo_nn *nn, const double *q, int64_t nq, int
 gbo_status gbo_nn_add_host(gbo_nn *nn, const double *states, int64_t n, int64_t *first_key);
 gbo_status gbo_nn_remove_host(gbo_nn *nn, const int64_t *keys, int64_t n);
 gbo_status gbo_nn_nearest_k_host(gbo_nn *nn, const double *q, int64_t nq, int k, int64_t *idx, double *dist);
+gbo_status gbo_nn_nearest_k_rows(gbo_nn *nn, const double *q, int64_t nq, int k, int64_t *idx, double *dist,
+                                 gbo_stream stream);
 gbo_status gbo_nn_nearest_r_host(gbo_nn *nn, const double *q, double r, int64_t cap, int64_t *count, int64_t *idx,
                                  double *dist);
 /* Host-memory sampling (AoS rows; synchronous). */

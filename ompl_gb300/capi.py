@@ -97,6 +97,9 @@ SIGNATURES = {
     "gbo_nn_nearest_sqrt_approx": (C.c_int, [_P, _P, _I64, _I64, C.c_int, _P, _P, _P, _P]),
     "gbo_nn_nearest_sqrt_approx_host": (C.c_int, [_P, _P, _I64, _P, _P, _P]),
     "gbo_nn_search_bytes": (C.c_int, [_P, _P]),
+    "gbo_is_valid_rows": (C.c_int, [_P, _P, _I64, _P, _P]),
+    "gbo_check_motion_rows": (C.c_int, [_P, _P, _P, _I64, C.c_int, _P, _P, _P, _P]),
+    "gbo_nn_nearest_k_rows": (C.c_int, [_P, _P, _I64, C.c_int, _P, _P, _P]),
 }
 
 

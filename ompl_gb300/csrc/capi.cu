@@ -1431,6 +1431,64 @@ gbo_status gbo_check_motion_host(gbo_checker *c, const double *s1, const double 
     return GBO_OK;
 }
 
+// Small batches in host memory on the caller's stream (ordered after its earlier work, unlike the *_host
+// calls' own stream): one copy in, the kernels, one copy out through the object's page-locked buffer.
+gbo_status gbo_is_valid_rows(gbo_checker *c, const double *states, int64_t n, uint8_t *out, gbo_stream stream)
+{
+    if (!c || n < 0 || (n > 0 && (!states || !out)))
+        return fail(GBO_ERR_INVALID_ARGUMENT, "bad isValid arguments");
+    if (n == 0)
+        return GBO_OK;
+    const cudaStream_t st = (cudaStream_t)stream;
+    std::lock_guard<std::mutex> lk(c->mu);
+    const size_t bin = (size_t)n * c->sp.dim * sizeof(double);
+    if (auto e = c->pin_in.reserve(bin + (size_t)n))
+        return e;
+    if (auto e = c->dev_in.reserve(bin + (size_t)n, st))
+        return e;
+    char *h = (char *)c->pin_in.p, *d = (char *)c->dev_in.p;
+    std::memcpy(h, states, bin);
+    CUDA_TRY(cudaMemcpyAsync(d, h, bin, cudaMemcpyHostToDevice, st));
+    if (auto e = gbo_is_valid(c, (const double *)d, n, c->sp.dim, GBO_LAYOUT_AOS, (uint8_t *)d + bin, stream))
+        return e;
+    CUDA_TRY(cudaMemcpyAsync(h + bin, d + bin, (size_t)n, cudaMemcpyDeviceToHost, st));
+    CUDA_TRY(cudaStreamSynchronize(st));
+    std::memcpy(out, h + bin, (size_t)n);
+    return GBO_OK;
+}
+
+gbo_status gbo_check_motion_rows(gbo_checker *c, const double *s1, const double *s2, int64_t n, int schedule,
+                                 uint8_t *ok, int32_t *first_j, int32_t *nd, gbo_stream stream)
+{
+    if (!c || n < 0 || (n > 0 && (!s1 || !s2 || !ok || !first_j || !nd)) || schedule < GBO_SCHEDULE_PLAIN ||
+        schedule > GBO_SCHEDULE_AUTO)
+        return fail(GBO_ERR_INVALID_ARGUMENT, "bad checkMotion arguments");
+    if (n == 0)
+        return GBO_OK;
+    const cudaStream_t st = (cudaStream_t)stream;
+    std::lock_guard<std::mutex> lk(c->mu);
+    const size_t bst = (size_t)n * c->sp.dim * sizeof(double), out = 9 * (size_t)n;
+    if (auto e = c->pin_in.reserve(2 * bst + out))
+        return e;
+    if (auto e = c->dev_in.reserve(2 * bst + out, st))
+        return e;
+    char *h = (char *)c->pin_in.p, *d = (char *)c->dev_in.p;
+    std::memcpy(h, s1, bst);
+    std::memcpy(h + bst, s2, bst);
+    CUDA_TRY(cudaMemcpyAsync(d, h, 2 * bst, cudaMemcpyHostToDevice, st));
+    int32_t *fj = (int32_t *)(d + 2 * bst), *ndv = fj + n;
+    uint8_t *okd = (uint8_t *)(ndv + n);
+    if (auto e = gbo_check_motion(c, (const double *)d, (const double *)(d + bst), n, c->sp.dim, GBO_LAYOUT_AOS, schedule,
+                                  okd, fj, ndv, stream))
+        return e;
+    CUDA_TRY(cudaMemcpyAsync(h + 2 * bst, d + 2 * bst, out, cudaMemcpyDeviceToHost, st));
+    CUDA_TRY(cudaStreamSynchronize(st));
+    std::memcpy(first_j, h + 2 * bst, 4 * (size_t)n);
+    std::memcpy(nd, h + 2 * bst + 4 * (size_t)n, 4 * (size_t)n);
+    std::memcpy(ok, h + 2 * bst + 8 * (size_t)n, (size_t)n);
+    return GBO_OK;
+}
+
 // ---------------------------------------------------------------- samplers
 gbo_status gbo_sampler_create(const gbo_space *space, uint32_t local_seed, gbo_sampler **out)
 {
@@ -2157,6 +2215,33 @@ gbo_status gbo_nn_nearest_k_host(gbo_nn *nn, const double *q, int64_t nq, int k,
     std::memcpy(idx, nn->pin.p, bo);
     if (dist)
         std::memcpy(dist, (char *)nn->pin.p + bo, bo);
+    return GBO_OK;
+}
+
+gbo_status gbo_nn_nearest_k_rows(gbo_nn *nn, const double *q, int64_t nq, int k, int64_t *idx, double *dist,
+                                 gbo_stream stream)
+{
+    if (!nn || nq < 0 || k < 1 || (nq > 0 && (!q || !idx || !dist)))
+        return fail(GBO_ERR_INVALID_ARGUMENT, "bad nearestK arguments");
+    if (nq == 0)
+        return GBO_OK;
+    const cudaStream_t st = (cudaStream_t)stream;
+    std::lock_guard<std::mutex> lk(nn->mu);
+    const size_t bq = (size_t)nq * nn->sp.dim * sizeof(double), bo = (size_t)nq * k * 8;
+    if (auto e = nn->pin.reserve(bq + 2 * bo))
+        return e;
+    if (auto e = nn->dev.reserve(bq + 2 * bo, st))
+        return e;
+    char *h = (char *)nn->pin.p, *d = (char *)nn->dev.p;
+    std::memcpy(h, q, bq);
+    CUDA_TRY(cudaMemcpyAsync(d, h, bq, cudaMemcpyHostToDevice, st));
+    if (auto e = gbo_nn_nearest_k(nn, (const double *)d, nq, nn->sp.dim, GBO_LAYOUT_AOS, k, nullptr,
+                                  (int64_t *)(d + bq), (double *)(d + bq + bo), stream))
+        return e;
+    CUDA_TRY(cudaMemcpyAsync(h + bq, d + bq, 2 * bo, cudaMemcpyDeviceToHost, st));
+    CUDA_TRY(cudaStreamSynchronize(st));
+    std::memcpy(idx, h + bq, bo);
+    std::memcpy(dist, h + bq + bo, bo);
     return GBO_OK;
 }
 
