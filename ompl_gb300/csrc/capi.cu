@@ -15,7 +15,7 @@
 #include <nvtx3/nvToolsExt.h>
 
 #include "chain_state.cuh"
-#include "kernels_nn.cuh"
+#include "nn_device.cuh"
 #include "tma.cuh"
 
 using namespace gbo;
@@ -252,15 +252,32 @@ struct gbo_sampler
     }
 };
 
-// Cell index of a gbo_nn over a RealVector / wrapped space (kernels_nn.cu): built by the first large
-// batch after a change of the element set (add / remove / clear clear `valid`).
+// Cell index of a gbo_nn over a RealVector / wrapped space (kernels_nn_cells.cu), over its first `size` elements:
+// built by the first large batch after a change of the element set (add / remove / clear clear `size`).
 struct NNBoxCells
 {
-    bool valid = false;
-    int L = 0, C = 0;
-    DevBuf cell, count, start, fill, skey, pts8, box;
-    DevBuf qcell, qcount, qstart, qfill, qorder;
+    int64_t size = 0;
+    BoxCellShape shape{};
+    DevBuf start, cstart, skey, kmin, pts8, box, extent;
+    gbo_status reserve(int64_t n, cudaStream_t s)
+    {
+        const size_t sub = (size_t)shape.C << shape.bits, chunks = (size_t)n / 32 + shape.C + 1;
+        for (auto r : {start.reserve((sub + 1) * sizeof(int), s), cstart.reserve(((size_t)shape.C + 1) * sizeof(int), s),
+                       skey.reserve((size_t)n * sizeof(int), s), kmin.reserve(chunks * sizeof(int), s),
+                       pts8.reserve((size_t)n * 2 * sizeof(float4), s), box.reserve(chunks * 4 * sizeof(float4), s),
+                       extent.reserve(16 * sizeof(float), s)})
+            if (r)
+                return r;
+        return GBO_OK;
+    }
+    BoxCellArgs args() const
+    {
+        return BoxCellArgs{shape.L, shape.C, shape.bits, shape.dA, shape.nA, shape.nB, (const int *)start.p,
+                           (const int *)cstart.p, (const int *)skey.p, (const int *)kmin.p, (const float4 *)pts8.p,
+                           (const float4 *)box.p, (const float *)extent.p};
+    }
 };
+constexpr int kCellLevels = 12;  // indexes over size, size / 2, ... elements (prefix limits)
 
 // Cell index of a kinematic-chain gbo_nn (kernels_nn.cu), built like NNBoxCells.
 struct NNChainCells
@@ -281,7 +298,9 @@ struct gbo_nn
     int *outside = nullptr;  // device flag: an element lies outside the bounds eps32 was derived for
     unsigned char *alive = nullptr;
     float eps32 = 0.f;
-    NNBoxCells cells;
+    NNBoxCells cells[kCellLevels];
+    int64_t pairs_seen = 0;  // query-element pairs since the element set last changed
+    DevBuf cwork;  // scratch of the cell builds and query orders
     NNChainCells ccells;
     DevBuf qfeat, fb_list, part, qorder;
     DevBuf ranks;  // keys of the present elements in order (approximate nearest after removals)
@@ -1798,7 +1817,9 @@ gbo_status gbo_nn_add(gbo_nn *nn, const double *states, int64_t n, int64_t ld, i
     CHECK_LAUNCH();
     nn->size += n;
     nn->alive_count += n;
-    nn->cells.valid = false;
+    for (auto &c : nn->cells)
+        c.size = 0;
+    nn->pairs_seen = 0;
     nn->ccells.valid = false;
     return GBO_OK;
 }
@@ -1810,7 +1831,9 @@ gbo_status gbo_nn_remove(gbo_nn *nn, const int64_t *keys, int64_t n, gbo_stream 
     launch_remove(lcfg(stream), keys, n, nn->size, nn->alive);
     CHECK_LAUNCH();
     nn->alive_count = -1;  // recounted on demand
-    nn->cells.valid = false;
+    for (auto &c : nn->cells)
+        c.size = 0;
+    nn->pairs_seen = 0;
     nn->ccells.valid = false;
     return GBO_OK;
 }
@@ -1824,7 +1847,9 @@ gbo_status gbo_nn_clear(gbo_nn *nn)
     CUDA_TRY(cudaMemset(nn->outside, 0, sizeof(int)));
     nn->size = 0;
     nn->alive_count = 0;
-    nn->cells.valid = false;
+    for (auto &c : nn->cells)
+        c.size = 0;
+    nn->pairs_seen = 0;
     nn->ccells.valid = false;
     return GBO_OK;
 }
@@ -1862,28 +1887,46 @@ static NNArgs nn_args(const gbo_nn *nn)
     return a;
 }
 
-// (Re)build the cell index of a RealVector / wrapped gbo_nn in stream order.
-static gbo_status ensure_box_cells(gbo_nn *nn, const LaunchCfg &lc)
+// The cell search of a batch over a RealVector / wrapped gbo_nn, building the indexes it needs in stream order.
+static gbo_status box_cells_call(gbo_nn *nn, const LaunchCfg &lc, const float *qf, int64_t nq, const int64_t *prefix,
+                                 int k, const KnnOut &out)
 {
-    NNBoxCells &c = nn->cells;
-    if (c.valid)
-        return GBO_OK;
-    c.L = bcell_levels(nn->sp.dim, nn->size);
-    c.C = 1;
-    for (int d = 0; d < nn->sp.dim; ++d)
-        c.C *= c.L;
-    const int64_t n = std::max<int64_t>(nn->size, 1);
     const cudaStream_t s = lc.stream;
-    for (auto r : {c.cell.reserve((size_t)n * sizeof(int), s), c.count.reserve((size_t)c.C * sizeof(int), s),
-                   c.start.reserve((size_t)(c.C + 1) * sizeof(int), s), c.fill.reserve((size_t)c.C * sizeof(int), s),
-                   c.skey.reserve((size_t)n * sizeof(int64_t), s), c.pts8.reserve((size_t)n * 2 * sizeof(float4), s),
-                   c.box.reserve((size_t)c.C * 4 * sizeof(float4), s)})
-        if (r)
-            return r;
-    launch_bcell_build(lc, nn_args(nn), nn->sp, c.L, c.C, (int *)c.cell.p, (int *)c.count.p, (int *)c.start.p,
-                       (int *)c.fill.p, (int64_t *)c.skey.p, (float4 *)c.pts8.p, (float4 *)c.box.p);
+    int64_t size = nn->size;
+    for (int level = 0; level < kCellLevels; ++level, size /= 2)
+    {
+        NNBoxCells &c = nn->cells[level];
+        KnnOut o = out;
+        o.nn.size = size;
+        const BoxCellShape shape = cell_shape(nn->sp.dim, size);
+        const size_t sub = (size_t)shape.C << shape.bits, sums = sub / 4096 + 2;
+        // [element or query keys | counts | fill | block sums | query starts | query order]
+        const size_t words = (size_t)std::max(size, nq) + 2 * sub + sums + (size_t)shape.C + 1 + (size_t)nq;
+        if (auto e = nn->cwork.reserve(words * sizeof(int), s))
+            return e;
+        int *key = (int *)nn->cwork.p, *count = key + std::max(size, nq), *fill = count + sub, *bs = fill + sub;
+        int *qstart = bs + sums, *qorder = qstart + shape.C + 1;
+        if (c.size != size)
+        {
+            c.shape = shape;
+            if (auto e = c.reserve(size, s))
+                return e;
+            launch_cell_build(lc, o.nn, nn->sp, shape, key, count, bs, fill, c.args());
+            CHECK_LAUNCH();
+            c.size = size;
+        }
+        // limits in (size / 2, size]; without limits, and below 65,536 elements, all that are left
+        const bool last = !prefix || size / 2 < 32768 || level == kCellLevels - 1;
+        launch_knn_cells(lc, c.args(), nn->sp, qf, nq, prefix, size / 2, level == 0, k, key, count, qstart, fill, qorder,
+                         bs, o);
+        CHECK_LAUNCH();
+        if (last)
+            break;
+    }
+    if (prefix && !launch_knn_group(lc, out.nn, nn->sp, out.qv, nq, k, prefix, size / 2, out.idx, out.dist, out.fb_list,
+                                    out.fb_n, out.ctr))
+        return fail(GBO_ERR_UNSUPPORTED, "nearestK: no form for the low prefix limits");
     CHECK_LAUNCH();
-    c.valid = true;
     return GBO_OK;
 }
 
@@ -1930,14 +1973,24 @@ gbo_status gbo_nn_nearest_k(gbo_nn *nn, const double *q, int64_t nq, int64_t ld,
         if (auto st = nn->fb_list.reserve(sizeof(unsigned long long) * nq, lc.stream))
             return st;
         unsigned long long *fb_n = &ctr->queue;
-        // The cell searches take batches large enough to win over reading every element: their fixed cost
-        // (query order, one search per warp) is 0.2 to 0.6 ms. Measured (cells / group kernel): planar,
-        // 200,000 elements, 1,000 queries 184 / 152 us, 4,096 queries 264 / 490 us; wrapped 7-D, 200,000
-        // elements, 1,000 queries 651 / 432 us, 4,096 queries 646 / 1,586 us; 1M elements, 500 queries
-        // 795 / 952 us; chain, 200,000 elements, 4,096 queries 2.37 / 2.58 ms.
+        // The cell searches take batches that are worth more than their fixed cost (query order, the longest
+        // search), counted in query-element pairs. Measured cells / group kernel: 3-D, 60,000 elements, 500
+        // queries (3e7 pairs) 62 / 70 us, 4,096 queries 69 / 327 us; 5-D wrapped, 60,000 elements, 1,000 queries
+        // 121 / 178 us; 7-D, 200,000 elements, 1,000 queries (2e8) 329 / 314 us, 2,000 queries 362 / 568 us;
+        // chain, 200,000 elements, 4,096 queries (8e8) 2.37 / 2.58 ms. An index that is not built yet (0.1 to
+        // 0.3 ms) waits until the set has seen four times that many pairs.
         const bool chain = nn->sp.kind == GBO_SPACE_KINEMATIC_CHAIN;
-        const bool cells = nn->size >= 65536 && nn->size < (1ll << 31) && nq >= (chain ? 1024 : 256) &&
-                           nq * nn->size >= (chain ? 800000000ll : 400000000ll) && !(chain && prefix);
+        const int dim = nn->sp.dim;
+        const int64_t worth = chain ? 800000000ll
+                                    : (dim <= 3 ? 30000000ll
+                                                : dim <= 5 ? 50000000ll
+                                                           : dim == 6 ? 120000000ll : dim == 7 ? 250000000ll : 400000000ll);
+        const bool built = chain ? nn->ccells.valid : nn->cells[0].size == nn->size;
+        const int64_t pairs = nq * nn->size;
+        nn->pairs_seen = std::min<int64_t>(nn->pairs_seen + pairs, 1ll << 60);
+        const bool cells = nn->size >= (chain ? 65536 : 16384) && nn->size < (1ll << 30) && nq < (1ll << 31) &&
+                           nq >= (chain ? 1024 : 64) && pairs >= worth && (chain || built || nn->pairs_seen >= 4 * worth) &&
+                           !(chain && prefix);
         // a huge batch over a tiny index: thread per query (100 elements, 20,000 queries: 148 us against
         // 186 us wrapped, 0.62 ms against 0.91 ms on the chain)
         const bool tiny = nq >= 16384 && nn->size <= 256;
@@ -1946,8 +1999,8 @@ gbo_status gbo_nn_nearest_k(gbo_nn *nn, const double *q, int64_t nq, int64_t ld,
             NNArgs g = a;
             if (nn->alive_count == nn->size)
                 g.alive = nullptr;
-            if (launch_knn_group(lc, g, nn->sp, qv, nq, k, prefix, idx, dist, (unsigned long long *)nn->fb_list.p,
-                                 fb_n, ctr))
+            if (launch_knn_group(lc, g, nn->sp, qv, nq, k, prefix, INT64_MAX, idx, dist,
+                                 (unsigned long long *)nn->fb_list.p, fb_n, ctr))
             {
                 launch_knn_exact(lc, a, nn->sp, qv, nq, k, prefix, idx, dist,
                                  (const unsigned long long *)nn->fb_list.p, fb_n, std::min<int64_t>(nq, 4096));
@@ -1957,42 +2010,17 @@ gbo_status gbo_nn_nearest_k(gbo_nn *nn, const double *q, int64_t nq, int64_t ld,
         }
         if (auto st = nn->qfeat.reserve(sizeof(float) * nn->F * nq, lc.stream))
             return st;
-        const int P = knn_chunks(lc, nq, nn->size);
-        const int keep = knn_keep(k);
-        const size_t pl = (size_t)P * nq * keep;
-        if (auto st = nn->part.reserve(pl * (sizeof(float) + sizeof(int64_t)) + 64, lc.stream))
-            return st;
-        int64_t *part_k = (int64_t *)nn->part.p;
-        float *part_d = (float *)(part_k + pl);
         launch_features(lc, nn->sp, qv, nq, (float *)nn->qfeat.p, nq);
-        // large batches over a large RealVector / wrapped index: cell index (PRM's prefix kNN)
+        // large batches over a large RealVector / wrapped index: cell search (PRM's prefix kNN)
         if (cells && (nn->sp.kind == GBO_SPACE_WRAP_L2 || nn->sp.kind == GBO_SPACE_REAL_VECTOR) && nn->sp.dim <= 8)
         {
-            if (auto st = ensure_box_cells(nn, lc))
+            if (auto st = box_cells_call(nn, lc, (const float *)nn->qfeat.p, nq, prefix, k,
+                                         KnnOut{a, qv, idx, dist, (unsigned long long *)nn->fb_list.p, fb_n, ctr}))
                 return st;
-            NNBoxCells &c = nn->cells;
-            const int bands = prefix ? 4 : 1, keys = bands * c.C;
-            for (auto r : {c.qcell.reserve((size_t)nq * sizeof(int), lc.stream),
-                           c.qcount.reserve((size_t)keys * sizeof(int), lc.stream),
-                           c.qstart.reserve((size_t)(keys + 1) * sizeof(int), lc.stream),
-                           c.qfill.reserve((size_t)keys * sizeof(int), lc.stream),
-                           c.qorder.reserve((size_t)nq * sizeof(int64_t), lc.stream)})
-                if (r)
-                    return r;
-            launch_bcell_query_order(lc, nn->sp, c.L, c.C, (const float *)nn->qfeat.p, nq, prefix, nn->size, bands,
-                                     (int *)c.qcell.p, (int *)c.qcount.p, (int *)c.qstart.p, (int *)c.qfill.p,
-                                     (int64_t *)c.qorder.p);
-            BoxCellArgs ci{(const int *)c.start.p, (const int64_t *)c.skey.p, (const float4 *)c.pts8.p,
-                           (const float4 *)c.box.p, c.C};
-            if (launch_knn_bcell(lc, a, ci, nn->sp, qv, (const float *)nn->qfeat.p, nq, (const int64_t *)c.qorder.p,
-                                 (const int *)c.qcell.p, k, prefix, idx, dist, (unsigned long long *)nn->fb_list.p,
-                                 fb_n, ctr, part_d, part_k))
-            {
-                launch_knn_exact(lc, a, nn->sp, qv, nq, k, prefix, idx, dist,
-                                 (const unsigned long long *)nn->fb_list.p, fb_n, std::min<int64_t>(nq, 4096));
-                CHECK_LAUNCH();
-                return GBO_OK;
-            }
+            launch_knn_exact(lc, a, nn->sp, qv, nq, k, prefix, idx, dist, (const unsigned long long *)nn->fb_list.p, fb_n,
+                             std::min<int64_t>(nq, 4096));
+            CHECK_LAUNCH();
+            return GBO_OK;
         }
         // a large chain index: the cell search, one warp per query (the query order's keys are the cells)
         if (cells && chain && nn->sp.dim <= 10 && k <= 20)
@@ -2010,7 +2038,7 @@ gbo_status gbo_nn_nearest_k(gbo_nn *nn, const double *q, int64_t nq, int64_t ld,
                                    (const float4 *)c.sfeat.p, nn->size,  (const uint4 *)c.box.p,
                                    (const int *)c.cstart.p,   (const uint4 *)c.cbox.p};
             if (launch_knn_ccell(lc, a, ci, nn->sp, qv, (const float *)nn->qfeat.p, nq, ord, work + 3 * kQueryKeys, k,
-                                 idx, dist, (unsigned long long *)nn->fb_list.p, fb_n, ctr, part_d, part_k))
+                                 idx, dist, (unsigned long long *)nn->fb_list.p, fb_n, ctr))
             {
                 launch_knn_exact(lc, a, nn->sp, qv, nq, k, prefix, idx, dist,
                                  (const unsigned long long *)nn->fb_list.p, fb_n, std::min<int64_t>(nq, 4096));
@@ -2018,6 +2046,13 @@ gbo_status gbo_nn_nearest_k(gbo_nn *nn, const double *q, int64_t nq, int64_t ld,
                 return GBO_OK;
             }
         }
+        const int P = knn_chunks(lc, nq, nn->size);
+        const int keep = knn_keep(k);
+        const size_t pl = (size_t)P * nq * keep;
+        if (auto st = nn->part.reserve(pl * (sizeof(float) + sizeof(int64_t)) + 64, lc.stream))
+            return st;
+        int64_t *part_k = (int64_t *)nn->part.p;
+        float *part_d = (float *)(part_k + pl);
         if (launch_knn_fp32(lc, a, nn->sp, qv, (const float *)nn->qfeat.p, nq, k, prefix, idx, dist,
                             (unsigned long long *)nn->fb_list.p, fb_n, ctr, part_d, part_k, P))
         {

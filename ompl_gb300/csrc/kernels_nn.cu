@@ -10,10 +10,11 @@
 //                     query blocks x chunks, so that few queries still fill the GPU), element features
 //                     staged in shared-memory tiles and read as float4; keeps the best K_KEEP by FP32
 //                     distance (kinematic chain: an L1 lower bound skips the square roots of far elements).
-//   knn_bcell_warp_kernel, knn_ccell_warp_kernel
-//                     FP32 bulk over a cell index of the elements (box / wrapped spaces; the chain
-//                     metric), one warp per query: the lanes test 32 cell boxes at a time and scan a
-//                     needed cell's elements 32 at a time; the kept list lives in the lanes.
+//   knn_ccell_warp_kernel
+//                     FP32 bulk over a cell index of the elements (the chain metric; box / wrapped spaces:
+//                     kernels_nn_cells.cu), one warp per query: the lanes test 32 cell boxes at a time and
+//                     scan a needed cell's elements 32 at a time; the kept list lives in the lanes and is
+//                     decided there in FP64.
 //   knn_finish_kernel merges the chunk lists; every kept element within 2*eps of the k-th FP32
 //                     distance is re-evaluated in FP64 and the final order is decided in FP64. If the
 //                     band may hold more than K_KEEP elements the query is queued for knn_exact_kernel.
@@ -146,16 +147,11 @@ __device__ __forceinline__ float chain_l1(const float *a, const float *b, int di
 }
 
 // Partial scan: CTA (x = block of 128 queries, y = chunk of elements). Each thread keeps the K_KEEP
-// smallest FP32 distances (squared for box/wrapped kinds) of its query within the chunk. qorder
-// (nullable): thread qs takes query qorder[qs] (queries in spatial order, so that the lanes of a warp
-// prune the same elements); its list is kept at position qs.
-// qkey (nullable): only the queries with qkey < key_limit are this launch's (the others' lists are
-// written by the cell kernel).
+// smallest FP32 distances (squared for box/wrapped kinds) of its query within the chunk.
 template <int KIND, int MAXF, int K_KEEP>
 __global__ void __launch_bounds__(128) knn_scan_kernel(NNArgs nn, SpaceParams sp, const float *qf, int64_t nq,
                                                        const int64_t *prefix, int64_t chunk, float *part_d,
-                                                       int64_t *part_k, const int64_t *qorder, const int *qkey,
-                                                       int key_limit)
+                                                       int64_t *part_k)
 {
     constexpr int TILE = 128;
     constexpr int FP = (MAXF + 3) / 4 * 4;
@@ -164,8 +160,8 @@ __global__ void __launch_bounds__(128) knn_scan_kernel(NNArgs nn, SpaceParams sp
     __shared__ unsigned long long s_limit;
     const int F = KIND == GBO_SPACE_KINEMATIC_CHAIN ? 2 * sp.dim : sp.dim;
     const int64_t qs = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int64_t qi = qs < nq && qorder ? qorder[qs] : qs;
-    const bool active = qs < nq && (!qkey || qkey[qi] < key_limit);
+    const int64_t qi = qs;
+    const bool active = qs < nq;
     const int64_t c0 = (int64_t)blockIdx.y * chunk;
     const int64_t c1 = min(c0 + chunk, nn.size);
     float qfe[FP];
@@ -258,18 +254,16 @@ __global__ void __launch_bounds__(128) knn_scan_kernel(NNArgs nn, SpaceParams sp
 // Merge the per-chunk lists, then decide in FP64: every element within 2*eps of the k-th FP32
 // distance is re-evaluated with the reference-order FP64 distance and the final order is
 // (FP64 distance, key). If the band may hold more than K_KEEP elements the query goes to the FP64 scan.
-// qorder (nullable): the lists are kept per position qs of the query order, query qorder[qs].
 template <int KIND, int MAXD, int K_KEEP>
 __global__ void __launch_bounds__(128) knn_finish_kernel(NNArgs nn, SpaceParams sp, StatesView qv, int64_t nq, int k,
                                                          int P, const float *part_d, const int64_t *part_k,
                                                          int64_t *idx, double *dist, unsigned long long *fb_list,
-                                                         unsigned long long *fb_n, RunCounters *ctr,
-                                                         const int64_t *qorder)
+                                                         unsigned long long *fb_n, RunCounters *ctr)
 {
     const int64_t qs = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (qs >= nq)
         return;
-    const int64_t qi = qorder ? qorder[qs] : qs;
+    const int64_t qi = qs;
     float dk[K_KEEP];
     int64_t ik[K_KEEP];
 #pragma unroll
@@ -609,9 +603,9 @@ static void launch_fp32_t(const LaunchCfg &lc, const NNArgs &nn, const SpacePara
 {
     const int qb = (int)((nq + 127) / 128);
     knn_scan_kernel<KIND, MAXF, K_KEEP><<<dim3(qb, P), 128, 0, lc.stream>>>(nn, sp, qf, nq, prefix, chunk, part_d,
-                                                                           part_k, nullptr, nullptr, 0);
+                                                                           part_k);
     knn_finish_kernel<KIND, MAXD, K_KEEP><<<qb, 128, 0, lc.stream>>>(nn, sp, qv, nq, k, P, part_d, part_k, idx, dist,
-                                                                    fb_list, fb_n, ctr, nullptr);
+                                                                    fb_list, fb_n, ctr);
     note_launch();
     note_launch();
 }
@@ -821,491 +815,11 @@ void launch_query_order(const LaunchCfg &lc, const SpaceParams &sp, const float 
         note_launch();
 }
 
-// ---------------------------------------------------------------- cell index for box and wrapped spaces
-// Large batches over a large RealVector / wrapped index (PRM's prefix kNN): the alive elements are
-// bucketed by a uniform grid of L levels per coordinate (counting sort); each cell keeps its elements'
-// FP32 coordinates (two float4 per element, sorted by cell) and their bounding box. Queries are
-// processed in (band of their prefix limit, cell) order: each query seeds its threshold T with the k-th
-// FP32 distance among the eligible elements of its own cell (an upper bound on its k-th overall), and
-// skips a cell when the distance from the query to the cell's box is at least min(T, its current
-// K_KEEP-th). Elements beyond T are left out of the lists; the FP64 band of the finish kernel lies
-// below T, so its decisions are unchanged.
-
-__device__ __forceinline__ void bcell_range(const SpaceParams &sp, int d, float &lo, float &hi)
-{
-    if (sp.kind == GBO_SPACE_REAL_VECTOR)
-    {
-        lo = (float)sp.low[d];
-        hi = (float)sp.high[d];
-    }
-    else
-    {
-        lo = -3.14159265358979f;
-        hi = 3.14159265358979f;
-    }
-}
-
-__device__ __forceinline__ int bcell_of(const SpaceParams &sp, int L, const float *f, int64_t ld, int64_t i)
-{
-    int c = 0;
-    for (int d = sp.dim - 1; d >= 0; --d)
-    {
-        float lo, hi;
-        bcell_range(sp, d, lo, hi);
-        int l = hi > lo ? (int)floorf((f[(int64_t)d * ld + i] - lo) * ((float)L / (hi - lo))) : 0;
-        l = l < 0 ? 0 : (l >= L ? L - 1 : l);
-        c = c * L + l;
-    }
-    return c;
-}
-
-__global__ void bcell_assign_kernel(SpaceParams sp, int L, const float *feat, int64_t cap,
-                                    const unsigned char *alive, int64_t n, int *cell, int *count)
-{
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    {
-        if (!alive[i])
-        {
-            cell[i] = -1;
-            continue;
-        }
-        const int c = bcell_of(sp, L, feat, cap, i);
-        cell[i] = c;
-        atomicAdd(&count[c], 1);
-    }
-}
-
-// Exclusive scan of C counts (one CTA of 1024 threads): start[0..C], fill[] cleared.
-__global__ void __launch_bounds__(1024) bcell_scan_kernel(const int *count, int C, int *start, int *fill)
-{
-    __shared__ int part[1024];
-    const int per = (C + 1023) / 1024, i0 = threadIdx.x * per, i1 = min(i0 + per, C);
-    int s = 0;
-    for (int i = i0; i < i1; ++i)
-        s += count[i];
-    part[threadIdx.x] = s;
-    __syncthreads();
-    for (int o = 1; o < 1024; o <<= 1)
-    {
-        const int v = threadIdx.x >= o ? part[threadIdx.x - o] : 0;
-        __syncthreads();
-        part[threadIdx.x] += v;
-        __syncthreads();
-    }
-    int run = part[threadIdx.x] - s;
-    for (int i = i0; i < i1; ++i)
-    {
-        start[i] = run;
-        fill[i] = 0;
-        run += count[i];
-    }
-    if (threadIdx.x == 1023)
-        start[C] = part[1023];
-}
-
-// out[start[c] + arrival order] = i for every row i with c = cell[i] >= 0
-__global__ void bcell_scatter_kernel(const int *cell, int64_t n, const int *start, int *fill, int64_t *out)
-{
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    {
-        const int c = cell[i];
-        if (c >= 0)
-            out[start[c] + atomicAdd(&fill[c], 1)] = i;
-    }
-}
-
-// sorted coordinates: pts8[2p], pts8[2p + 1] = element skey[p] (unused coordinates 0), p < start[C]
-__global__ void bcell_gather_kernel(const int64_t *skey, const int *start, int C, const float *feat, int64_t cap,
-                                    int dim, float4 *pts8)
-{
-    const int64_t total = start[C];
-    for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < total; p += (int64_t)gridDim.x * blockDim.x)
-    {
-        const int64_t key = skey[p];
-        float v[8];
-#pragma unroll
-        for (int d = 0; d < 8; ++d)
-            v[d] = d < dim ? feat[(int64_t)d * cap + key] : 0.f;
-        pts8[2 * p] = make_float4(v[0], v[1], v[2], v[3]);
-        pts8[2 * p + 1] = make_float4(v[4], v[5], v[6], v[7]);
-    }
-}
-
-// box[c] = 4 float4: min of coordinates 0-3, 4-7, then max (warp per cell)
-__global__ void bcell_box_kernel(const float4 *pts8, const int *start, int C, float4 *box)
-{
-    const int lane = threadIdx.x & 31;
-    for (int c = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); c < C; c += (int)((gridDim.x * blockDim.x) >> 5))
-    {
-        float mn[8], mx[8];
-#pragma unroll
-        for (int d = 0; d < 8; ++d)
-        {
-            mn[d] = __int_as_float(0x7f800000);
-            mx[d] = -__int_as_float(0x7f800000);
-        }
-        for (int p = start[c] + lane; p < start[c + 1]; p += 32)
-        {
-            const float4 a = pts8[2 * p], b = pts8[2 * p + 1];
-            const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-#pragma unroll
-            for (int d = 0; d < 8; ++d)
-            {
-                mn[d] = fminf(mn[d], v[d]);
-                mx[d] = fmaxf(mx[d], v[d]);
-            }
-        }
-#pragma unroll
-        for (int d = 0; d < 8; ++d)
-            for (int o = 16; o > 0; o >>= 1)
-            {
-                mn[d] = fminf(mn[d], __shfl_xor_sync(0xffffffffu, mn[d], o));
-                mx[d] = fmaxf(mx[d], __shfl_xor_sync(0xffffffffu, mx[d], o));
-            }
-        if (lane == 0)
-        {
-            box[4 * c] = make_float4(mn[0], mn[1], mn[2], mn[3]);
-            box[4 * c + 1] = make_float4(mn[4], mn[5], mn[6], mn[7]);
-            box[4 * c + 2] = make_float4(mx[0], mx[1], mx[2], mx[3]);
-            box[4 * c + 3] = make_float4(mx[4], mx[5], mx[6], mx[7]);
-        }
-    }
-}
-
-// query key: band then cell. Without prefix limits one band. With them, band 0 holds the queries whose
-// limit is below a quarter of the index (left to the prefix scan: few eligible elements, no useful
-// threshold; keyed by decreasing limit), bands 1 .. bands - 1 split the rest evenly.
-__global__ void bcell_query_key_kernel(SpaceParams sp, int L, int C, const float *qf, int64_t nq,
-                                       const int64_t *prefix, int64_t index_n, int bands, int *key, int *count)
-{
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nq; i += (int64_t)gridDim.x * blockDim.x)
-    {
-        int band = 0, c;
-        if (prefix && bands > 1)
-        {
-            const int64_t lim = prefix[i] < 0 ? 0 : (prefix[i] > index_n ? index_n : prefix[i]);
-            const int64_t q4 = index_n / 4, rest = index_n - q4;
-            band = lim < q4 ? 0 : 1 + (int)min((int64_t)bands - 2, (lim - q4) * (bands - 1) / (rest > 0 ? rest : 1));
-            // band 0 goes to the prefix scan, whose CTAs scan up to their largest limit: its queries are
-            // ordered by decreasing limit (C buckets), so that a CTA's limits are close and the longest
-            // CTAs start first
-            c = band == 0 ? (C - 1) - (int)min((int64_t)C - 1, lim * C / (q4 > 0 ? q4 : 1))
-                          : band * C + bcell_of(sp, L, qf, nq, i);
-        }
-        else
-            c = bcell_of(sp, L, qf, nq, i);
-        key[i] = c;
-        atomicAdd(&count[c], 1);
-    }
-}
-
-// distance from query q to the box (lo, hi per coordinate), squared, scaled down by (1 - 1e-5) against
-// the rounding of both sides
-template <int KIND, int MAXF>
-__device__ __forceinline__ float bcell_lb(const float4 *b, const float *q, int dim)
-{
-    const float4 l0 = b[0], l1 = b[1], h0 = b[2], h1 = b[3];
-    const float lo[8] = {l0.x, l0.y, l0.z, l0.w, l1.x, l1.y, l1.z, l1.w};
-    const float hi[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
-    float s = 0.f;
-#pragma unroll
-    for (int i = 0; i < MAXF; ++i)
-        if (i < dim)
-        {
-            const float x = q[i];
-            float d;
-            if constexpr (KIND == GBO_SPACE_WRAP_L2 || KIND == GBO_SPACE_SO2)
-            {
-                // nearest point of [lo, hi] on the circle: 0 inside, else the nearer end
-                const float a = fabsf(x - lo[i]), c = fabsf(x - hi[i]);
-                const float wa = fminf(a, 6.28318530717958647692f - a), wc = fminf(c, 6.28318530717958647692f - c);
-                d = (x >= lo[i] && x <= hi[i]) ? 0.f : fminf(wa, wc);
-            }
-            else
-                d = fmaxf(fmaxf(lo[i] - x, x - hi[i]), 0.f);
-            s = fmaf(d, d, s);
-        }
-    return s * (1.0f - 1e-5f);
-}
-
-// Cell search, one warp per query: the 32 lanes test 32 cells' boxes at a time and evaluate a needed
-// cell's elements 32 at a time, so a warp visits only the cells its own query needs (a lane-per-query
-// form, where a warp's 32 queries visit the union of their cells, kept about 10 of 32 lanes busy). The
-// kept list is spread over the lanes (WarpList). Seed and thresholds as above: the own cell first, T
-// from its k-th distance, then every other cell whose box is nearer than min(T, the list's last entry).
-// One list per query (P = 1).
-// The kept list spread over a warp: entry j = 32 s + lane in slot s of the lane (S = K_KEEP / 32
-// rounded up slots), ascending, unused entries +inf / -1.
-template <int K_KEEP>
-struct WarpList
-{
-    static constexpr int S = (K_KEEP + 31) / 32;
-    float d[S];
-    int k[S];
-    __device__ __forceinline__ void init()
-    {
-#pragma unroll
-        for (int s = 0; s < S; ++s)
-        {
-            d[s] = __int_as_float(0x7f800000);
-            k[s] = -1;
-        }
-    }
-    // entry j of the list, in every lane
-    __device__ __forceinline__ float at(int j) const
-    {
-        float v = d[0];
-#pragma unroll
-        for (int s = 1; s < S; ++s)
-            if (j >> 5 == s)
-                v = d[s];
-        return __shfl_sync(0xffffffffu, v, j & 31);
-    }
-    __device__ __forceinline__ float last() const { return at(K_KEEP - 1); }
-    // inserts (dd, kk) after the entries with a distance <= dd (those kept earlier stay first)
-    __device__ __forceinline__ void insert(float dd, int kk, int lane)
-    {
-        int pos = 0;
-#pragma unroll
-        for (int s = 0; s < S; ++s)
-            pos += __popc(__ballot_sync(0xffffffffu, 32 * s + lane < K_KEEP && d[s] <= dd));
-        if (pos >= K_KEEP)
-            return;
-        float up_d[S];
-        int up_k[S];
-#pragma unroll
-        for (int s = 0; s < S; ++s)
-        {
-            up_d[s] = __shfl_up_sync(0xffffffffu, d[s], 1);
-            up_k[s] = __shfl_up_sync(0xffffffffu, k[s], 1);
-            if (s > 0)
-            {
-                // lane 0 of slot s takes entry 32 s - 1: lane 31 of slot s - 1
-                const float cd = __shfl_sync(0xffffffffu, d[s - 1], 31);
-                const int ck = __shfl_sync(0xffffffffu, k[s - 1], 31);
-                if (lane == 0)
-                {
-                    up_d[s] = cd;
-                    up_k[s] = ck;
-                }
-            }
-        }
-#pragma unroll
-        for (int s = 0; s < S; ++s)
-        {
-            const int j = 32 * s + lane;
-            if (j >= pos && j < K_KEEP)
-            {
-                d[s] = j == pos ? dd : up_d[s];
-                k[s] = j == pos ? kk : up_k[s];
-            }
-        }
-    }
-};
-
-template <int KIND, int K_KEEP>
-__global__ void __launch_bounds__(256) knn_bcell_warp_kernel(BoxCellArgs ci, SpaceParams sp, float eps,
-                                                             const float *qf, int64_t nq, const int64_t *qorder,
-                                                             const int *qcell, const int64_t *prefix, int k,
-                                                             float *part_d, int64_t *part_k)
-{
-    const int lane = threadIdx.x & 31;
-    const int64_t qs = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (qs >= nq)
-        return;
-    const int64_t qi = qorder[qs];
-    if (prefix && qcell[qi] < ci.C)
-        return;  // band 0 belongs to the prefix scan
-    float qfe[8];
-#pragma unroll
-    for (int f = 0; f < 8; ++f)
-        qfe[f] = f < sp.dim ? qf[(int64_t)f * nq + qi] : 0.f;
-    const int64_t limit = prefix ? prefix[qi] : INT64_MAX;
-    WarpList<K_KEEP> L;
-    L.init();
-    // one cell's eligible elements, 32 at a time; candidates below `cut` enter the list in lane order
-    auto scan_cell = [&](int c, float T) {
-        const int s0 = ci.start[c], s1 = ci.start[c + 1];
-        for (int p0 = s0; p0 < s1; p0 += 32)
-        {
-            const int p = p0 + lane;
-            float d = __int_as_float(0x7f800000);
-            int key = -1;
-            if (p < s1)
-            {
-                const int64_t kk = ci.skey[p];
-                if (kk < limit)
-                {
-                    const float4 a = ci.pts8[2 * (int64_t)p], b = ci.pts8[2 * (int64_t)p + 1];
-                    const float pf[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-                    d = box_dist2<KIND, 8>(pf, qfe, sp.dim);
-                    key = (int)kk;
-                }
-            }
-            const float last = L.last();
-            unsigned m = __ballot_sync(0xffffffffu, d < last && d <= T);
-            while (m)
-            {
-                const int src = __ffs(m) - 1;
-                m &= m - 1;
-                const float dc = __shfl_sync(0xffffffffu, d, src);
-                const int kc = __shfl_sync(0xffffffffu, key, src);
-                if (dc < L.last())
-                    L.insert(dc, kc, lane);
-            }
-        }
-    };
-    // seed: the query's own cell, then T from its k-th distance
-    const int oc = qcell[qi] % ci.C;  // the query key is band * C + cell
-    scan_cell(oc, __int_as_float(0x7f800000));
-    float T = __int_as_float(0x7f800000);
-    const float dkk = L.at(k - 1);
-    if (dkk < __int_as_float(0x7f800000))
-    {
-        const float r = sqrtf(dkk) + 2.f * eps;
-        T = r * r * (1.0f + 1e-5f);
-    }
-    for (int cb = 0; cb < ci.C; cb += 32)
-    {
-        const int c = cb + lane;
-        float lb = __int_as_float(0x7f800000);
-        if (c < ci.C && c != oc && ci.start[c] != ci.start[c + 1])
-            lb = bcell_lb<KIND, 8>(ci.box + 4 * (int64_t)c, qfe, sp.dim);
-        unsigned m = __ballot_sync(0xffffffffu, lb < fminf(T, L.last()));
-        while (m)
-        {
-            const int src = __ffs(m) - 1;
-            m &= m - 1;
-            // the list may have tightened since the cells were tested
-            if (__shfl_sync(0xffffffffu, lb, src) < fminf(T, L.last()))
-            {
-                scan_cell(cb + src, T);
-                // T follows the list's k-th distance (the final band only lies lower)
-                const float dk = L.at(k - 1);
-                if (dk < __int_as_float(0x7f800000))
-                {
-                    const float r = sqrtf(dk) + 2.f * eps;
-                    T = fminf(T, r * r * (1.0f + 1e-5f));
-                }
-            }
-        }
-    }
-#pragma unroll
-    for (int s = 0; s < WarpList<K_KEEP>::S; ++s)
-        if (32 * s + lane < K_KEEP)
-        {
-            part_d[qs * K_KEEP + 32 * s + lane] = L.d[s];
-            part_k[qs * K_KEEP + 32 * s + lane] = L.k[s];
-        }
-}
-
-int bcell_levels(int dim, int64_t n)
-{
-    // about 40 elements per cell, at most 65536 cells
-    int L = 2;
-    while (true)
-    {
-        int64_t c = 1;
-        for (int d = 0; d < dim; ++d)
-            c *= L + 1;
-        if (c > 65536 || c * 40 > n)
-            break;
-        ++L;
-    }
-    return L;
-}
-
 static int grid_for(const LaunchCfg &lc, int64_t n)
 {
     return (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, (int64_t)lc.sm_count * 8));
 }
 
-void launch_bcell_build(const LaunchCfg &lc, const NNArgs &nn, const SpaceParams &sp, int L, int C, int *cell,
-                        int *count, int *start, int *fill, int64_t *skey, float4 *pts8, float4 *box)
-{
-    cudaMemsetAsync(count, 0, (size_t)C * sizeof(int), lc.stream);
-    bcell_assign_kernel<<<grid_for(lc, nn.size), 256, 0, lc.stream>>>(sp, L, nn.feat32, nn.cap, nn.alive, nn.size,
-                                                                      cell, count);
-    bcell_scan_kernel<<<1, 1024, 0, lc.stream>>>(count, C, start, fill);
-    bcell_scatter_kernel<<<grid_for(lc, nn.size), 256, 0, lc.stream>>>(cell, nn.size, start, fill, skey);
-    bcell_gather_kernel<<<grid_for(lc, nn.size), 256, 0, lc.stream>>>(skey, start, C, nn.feat32, nn.cap, sp.dim,
-                                                                      pts8);
-    bcell_box_kernel<<<grid_for(lc, (int64_t)C * 32), 256, 0, lc.stream>>>(pts8, start, C, box);
-    for (int i = 0; i < 5; ++i)
-        note_launch();
-}
-
-void launch_bcell_query_order(const LaunchCfg &lc, const SpaceParams &sp, int L, int C, const float *qf, int64_t nq,
-                              const int64_t *prefix, int64_t index_n, int bands, int *qcell, int *count, int *start,
-                              int *fill, int64_t *qorder)
-{
-    const int keys = bands * C;
-    cudaMemsetAsync(count, 0, (size_t)keys * sizeof(int), lc.stream);
-    bcell_query_key_kernel<<<grid_for(lc, nq), 256, 0, lc.stream>>>(sp, L, C, qf, nq, prefix, index_n, bands, qcell,
-                                                                    count);
-    bcell_scan_kernel<<<1, 1024, 0, lc.stream>>>(count, keys, start, fill);
-    bcell_scatter_kernel<<<grid_for(lc, nq), 256, 0, lc.stream>>>(qcell, nq, start, fill, qorder);
-    for (int i = 0; i < 3; ++i)
-        note_launch();
-}
-
-template <int KIND, int K_KEEP>
-static void launch_bcell_t(const LaunchCfg &lc, const NNArgs &nn, const BoxCellArgs &ci, const SpaceParams &sp,
-                           StatesView qv, const float *qf, int64_t nq, const int64_t *qorder, const int *qcell, int k,
-                           const int64_t *prefix, int64_t *idx, double *dist, unsigned long long *fb_list,
-                           unsigned long long *fb_n, RunCounters *ctr, float *part_d, int64_t *part_k)
-{
-    // one list per query (P = 1): the warp kernel visits every cell a query needs, and the prefix scan
-    // of band 0 covers each of its queries' limits in one CTA
-    const int qb = (int)((nq + 127) / 128), P = 1;
-    knn_bcell_warp_kernel<KIND, K_KEEP><<<(int)((nq * 32 + 255) / 256), 256, 0, lc.stream>>>(
-        ci, sp, nn.eps32, qf, nq, qorder, qcell, prefix, k, part_d, part_k);
-    if (prefix)
-    {
-        // band 0 (limits below a quarter of the index) through the prefix scan, same P lists
-        knn_scan_kernel<KIND, 8, K_KEEP><<<dim3(qb, P), 128, 0, lc.stream>>>(nn, sp, qf, nq, prefix,
-                                                                            (nn.size + P - 1) / P, part_d, part_k,
-                                                                            qorder, qcell, ci.C);
-        note_launch();
-    }
-    knn_finish_kernel<KIND, 8, K_KEEP><<<qb, 128, 0, lc.stream>>>(nn, sp, qv, nq, k, P, part_d, part_k, idx, dist,
-                                                                 fb_list, fb_n, ctr, qorder);
-    note_launch();
-    note_launch();
-}
-
-bool launch_knn_bcell(const LaunchCfg &lc, const NNArgs &nn, const BoxCellArgs &ci, const SpaceParams &sp,
-                      StatesView qv, const float *qf, int64_t nq, const int64_t *qorder, const int *qcell, int k,
-                      const int64_t *prefix, int64_t *idx, double *dist, unsigned long long *fb_list,
-                      unsigned long long *fb_n, RunCounters *ctr, float *part_d, int64_t *part_k)
-{
-    if (nq == 0 || sp.dim > 8 || k > knn_fp32_max_k(sp))
-        return false;
-#define GBO_BCELL_T(KIND, KK)                                                                                         \
-    launch_bcell_t<KIND, KK>(lc, nn, ci, sp, qv, qf, nq, qorder, qcell, k, prefix, idx, dist, fb_list, fb_n, ctr,     \
-                             part_d, part_k)
-#define GBO_BCELL(KIND)                                                                                                \
-    do                                                                                                                \
-    {                                                                                                                 \
-        if (k <= 12)                                                                                                  \
-            GBO_BCELL_T(KIND, 16);                                                                                    \
-        else if (k <= 20)                                                                                             \
-            GBO_BCELL_T(KIND, 24);                                                                                    \
-        else if (k <= 40)                                                                                             \
-            GBO_BCELL_T(KIND, 48);                                                                                    \
-        else                                                                                                          \
-            GBO_BCELL_T(KIND, 72);                                                                                    \
-    } while (0)
-    if (sp.kind == GBO_SPACE_WRAP_L2)
-        GBO_BCELL(GBO_SPACE_WRAP_L2);
-    else if (sp.kind == GBO_SPACE_REAL_VECTOR)
-        GBO_BCELL(GBO_SPACE_REAL_VECTOR);
-    else
-        return false;
-#undef GBO_BCELL_T
-#undef GBO_BCELL
-    return true;
-}
 
 
 // ---------------------------------------------------------------- cell index for the chain metric
@@ -1623,8 +1137,8 @@ __device__ __forceinline__ float ccell_lb(const uint4 *b, const float *q, int di
 template <int K_KEEP>
 __global__ void __launch_bounds__(256, 3) knn_ccell_warp_kernel(ChainCellArgs ci, SpaceParams sp, float eps,
                                                              const float *qf, int64_t nq, const int64_t *qorder,
-                                                             const int *qkey, int k, float *part_d, int64_t *part_k,
-                                                             RunCounters *ctr)
+                                                             const int *qkey, int k,
+                                                             const __grid_constant__ KnnOut out)
 {
     const int lane = threadIdx.x & 31;
     const int64_t qs = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -1837,40 +1351,24 @@ __global__ void __launch_bounds__(256, 3) knn_ccell_warp_kernel(ChainCellArgs ci
             }
         }
     }
-#pragma unroll
-    for (int s = 0; s < WarpList<K_KEEP>::S; ++s)
-        if (32 * s + lane < K_KEEP)
-        {
-            part_d[qs * K_KEEP + 32 * s + lane] = L.d[s];
-            part_k[qs * K_KEEP + 32 * s + lane] = L.k[s];
-        }
-    if (lane == 0 && ctr)
-        atomicAdd(&ctr->bytes, nbytes);
+    if (lane == 0)
+        atomicAdd(&out.ctr->bytes, nbytes);
+    warp_finish<GBO_SPACE_KINEMATIC_CHAIN, 10, K_KEEP>(out, sp, qi, k, L, lane);
 }
 
 bool launch_knn_ccell(const LaunchCfg &lc, const NNArgs &nn, const ChainCellArgs &ci, const SpaceParams &sp,
                       StatesView qv, const float *qf, int64_t nq, const int64_t *qorder, const int *qkey, int k,
                       int64_t *idx, double *dist, unsigned long long *fb_list, unsigned long long *fb_n,
-                      RunCounters *ctr, float *part_d, int64_t *part_k)
+                      RunCounters *ctr)
 {
     if (nq == 0 || sp.kind != GBO_SPACE_KINEMATIC_CHAIN || sp.dim > 10 || k > 20)
         return false;
-    const int qb = (int)((nq + 127) / 128), wg = (int)((nq * 32 + 255) / 256);
+    const int wg = (int)((nq * 32 + 255) / 256);
+    const KnnOut out{nn, qv, idx, dist, fb_list, fb_n, ctr};
     if (k <= 12)
-    {
-        knn_ccell_warp_kernel<16><<<wg, 256, 0, lc.stream>>>(ci, sp, nn.eps32, qf, nq, qorder, qkey, k, part_d, part_k,
-                                                             ctr);
-        knn_finish_kernel<GBO_SPACE_KINEMATIC_CHAIN, 10, 16><<<qb, 128, 0, lc.stream>>>(
-            nn, sp, qv, nq, k, 1, part_d, part_k, idx, dist, fb_list, fb_n, ctr, qorder);
-    }
+        knn_ccell_warp_kernel<16><<<wg, 256, 0, lc.stream>>>(ci, sp, nn.eps32, qf, nq, qorder, qkey, k, out);
     else
-    {
-        knn_ccell_warp_kernel<24><<<wg, 256, 0, lc.stream>>>(ci, sp, nn.eps32, qf, nq, qorder, qkey, k, part_d, part_k,
-                                                             ctr);
-        knn_finish_kernel<GBO_SPACE_KINEMATIC_CHAIN, 10, 24><<<qb, 128, 0, lc.stream>>>(
-            nn, sp, qv, nq, k, 1, part_d, part_k, idx, dist, fb_list, fb_n, ctr, qorder);
-    }
-    note_launch();
+        knn_ccell_warp_kernel<24><<<wg, 256, 0, lc.stream>>>(ci, sp, nn.eps32, qf, nq, qorder, qkey, k, out);
     note_launch();
     return true;
 }

@@ -26,29 +26,38 @@ bool launch_knn_fp32(const LaunchCfg &lc, const NNArgs &nn, const SpaceParams &s
                      int64_t nq, int k, const int64_t *prefix, int64_t *idx, double *dist, unsigned long long *fb_list,
                      unsigned long long *fb_n, RunCounters *ctr, float *part_d, int64_t *part_k, int P);
 // nearestK in one launch (kernels_nn_group.cu): no query features, partial lists or order; nn.alive may be
-// null (every element present). False when the space or k has no FP32 form.
+// null (every element present). max_limit: queries with a larger prefix limit are left out. False when the space
+// or k has no FP32 form.
 bool launch_knn_group(const LaunchCfg &lc, const NNArgs &nn, const SpaceParams &sp, StatesView qv, int64_t nq, int k,
-                      const int64_t *prefix, int64_t *idx, double *dist, unsigned long long *fb_list,
+                      const int64_t *prefix, int64_t max_limit, int64_t *idx, double *dist, unsigned long long *fb_list,
                       unsigned long long *fb_n, RunCounters *ctr);
-// Cell index of a RealVector / wrapped nearest-neighbour index (large batches, PRM prefix kNN).
+// Cell index of a RealVector / wrapped nearest-neighbour index (kernels_nn_cells.cu).
+struct BoxCellShape
+{
+    int L, C, bits;   // levels per coordinate, cells L^dim, sub-cell bits
+    int dA, nA, nB;   // coordinates of the first partial sum, entries of both
+};
 struct BoxCellArgs
 {
-    const int *start;      // [C + 1] first sorted position of each cell
-    const int64_t *skey;   // element key at each sorted position
-    const float4 *pts8;    // two float4 (8 coordinates) per sorted position
-    const float4 *box;     // four float4 per cell: min of coordinates 0-3, 4-7, max 0-3, 4-7
-    int C;
+    int L, C, bits, dA, nA, nB;
+    const int *start;     // [(C << bits) + 1] first sorted position of each sub-cell
+    const int *cstart;    // [C + 1] first chunk of each cell
+    const int *skey;      // element key at each sorted position
+    const int *kmin;      // smallest key of each chunk
+    const float4 *pts8;   // two float4 (8 coordinates) per sorted position
+    const float4 *box;    // four float4 per chunk: min of coordinates 0-3, 4-7, max 0-3, 4-7
+    const float *extent;  // per coordinate: smallest and largest value (16 floats)
 };
-int bcell_levels(int dim, int64_t n);
-void launch_bcell_build(const LaunchCfg &lc, const NNArgs &nn, const SpaceParams &sp, int L, int C, int *cell,
-                        int *count, int *start, int *fill, int64_t *skey, float4 *pts8, float4 *box);
-void launch_bcell_query_order(const LaunchCfg &lc, const SpaceParams &sp, int L, int C, const float *qf, int64_t nq,
-                              const int64_t *prefix, int64_t index_n, int bands, int *qcell, int *count, int *start,
-                              int *fill, int64_t *qorder);
-bool launch_knn_bcell(const LaunchCfg &lc, const NNArgs &nn, const BoxCellArgs &ci, const SpaceParams &sp,
-                      StatesView qv, const float *qf, int64_t nq, const int64_t *qorder, const int *qcell, int k,
-                      const int64_t *prefix, int64_t *idx, double *dist, unsigned long long *fb_list,
-                      unsigned long long *fb_n, RunCounters *ctr, float *part_d, int64_t *part_k);
+struct KnnOut;
+BoxCellShape cell_shape(int dim, int64_t n);
+// index over the first nn.size elements; key: [size], count, fill: [C << bits], sums: [(C << bits) / 4096 + 1]
+void launch_cell_build(const LaunchCfg &lc, const NNArgs &nn, const SpaceParams &sp, const BoxCellShape &s, int *key,
+                       int *count, int *sums, int *fill, const BoxCellArgs &ci);
+// the queries with a limit in (above, out.nn.size] (top: above alone; no limits: all). qkey, qorder: [nq],
+// qcount, qfill: [C], qstart: [C + 1]
+void launch_knn_cells(const LaunchCfg &lc, const BoxCellArgs &ci, const SpaceParams &sp, const float *qf, int64_t nq,
+                      const int64_t *prefix, int64_t above, bool top, int k, int *qkey, int *qcount, int *qstart,
+                      int *qfill, int *qorder, int *sums, const KnnOut &out);
 
 // Spatial processing order of a query batch (counting sort by a cell key of its FP32 features):
 // work holds 3 * kQueryKeys + nq ints, order nq entries.
@@ -73,11 +82,11 @@ struct ChainCellArgs
 void launch_ccell_build(const LaunchCfg &lc, const NNArgs &nn, const SpaceParams &sp, int *key, int *count,
                         int *start, int *fill, int64_t *skey, float4 *sfeat, uint4 *box, int *cstart, uint4 *cbox);
 // qorder / qkey: the query order and each query's key (launch_query_order's order and key arrays).
-// Returns true when launched (lists for every query, P = 1, and the finish kernel).
+// Returns true when launched.
 bool launch_knn_ccell(const LaunchCfg &lc, const NNArgs &nn, const ChainCellArgs &ci, const SpaceParams &sp,
                       StatesView qv, const float *qf, int64_t nq, const int64_t *qorder, const int *qkey, int k,
                       int64_t *idx, double *dist, unsigned long long *fb_list, unsigned long long *fb_n,
-                      RunCounters *ctr, float *part_d, int64_t *part_k);
+                      RunCounters *ctr);
 
 int knn_chunks(const LaunchCfg &lc, int64_t nq, int64_t size);
 // largest k of the FP32-guarded kNN forms (64 for box / wrapped kinds of dim <= 8, else 20; larger k

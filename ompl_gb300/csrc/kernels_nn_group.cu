@@ -18,6 +18,8 @@
 // 44 us. Bound: at 500 queries the kernel issues on 36% of its cycles (57 warp instructions per 32
 // pairs; the waves of CTAs are short); DRAM and L2 are below 10%.
 #include <algorithm>
+#include <climits>
+#include <cstdint>
 
 #include <cooperative_groups.h>
 
@@ -141,7 +143,7 @@ __device__ __forceinline__ void element_features(const NNArgs &nn, const SpacePa
 template <int KIND, int MAXF, int QG, int kThreads>
 __global__ void __launch_bounds__(kThreads, QG == 4 ? (MAXF <= 8 ? 768 : 512) / kThreads : 2) knn_group_kernel(NNArgs nn, SpaceParams sp, StatesView qv, int64_t nq,
                                                              int k, int K, int buckets, const int64_t *prefix,
-                                                             int64_t *idx, double *dist, unsigned long long *fb_list,
+                                                             int64_t max_limit, int64_t *idx, double *dist, unsigned long long *fb_list,
                                                              unsigned long long *fb_n, RunCounters *ctr)
 {
     constexpr int MAXD = KIND == GBO_SPACE_KINEMATIC_CHAIN ? MAXF / 2 : MAXF;
@@ -153,6 +155,20 @@ __global__ void __launch_bounds__(kThreads, QG == 4 ? (MAXF <= 8 ? 768 : 512) / 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t q0 = (int64_t)(blockIdx.x / CS) * QG;
     const float link = (float)sp.link;
+    // queries of another launch (the same ones in every CTA of a cluster)
+    unsigned skip = 0;
+    if (prefix && max_limit < INT64_MAX)
+    {
+        bool any = false;
+        for (int g = 0; g < QG && q0 + g < nq; ++g)
+        {
+            const bool theirs = prefix[q0 + g] > max_limit;
+            skip |= theirs ? 1u << g : 0u;
+            any |= !theirs;
+        }
+        if (!any)
+            return;
+    }
 
     // queries: their FP32 features (as features_kernel forms them) and the number of elements they see
     float qf[QG][MAXF];
@@ -166,7 +182,7 @@ __global__ void __launch_bounds__(kThreads, QG == 4 ? (MAXF <= 8 ? 768 : 512) / 
         {
             l = nn.size;
             if (prefix)
-                l = min(l, prefix[q]);
+                l = skip >> g & 1u ? 0 : min(l, prefix[q]);
         }
         lim[g] = (int)max(l, (int64_t)0);
         top = max(top, lim[g]);
@@ -332,7 +348,7 @@ __global__ void __launch_bounds__(kThreads, QG == 4 ? (MAXF <= 8 ? 768 : 512) / 
 
     // finish: warp w of the owning CTA takes query g with g / CS == w
     const int g = warp * CS + rank;
-    if (g >= QG || q0 + g >= nq)
+    if (g >= QG || q0 + g >= nq || (skip >> g & 1u))
         return;
     const int64_t qi = q0 + g;
     const float T = sm.T[g], eps = nn.eps32;
@@ -443,7 +459,7 @@ namespace
 {
 template <int KIND, int MAXF, int QG, int kThreads>
 void launch_group_t(const LaunchCfg &lc, const NNArgs &nn, const SpaceParams &sp, StatesView qv, int64_t nq, int k,
-                    int K, int CS, const int64_t *prefix, int64_t *idx, double *dist, unsigned long long *fb_list,
+                    int K, int CS, const int64_t *prefix, int64_t max_limit, int64_t *idx, double *dist, unsigned long long *fb_list,
                     unsigned long long *fb_n, RunCounters *ctr)
 {
     const int buckets = std::min(kBuckets, (2 * K + 31) / 32 * 32);
@@ -457,15 +473,15 @@ void launch_group_t(const LaunchCfg &lc, const NNArgs &nn, const SpaceParams &sp
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, knn_group_kernel<KIND, MAXF, QG, kThreads>, nn, sp, qv, nq, k, K, buckets, prefix, idx, dist,
+    cudaLaunchKernelEx(&cfg, knn_group_kernel<KIND, MAXF, QG, kThreads>, nn, sp, qv, nq, k, K, buckets, prefix, max_limit, idx, dist,
                        fb_list, fb_n, ctr);
     note_launch();
 }
 }  // namespace
 
 bool launch_knn_group(const LaunchCfg &lc, const NNArgs &nn, const SpaceParams &sp, StatesView qv, int64_t nq, int k,
-                      const int64_t *prefix, int64_t *idx, double *dist, unsigned long long *fb_list,
-                      unsigned long long *fb_n, RunCounters *ctr)
+                      const int64_t *prefix, int64_t max_limit, int64_t *idx, double *dist,
+                      unsigned long long *fb_list, unsigned long long *fb_n, RunCounters *ctr)
 {
     if (nq == 0 || k > knn_fp32_max_k(sp) || nn.size >= (1ll << 30))
         return false;
@@ -485,14 +501,14 @@ bool launch_knn_group(const LaunchCfg &lc, const NNArgs &nn, const SpaceParams &
     do                                                                                                                \
     {                                                                                                                 \
         if (QG == 1)                                                                                                  \
-            launch_group_t<KIND, MAXF, 1, 256>(lc, nn, sp, qv, nq, k, knn_keep(k), CS, prefix, idx, dist, fb_list,    \
-                                               fb_n, ctr);                                                           \
+            launch_group_t<KIND, MAXF, 1, 256>(lc, nn, sp, qv, nq, k, knn_keep(k), CS, prefix, max_limit, idx, dist,  \
+                                               fb_list, fb_n, ctr);                                                        \
         else if (threads == 256)                                                                                      \
-            launch_group_t<KIND, MAXF, 4, 256>(lc, nn, sp, qv, nq, k, knn_keep(k), CS, prefix, idx, dist, fb_list,    \
-                                               fb_n, ctr);                                                           \
+            launch_group_t<KIND, MAXF, 4, 256>(lc, nn, sp, qv, nq, k, knn_keep(k), CS, prefix, max_limit, idx, dist,  \
+                                               fb_list, fb_n, ctr);                                                        \
         else                                                                                                          \
-            launch_group_t<KIND, MAXF, 4, 128>(lc, nn, sp, qv, nq, k, knn_keep(k), CS, prefix, idx, dist, fb_list,    \
-                                               fb_n, ctr);                                                           \
+            launch_group_t<KIND, MAXF, 4, 128>(lc, nn, sp, qv, nq, k, knn_keep(k), CS, prefix, max_limit, idx, dist,  \
+                                               fb_list, fb_n, ctr);                                                        \
     } while (0)
     if (sp.kind == GBO_SPACE_KINEMATIC_CHAIN && sp.dim <= 10)
         GBO_GROUP(GBO_SPACE_KINEMATIC_CHAIN, 20);
