@@ -204,6 +204,7 @@ struct gbo_checker
     __half *clr = nullptr;
     ArmTail *tail = nullptr;  // one list per counter slot
     unsigned *test_order = nullptr;
+    unsigned long long *masks = nullptr;
     CounterRing ctr;
     int tuned_schedule = -1;
     std::mutex mu, tune_mu;
@@ -228,6 +229,8 @@ struct gbo_checker
             cudaFree(tail);
         if (test_order)
             cudaFree(test_order);
+        if (masks)
+            cudaFree(masks);
         if (host_stream)
             cudaStreamDestroy(host_stream);
     }
@@ -576,6 +579,58 @@ static gbo_status order_chain_tests(gbo_checker *c)
     CUDA_TRY(cudaMalloc(&c->test_order, order.size() * sizeof(unsigned)));
     CUDA_TRY(cudaMemcpy(c->test_order, order.data(), order.size() * sizeof(unsigned), cudaMemcpyHostToDevice));
     c->wa.test_order = c->test_order;
+    return GBO_OK;
+}
+
+// The masks of ChainMasks for a world of at most 64 finite segments.
+static gbo_status build_chain_masks(gbo_checker *c, const double *world, int n)
+{
+    const double L = c->sp.link;
+    if (n > 64 || !(L > 1e-3 && L < 1e3))
+        return GBO_OK;
+    for (int i = 0; i < 4 * n; ++i)
+        if (!(std::fabs(world[i]) < 1e3 * L))
+            return GBO_OK;
+    constexpr int G = kChainMaskCells, K = kChainMaskBins;
+    std::vector<unsigned long long> m((size_t)G * G + K, 0);
+    const double half = c->sp.dim * L * 1.01, cell = 2.0 * half / G, reach = L * 33.0 / 64.0 + cell * 0.70711 + 1e-3 * L;
+    const double eps = std::ldexp(1.0, -23);
+    // position of a direction in [0, 1): 0.5 - 0.5 cos / (|cos| + |sin|) over the half turn [0, pi)
+    auto place = [&](double t) {
+        const double x = std::cos(t), y = std::sin(t);
+        return 0.5 - 0.5 * (y < 0.0 ? -x : x) / (std::fabs(x) + std::fabs(y));
+    };
+    for (int j = 0; j < n; ++j)
+    {
+        const double dx = world[4 * j + 2] - world[4 * j], dy = world[4 * j + 3] - world[4 * j + 1];
+        const double ax = world[4 * j] - dx / 64.0, ay = world[4 * j + 1] - dy / 64.0;  // lengthened at both ends
+        const double bx = dx * (33.0 / 32.0), by = dy * (33.0 / 32.0), B = std::hypot(dx, dy);
+        for (int p = 0; p < G; ++p)
+            for (int q = 0; q < G; ++q)
+            {
+                const double x = -half + (p + 0.5) * cell - ax, y = -half + (q + 0.5) * cell - ay, b2 = bx * bx + by * by;
+                const double t = b2 > 0.0 ? std::min(1.0, std::max(0.0, (x * bx + y * by) / b2)) : 0.0;
+                if (std::hypot(x - t * bx, y - t * by) <= reach)
+                    m[(size_t)p * G + q] |= 1ull << j;
+            }
+        // |denom| = L B |sin|, 66 FLT_EPSILON against the rounding of the FP32 direction (and 1e-5 of an angle)
+        const double s = L * B > 0.0 ? 66.0 * eps / (L * B) : 2.0;
+        if (s >= 0.5)
+        {
+            for (int k = 0; k < K; ++k)
+                m[(size_t)G * G + k] |= 1ull << j;
+            continue;
+        }
+        const double d = std::asin(s) + 1e-5, phi = std::atan2(dy, dx);
+        const int k0 = (int)std::floor(place(phi - d) * K) - 1, k1 = (int)std::floor(place(phi + d) * K) + 1;
+        // increasing over the half turn; past its end the bins start again
+        const int count = (k1 - k0 + 2 * K) % K;
+        for (int k = 0; k <= count; ++k)
+            m[(size_t)G * G + ((k0 + k) % K + K) % K] |= 1ull << j;
+    }
+    CUDA_TRY(cudaMalloc(&c->masks, m.size() * sizeof(m[0])));
+    CUDA_TRY(cudaMemcpy(c->masks, m.data(), m.size() * sizeof(m[0]), cudaMemcpyHostToDevice));
+    c->wa.masks = ChainMasks{c->masks, c->masks + G * G, (float)half, (float)(G / (2.0 * half))};
     return GBO_OK;
 }
 
@@ -965,6 +1020,9 @@ gbo_status gbo_checker_create(const gbo_space *space, int kind, const double *wo
         if (b32 && sp.dim <= 31)
             if (auto st = order_chain_tests(c))
                 return cleanup(st);
+        if (b32)
+            if (auto st = build_chain_masks(c, world, (int)n_world))
+                return cleanup(st);
     }
     if (wa.kind == GBO_CHECK_DH_SPHERES)
     {
@@ -1270,6 +1328,9 @@ gbo_status gbo_check_motion(gbo_checker *c, const double *s1, const double *s2, 
         return GBO_OK;
     if (schedule == GBO_SCHEDULE_AUTO && c->wa.kind == GBO_CHECK_DH_SPHERES)
         schedule = GBO_SCHEDULE_WARP;  // one form for every schedule
+    if (schedule == GBO_SCHEDULE_AUTO && c->precision == GBO_PRECISION_FP32_GUARDED &&
+        chain_motion_lanes(lcfg(stream), c->sp, c->wa, n))
+        schedule = GBO_SCHEDULE_WARP;  // a large chain batch: its own form, nothing to tune
     if (schedule == GBO_SCHEDULE_AUTO)
     {
         std::lock_guard<std::mutex> lk(c->tune_mu);

@@ -250,6 +250,19 @@ struct __align__(16) ChainSegF32
     float x0, y0, sx, sy, lo, hi, e_den, pad;
 };
 
+// Which world segments (bits, at most 64) a chain's link may have to be tested against. The reference reports a
+// collision of a link and a segment only where |denom| >= DBL_EPSILON and the lines meet inside both, up to
+// FLT_EPSILON / |denom| beyond their ends (both sign branches of demos/KinematicChain.h:267-274). So with |denom| >=
+// 64 FLT_EPSILON the two, each lengthened by a 64th at both ends, meet: the segment passes within 33/64 of a link
+// length of the link's middle point. `cell` lists those per grid cell of the middle point, `bin` the segments whose
+// |denom| can be smaller per bin of the link's direction. Null: no masks.
+constexpr int kChainMaskCells = 64, kChainMaskBins = 1024;
+struct ChainMasks
+{
+    const unsigned long long *cell, *bin;
+    float half, inv;  // the grid covers [-half, half] on both axes
+};
+
 struct ChainGuard
 {
     float eps_dir;                      // bound on |cos/sin fp32 - fp64| of one link direction

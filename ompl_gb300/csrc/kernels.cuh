@@ -74,6 +74,7 @@ struct WorldArgs
     double hz_pos;
     double hz_dh;
     CircleGrid circles;
+    ChainMasks masks;
     // clearance grid of the DH arm's world (arm_device.cuh): clr_n^3 cells over the box of the obstacle grid
     const __half *clr;
     int clr_n;
@@ -110,6 +111,7 @@ void launch_arm_motion(const LaunchCfg &lc, int precision, const SpaceParams &sp
                        RunCounters *ctr);
 bool launch_chain_validity_warp(const LaunchCfg &lc, const SpaceParams &sp, const WorldArgs &wa, StatesView v,
                                 int64_t n, uint8_t *out, RunCounters *ctr);
+bool chain_motion_lanes(const LaunchCfg &lc, const SpaceParams &sp, const WorldArgs &wa, int64_t n);
 bool launch_chain_motion_warp(const LaunchCfg &lc, const SpaceParams &sp, const WorldArgs &wa, StatesView v1,
                               StatesView v2, int64_t n, uint8_t *ok, int32_t *fj, int32_t *nd, RunCounters *ctr);
 void launch_distance(const LaunchCfg &lc, const SpaceParams &sp, StatesView a, StatesView b, int64_t n, double *out);

@@ -209,8 +209,13 @@ __global__ void __launch_bounds__(256, 4) chain_motion_warp_kernel(const __grid_
         const ff tb = ff_add(ta, DS);
         int nd = chain_segment_count_warp(ta, tb, lane, dim, L, wa.inv_lvs32, wa.e_dist, sp.factor);
         const bool nd64 = nd < 0;
-        if (nd64)  // segment count not decided by the FP32 distance bound: the reference's FP64 count
-            nd = chain_nd64_warp(sp, v1, v2, e, lane);
+        if (nd64)
+        {
+            // not decided by the FP32 distance bound. Identical finite end points: every term of the reference's
+            // sum is exactly zero, so its count is; else the reference's FP64 count
+            const bool same = __all_sync(0xffffffffu, lane >= dim || (a64 == b64 && finite));
+            nd = same ? 0 : chain_nd64_warp(sp, v1, v2, e, lane);
+        }
         if (exact || nd64)
             ++rechecks;
         const int top = nd > 1 ? nd : 1;
@@ -265,6 +270,577 @@ __global__ void __launch_bounds__(256, 4) chain_motion_warp_kernel(const __grid_
         if (rechecks)
             atomicAdd(&ctr->rechecked, (unsigned long long)rechecks);
     }
+}
+
+// ---------------------------------------------------------------- large batches: lane per state, then warp per state
+// A warp evaluates 32 states at a time. Each lane forms its own state's links (no warp scans, all lanes busy) and
+// writes them to the warp's records; then the warp walks the test table with all lanes on the same test, 16
+// tests at a time, as long as that finds intersections: the order puts the likely ones first, so most
+// invalid states end here at about one warp instruction a state and test. The states left (valid ones mostly)
+// are finished one by one with 32 tests per round, as in chain_state_warp32. A definite intersection decides a
+// state whatever other tests say; a state with an undecided test that no definite one follows is run
+// through all tests again in rounds, where the FP64 code settles them.
+//
+// Worlds of at most 64 segments have masks (ChainMasks): a lane then tests its links against about 1.4 segments each
+// instead of all, before the rounds, and the rounds are left with the link-link and tip tests.
+//
+// Against one warp per state or edge throughout, whose kinematics, scans and edge setup keep 10 of 32 lanes
+// busy: a million states of 10 links among 32 segments 349 -> 101 us (worlds with hardly a valid state) and 367 ->
+// 171 us (0.5% valid); edges at chain_motion_lanes. Bound: the ALU pipe (the guarded test's comparisons) and, for
+// edges, the latency of the rounds at 20 warps an SM.
+struct ChainLanes
+{
+    const ChainSegF32 *w;   // world segments
+    const unsigned *tab;    // tests in order: chain_test_entry's format
+    float4 *rec;            // this warp's links: state (lane) s, link k at s * stride + k: start point, vector
+    float *edge;            // this warp's edges: rows of 32 (motion only)
+    const unsigned *first;  // link-link and tip tests (with masks)
+    int nw, n_tests, n_first, stride;
+};
+
+// Odd in float4 units: the 8 lanes of a 16-byte access phase then cover all banks
+__host__ __device__ inline int chain_lane_stride(int dim)
+{
+    return (dim + 1) | 1;
+}
+
+__device__ bool chain_lanes_setup(const SpaceParams &sp, const WorldArgs &wa, unsigned char *smem, uint64_t *bar,
+                                  RunCounters *ctr, ChainLanes &cl)
+{
+    if (!stage_bulk(smem, wa.data32, wa.bytes32, bar, &ctr->timeout, &ctr->error))
+        return false;
+    int n_self;
+    cl.w = (const ChainSegF32 *)smem;
+    cl.nw = wa.n;
+    cl.n_tests = chain_test_count(sp.dim, wa.n, n_self);
+    cl.stride = chain_lane_stride(sp.dim);
+    const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5;
+    float4 *rec = (float4 *)(smem + wa.bytes32);
+    cl.rec = rec + (size_t)warp * 32 * cl.stride;
+    unsigned *tab = (unsigned *)(rec + (size_t)warps * 32 * cl.stride);
+    unsigned *first = tab + ((cl.n_tests + 3) & ~3);
+    cl.first = first;
+    cl.n_first = wa.masks.cell ? n_self + wa.n : 0;
+    cl.edge = (float *)(first + ((cl.n_first + 3) & ~3)) + (size_t)warp * 4 * sp.dim * 32;
+    for (int t = threadIdx.x; t < cl.n_first; t += blockDim.x)
+        first[t] = t < n_self ? chain_test_entry(t, sp.dim, wa.n) : (unsigned)sp.dim | (unsigned)(t - n_self) << 8;
+    for (int t = threadIdx.x; t < cl.n_tests; t += blockDim.x)
+        tab[t] = wa.test_order ? wa.test_order[t] : chain_test_entry(t, sp.dim, wa.n);
+    cl.tab = tab;
+    if (threadIdx.x == 0)
+    {
+        chain_hz_pos = wa.hz_pos;
+        chain_hz = &ctr->hazards;
+    }
+    __syncthreads();
+    return true;
+}
+
+// One more link of the lane's state: angle th (float-float), start point x, y (moved on)
+__device__ __forceinline__ void chain_lane_link(float4 *rec, int k, ff th, float L, float &c, float &s, float &x, float &y)
+{
+    sincos_ff(th, c, s);
+    const float vx = c * L, vy = s * L;
+    rec[k] = make_float4(x, y, vx, vy);
+    x += vx;
+    y += vy;
+}
+
+// The shared walk over the table: hit / amb of the lane's state (work lanes), tests done returned.
+__device__ __forceinline__ int chain_lane_walk(const ChainLanes &cl, const ChainGuard &g, const float4 *rec, bool work,
+                                               bool masks, bool &hit, bool &amb)
+{
+    int t = 0;
+    hit = amb = false;
+    unsigned left = __ballot_sync(0xffffffffu, work);
+    while (left && t < cl.n_tests)
+    {
+        const int end = min(t + 16, cl.n_tests);
+        for (; t < end; ++t)
+        {
+            const unsigned e = cl.tab[t];
+            const float4 A = rec[chain_test_a(e)];
+            float4 Bs;
+            float lo, hi, den;
+            if (e & 0x80000000u)
+            {
+                Bs = rec[chain_test_b(e)];
+                lo = g.self_lo;
+                hi = g.self_hi;
+                den = g.self_den;
+            }
+            else
+            {
+                const ChainSegF32 ws = cl.w[chain_test_b(e)];
+                Bs = make_float4(ws.x0, ws.y0, ws.sx, ws.sy);
+                lo = ws.lo;
+                hi = ws.hi;
+                den = ws.e_den;
+            }
+            const int r = seg_intersect32(A.z, A.w, Bs.z, Bs.w, A.x - Bs.x, A.y - Bs.y, lo, hi, den);
+            hit |= r == kInvalid;
+            amb |= r == kAmbiguous;
+        }
+        hit = hit && work;
+        const unsigned now = __ballot_sync(0xffffffffu, work && !hit);
+        // a state left over costs about 250 instructions with masks (a warp's 16 tests: 650), 600 without
+        const bool stop = __popc(left) - __popc(now) < (masks ? 3 : 1);
+        left = now;
+        if (stop)
+            break;
+    }
+    return t;
+}
+
+// U tests per lane side by side (the warps are few, so each has to overlap its own latencies); act: the lane's
+// test counts. kInvalid when one of them intersects, undecided ones settled in FP64, else kValid (all lanes).
+template <int U, class Q64>
+__device__ __forceinline__ int chain_lane_tests(const ChainLanes &cl, const ChainGuard &g, const float4 *rec,
+                                                const unsigned (&e)[U], const bool (&act)[U], int lane, int n,
+                                                double L64, const double *w64, Q64 q64, bool &have64)
+{
+    int r[U];
+    bool clear = true;
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+    {
+        const bool link = e[u] & 0x80000000u;
+        const int b = chain_test_b(e[u]);
+        const float4 A = rec[chain_test_a(e[u])];
+        const float4 Bs = link ? rec[b] : *(const float4 *)&cl.w[b];
+        const float4 Bb = link ? make_float4(g.self_lo, g.self_hi, g.self_den, 0.f) : *(const float4 *)&cl.w[b].lo;
+        r[u] = seg_intersect32(A.z, A.w, Bs.z, Bs.w, A.x - Bs.x, A.y - Bs.y, Bb.x, Bb.y, Bb.z);
+        r[u] = act[u] ? r[u] : kValid;
+        clear &= r[u] == kValid;
+    }
+    if (!__ballot_sync(0xffffffffu, !clear))
+        return kValid;
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+    {
+        if (__any_sync(0xffffffffu, r[u] == kAmbiguous))
+        {
+            have64 = true;
+            // chain_round64 takes record indices: links from nw on
+            const unsigned ib = e[u] & 0x80000000u ? (unsigned)(cl.nw + chain_test_b(e[u])) : (unsigned)chain_test_b(e[u]);
+            r[u] = chain_round64(lane, n, L64, q64(lane), (unsigned)(cl.nw + chain_test_a(e[u])) | ib << 16, cl.nw, cl.nw,
+                                 r[u], w64);
+        }
+        if (__any_sync(0xffffffffu, r[u] == kInvalid))
+            return kInvalid;
+    }
+    return kValid;
+}
+
+// World segments that a link (start point and vector in `l`) may have to be tested against: those within reach of
+// its middle point, and those nearly parallel to it. All when the masks do not cover the link.
+__device__ __forceinline__ unsigned long long chain_link_mask(const ChainMasks &m, const float4 l, unsigned long long all)
+{
+    const float mx = fmaf(0.5f, l.z, l.x), my = fmaf(0.5f, l.w, l.y);
+    const float gx = (mx + m.half) * m.inv, gy = (my + m.half) * m.inv;
+    const float d = fabsf(l.z) + fabsf(l.w);
+    if (!(gx >= 0.f && gx < (float)kChainMaskCells && gy >= 0.f && gy < (float)kChainMaskCells && d > 0.f))
+        return all;
+    const float a = __fdividef(l.w < 0.f ? -l.z : l.z, d);  // cosine-like, decreasing over the half turn
+    const int bin = min(kChainMaskBins - 1, max(0, (int)((0.5f - 0.5f * a) * (float)kChainMaskBins)));
+    return __ldg(m.cell + (int)gx * kChainMaskCells + (int)gy) | __ldg(m.bin + bin);
+}
+
+// Each lane's own link-world tests by the masks (undecided lanes; the tip's tests are among the warp's rounds)
+__device__ __forceinline__ void chain_lane_world(const ChainLanes &cl, const ChainMasks &masks, const float4 *rec, int n,
+                                                 bool undecided, bool &hit, bool &amb)
+{
+    const unsigned long long all = ~0ull >> (64 - cl.nw);
+    unsigned long long m = 0;
+    float4 A = make_float4(0.f, 0.f, 0.f, 0.f);
+    int link = undecided ? 0 : n;
+    while (__any_sync(0xffffffffu, link < n || m))
+    {
+        // a lane takes its next test, from the next link that has one
+        while (!m && link < n)
+        {
+            A = rec[link++];
+            m = chain_link_mask(masks, A, all);
+        }
+        if (m)
+        {
+            const ChainSegF32 B = cl.w[__ffsll((long long)m) - 1];
+            m &= m - 1;
+            const int r = seg_intersect32(A.z, A.w, B.sx, B.sy, A.x - B.x0, A.y - B.y0, B.lo, B.hi, B.e_den);
+            amb |= r == kAmbiguous;
+            if (r == kInvalid)
+            {
+                hit = true;
+                m = 0;
+                link = n;
+            }
+        }
+    }
+}
+
+// The rest of the state in records `rec`: kInvalid or kValid in all lanes. With masks: the link-link and tip
+// tests, then (world: not done by chain_lane_world, or left undecided there) each link's own world segments,
+// several lanes a link; what is left out cannot intersect. Without
+// (more than 64 segments): the table from test `t` on (t = 0 for a state with an undecided test).
+template <class Q64>
+__device__ __forceinline__ int chain_lane_rounds(const ChainLanes &cl, const WorldArgs &wa, const float4 *rec, int t,
+                                                 bool world, int lane, int n, double L64, const double *w64, Q64 q64,
+                                                 unsigned &rechecked)
+{
+    const ChainGuard &g = wa.guard;
+    bool have64 = false;
+    int r = kValid;
+    if (wa.masks.cell)
+    {
+        const int n2 = cl.n_first;
+        for (int base = 0; base < n2 && r == kValid; base += 96)
+        {
+            unsigned e[3];
+            bool act[3];
+#pragma unroll
+            for (int u = 0; u < 3; ++u)
+            {
+                act[u] = base + 32 * u + lane < n2;
+                e[u] = cl.first[min(base + 32 * u + lane, n2 - 1)];
+            }
+            r = chain_lane_tests<3>(cl, g, rec, e, act, lane, n, L64, w64, q64, have64);
+        }
+        if (r == kValid && world)
+        {
+            const int parts = 32 / n, link = lane / parts, part = lane - link * parts;  // n <= 15: at least 2 lanes
+            const int bits = (64 + parts - 1) / parts;
+            unsigned long long m = 0;
+            if (link < n)
+                m = chain_link_mask(wa.masks, rec[link], ~0ull >> (64 - cl.nw)) >> (bits * part) & ((1ull << bits) - 1);
+            while (r == kValid && __any_sync(0xffffffffu, m != 0))
+            {
+                const bool act[1] = {m != 0};
+                const int j = act[0] ? bits * part + __ffsll((long long)m) - 1 : 0;
+                const unsigned e[1] = {(unsigned)(act[0] ? link : 0) | (unsigned)j << 8};
+                m &= m - 1;
+                r = chain_lane_tests<1>(cl, g, rec, e, act, lane, n, L64, w64, q64, have64);
+            }
+        }
+    }
+    else
+        for (int base = t; base < cl.n_tests && r == kValid; base += 96)
+        {
+            unsigned e[3];
+            bool act[3];
+#pragma unroll
+            for (int u = 0; u < 3; ++u)
+            {
+                act[u] = base + 32 * u + lane < cl.n_tests;
+                e[u] = cl.tab[min(base + 32 * u + lane, cl.n_tests - 1)];
+            }
+            r = chain_lane_tests<3>(cl, g, rec, e, act, lane, n, L64, w64, q64, have64);
+        }
+    rechecked += have64 && lane == 0;
+    return r;
+}
+
+__global__ void __launch_bounds__(128, 5) chain_validity_lane_kernel(const __grid_constant__ SpaceParams sp,
+                                                                  const __grid_constant__ WorldArgs wa,
+                                                                  const __grid_constant__ StatesView v, int64_t n,
+                                                                  uint8_t *out, RunCounters *ctr)
+{
+    extern __shared__ __align__(128) unsigned char smem[];
+    __shared__ uint64_t bar;
+    ChainLanes cl;
+    if (!chain_lanes_setup(sp, wa, smem, &bar, ctr, cl))
+        return;
+    const int lane = threadIdx.x & 31, dim = sp.dim;
+    const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    const float L = (float)sp.link;
+    const double *w64 = (const double *)wa.data64;
+    float4 *mine = cl.rec + lane * cl.stride;
+    unsigned rechecks = 0, evaluated = 0;
+    for (int64_t i0 = warp * 32; i0 < n; i0 += nwarps * 32)
+    {
+        const int64_t i = i0 + lane;
+        const bool work = i < n;
+        __syncwarp();  // the previous states' records are no longer read
+        if (work)
+        {
+            ++evaluated;
+            ff th{0.f, 0.f};
+            float c = 1.f, s = 0.f, x = 0.f, y = 0.f;
+            for (int d = 0; d < dim; ++d)
+            {
+                th = ff_add(th, split_double(v(i, d)));
+                chain_lane_link(mine, d, th, L, c, s, x, y);
+            }
+            mine[dim] = make_float4(x, y, c * 0.001f, s * 0.001f);
+        }
+        __syncwarp();
+        bool hit, amb;
+        const int t = chain_lane_walk(cl, wa.guard, mine, work, wa.masks.cell != nullptr, hit, amb);
+        if (wa.masks.cell)
+            chain_lane_world(cl, wa.masks, mine, dim, work && !hit, hit, amb);
+        unsigned left = __ballot_sync(0xffffffffu, work && !hit && (amb || t < cl.n_tests));
+        const unsigned unsure = __ballot_sync(0xffffffffu, amb);
+        while (left)
+        {
+            const int src = __ffs(left) - 1;
+            left &= left - 1;
+            auto q64 = [&](int ln) { return ln < dim ? v(i0 + src, ln) : 0.0; };
+            const int r = chain_lane_rounds(cl, wa, cl.rec + src * cl.stride, unsure >> src & 1u ? 0 : t,
+                                            unsure >> src & 1u, lane, dim,
+                                            sp.link, w64, q64, rechecks);
+            if (lane == src)
+                hit = r == kInvalid;
+        }
+        if (work)
+            out[i] = hit ? 0 : 1;
+    }
+    evaluated = __reduce_add_sync(0xffffffffu, evaluated);
+    if (lane == 0)
+    {
+        if (evaluated)
+            atomicAdd(&ctr->evaluated, (unsigned long long)evaluated);
+        if (rechecks)
+            atomicAdd(&ctr->rechecked, (unsigned long long)rechecks);
+    }
+}
+
+// Each lane owns an edge of the work queue (refilled when half are idle); with half or fewer live, the lanes
+// are spread over the live edges' next states. An edge's states are settled in order.
+__global__ void __launch_bounds__(128, 5) chain_motion_lane_kernel(const __grid_constant__ SpaceParams sp,
+                                                                const __grid_constant__ WorldArgs wa,
+                                                                const __grid_constant__ StatesView v1,
+                                                                const __grid_constant__ StatesView v2, int64_t n,
+                                                                uint8_t *ok, int32_t *first_j, int32_t *nd_out,
+                                                                RunCounters *ctr)
+{
+    extern __shared__ __align__(128) unsigned char smem[];
+    __shared__ uint64_t bar;
+    __shared__ unsigned char order[4][32];
+    ChainLanes cl;
+    if (!chain_lanes_setup(sp, wa, smem, &bar, ctr, cl))
+        return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, dim = sp.dim;
+    const float L = (float)sp.link;
+    const double *w64 = (const double *)wa.data64;
+    constexpr float kPiF = 3.14159265358979323846f;
+    float4 *mine = cl.rec + lane * cl.stride;
+    unsigned rechecks = 0, evaluated = 0;
+    int64_t e = 0;
+    int nd = 0, top = 0, next = 1, first = -1;
+    bool live = false, more = true, exact = false;
+    for (;;)
+    {
+        const unsigned idle = __ballot_sync(0xffffffffu, !live && more);
+        if (idle && (__popc(idle) >= 16 || !__any_sync(0xffffffffu, live)))
+        {
+            unsigned long long q = 0;
+            if (lane == __ffs(idle) - 1)
+                q = atomicAdd(&ctr->queue, (unsigned long long)__popc(idle));
+            q = __shfl_sync(0xffffffffu, q, __ffs(idle) - 1);
+            bool nd64 = false;
+            const bool fresh = idle >> lane & 1u;
+            if (fresh)
+            {
+                e = (int64_t)q + __popc(idle & ((1u << lane) - 1u));
+                more = e < n;
+                live = more;
+            }
+            if (fresh && live)
+            {
+                // as chain_motion_warp_kernel, joint by joint: shortest-arc differences, absolute angles of s1, their
+                // changes over the edge, and the segment count by the FP32 metric
+                exact = false;
+                bool same = true;  // identical finite end points
+                ff ta{0.f, 0.f}, DS{0.f, 0.f};
+                float dx = 0.f, dy = 0.f, dist = 0.f;
+                for (int d = 0; d < dim; ++d)
+                {
+                    const double a64 = v1(e, d), b64 = v2(e, d);
+                    const ff a = split_double(a64), b = split_double(b64);
+                    ff diff = two_sum(b.hi, -a.hi);
+                    diff = fast_two_sum(diff.hi, diff.lo + (b.lo - a.lo));
+                    const float adh = fabsf(diff.hi);
+                    const float over_pi = ((adh - kPiF) + (diff.hi < 0.f ? -diff.lo : diff.lo)) + 8.742278e-08f;
+                    const bool finite = ((__double2hiint(a64) & 0x7ff00000) != 0x7ff00000) &&
+                                        ((__double2hiint(b64) & 0x7ff00000) != 0x7ff00000);
+                    exact |= !(fabsf(over_pi) >= 1e-9f && finite);
+                    same &= a64 == b64 && finite;
+                    ff D = diff;
+                    if (over_pi > 0.f)
+                    {
+                        const float sgn = diff.hi > 0.f ? -1.f : 1.f;
+                        const ff t1 = two_sum(diff.hi, sgn * 6.28125f);
+                        const ff t2 = two_sum(t1.hi, sgn * (519505.0f / 268435456.0f));
+                        D = fast_two_sum(t2.hi, (t1.lo + t2.lo) + (diff.lo + sgn * 2.4308403e-10f));
+                    }
+                    ta = ff_add(ta, a);
+                    DS = ff_add(DS, D);
+                    cl.edge[(4 * d) * 32 + lane] = ta.hi;
+                    cl.edge[(4 * d + 1) * 32 + lane] = ta.lo;
+                    cl.edge[(4 * d + 2) * 32 + lane] = DS.hi;
+                    cl.edge[(4 * d + 3) * 32 + lane] = DS.lo;
+                    float c1, s1, c2, s2;
+                    sincos_ff(ta, c1, s1);
+                    sincos_ff(ff_add(ta, DS), c2, s2);
+                    dx += c1 - c2;
+                    dy += s1 - s2;
+                    dist += sqrtf(fmaf(dx, dx, dy * dy));
+                }
+                dist *= L;
+                const float lo = (dist - wa.e_dist) * wa.inv_lvs32 * (1.0f - 4.0f * 5.96e-8f);
+                const float hi = (dist + wa.e_dist) * wa.inv_lvs32 * (1.0f + 4.0f * 5.96e-8f);
+                const float cl_ = ceilf(lo), ch = ceilf(hi);
+                nd64 = !(lo > 0.f) || !(hi < 4.0e6f) || cl_ != ch;
+                if (!nd64)
+                    nd = (int)(sp.factor * (unsigned)cl_);
+                else if (same)
+                    nd = 0;  // every term of the reference's sum is exactly zero
+                rechecks += exact || nd64;
+                nd64 &= !same;
+            }
+            unsigned todo = __ballot_sync(0xffffffffu, nd64);
+            while (todo)
+            {
+                const int src = __ffs(todo) - 1;
+                todo &= todo - 1;
+                const int c = chain_nd64_warp(sp, v1, v2, __shfl_sync(0xffffffffu, e, src), lane);
+                if (lane == src)
+                    nd = c;
+            }
+            if (fresh && live)
+            {
+                top = nd > 1 ? nd : 1;
+                next = 1;
+                first = -1;
+            }
+        }
+        const unsigned M = __ballot_sync(0xffffffffu, live);
+        if (!M)
+        {
+            if (__any_sync(0xffffffffu, more))
+                continue;
+            break;
+        }
+        const int cnt = __popc(M), reps = 32 / cnt;
+        int owner = lane, rep = 0;
+        bool work = live;
+        if (reps > 1)
+        {
+            if (live)
+                order[warp][__popc(M & ((1u << lane) - 1u))] = (unsigned char)lane;
+            __syncwarp();
+            rep = lane / cnt;
+            owner = order[warp][lane - rep * cnt];
+            work = rep < reps;
+        }
+        const int o_next = __shfl_sync(0xffffffffu, next, owner), o_top = __shfl_sync(0xffffffffu, top, owner);
+        const int o_nd = __shfl_sync(0xffffffffu, nd, owner);
+        const int64_t o_e = __shfl_sync(0xffffffffu, e, owner);
+        const bool o_exact = __shfl_sync(0xffffffffu, (int)exact, owner);
+        work = work && o_top - o_next >= rep;
+        const int j = work ? o_next + rep : o_next;
+        __syncwarp();  // the previous states' records are no longer read
+        if (work)
+        {
+            ++evaluated;
+            const float ndf = float_of(o_nd > 0 ? o_nd : 1);
+            const float inv_hi = __frcp_rn(ndf), inv_lo = fmaf(-inv_hi, ndf, 1.0f) * inv_hi;
+            const float jf = float_of(j);
+            const float t_hi = jf * inv_hi, t_lo = fmaf(jf, inv_hi, -t_hi) + jf * inv_lo;
+            ff run{0.f, 0.f};
+            float c = 1.f, s = 0.f, x = 0.f, y = 0.f;
+            for (int d = 0; d < dim; ++d)
+            {
+                const ff ta{cl.edge[(4 * d) * 32 + owner], cl.edge[(4 * d + 1) * 32 + owner]};
+                const ff DS{cl.edge[(4 * d + 2) * 32 + owner], cl.edge[(4 * d + 3) * 32 + owner]};
+                ff th;
+                if (j == o_top)
+                    th = ff_add(ta, DS);
+                else if (o_exact)
+                    th = run = ff_add(run, split_double(motion_joint64(v1, v2, o_e, d, j, o_nd, o_top)));
+                else
+                {
+                    const float p_hi = DS.hi * t_hi;
+                    const float p_lo = fmaf(DS.hi, t_hi, -p_hi) + fmaf(DS.hi, t_lo, DS.lo * t_hi);
+                    th = ff_add(ta, {p_hi, p_lo});
+                }
+                chain_lane_link(mine, d, th, L, c, s, x, y);
+            }
+            mine[dim] = make_float4(x, y, c * 0.001f, s * 0.001f);
+        }
+        __syncwarp();
+        bool hit, amb;
+        const int t = chain_lane_walk(cl, wa.guard, mine, work, wa.masks.cell != nullptr, hit, amb);
+        if (wa.masks.cell)
+            chain_lane_world(cl, wa.masks, mine, dim, work && !hit, hit, amb);
+        // the states that are left, in order; those behind a colliding state of their edge do not matter
+        unsigned left = __ballot_sync(0xffffffffu, work && !hit && (amb || t < cl.n_tests));
+        const unsigned unsure = __ballot_sync(0xffffffffu, amb);
+        const int mate = reps > 1 ? cnt : 32;  // lanes of one owner are `mate` apart
+        while (left)
+        {
+            const int src = __ffs(left) - 1;
+            left &= left - 1;
+            // a state before it on the same edge already collides
+            const unsigned hits = __ballot_sync(0xffffffffu, hit);
+            bool behind = false;
+            for (int l = src - mate; l >= 0; l -= mate)
+                behind |= hits >> l & 1u;
+            if (behind)
+                continue;
+            const int64_t se = __shfl_sync(0xffffffffu, o_e, src);
+            const int sj = __shfl_sync(0xffffffffu, j, src), snd = __shfl_sync(0xffffffffu, o_nd, src);
+            const int stop = __shfl_sync(0xffffffffu, o_top, src);
+            auto q64 = [&](int ln) { return ln < dim ? motion_joint64(v1, v2, se, ln, sj, snd, stop) : 0.0; };
+            const int r = chain_lane_rounds(cl, wa, cl.rec + src * cl.stride, unsure >> src & 1u ? 0 : t,
+                                            unsure >> src & 1u, lane, dim,
+                                            sp.link, w64, q64, rechecks);
+            if (lane == src)
+                hit = r == kInvalid;
+        }
+        // the owner takes its states in order
+        const unsigned hits = __ballot_sync(0xffffffffu, hit && work), worked = __ballot_sync(0xffffffffu, work);
+        if (live)
+        {
+            const int rank = __popc(M & ((1u << lane) - 1u));
+            for (int i = 0; i < reps && first < 0; ++i)
+            {
+                const int l = reps > 1 ? rank + i * cnt : lane;
+                if (!(worked >> l & 1u))
+                    break;
+                if (hits >> l & 1u)
+                    first = next;
+                else
+                    ++next;
+            }
+            if (first >= 0 || next > top)
+            {
+                ok[e] = first < 0 ? 1 : 0;
+                if (first_j)
+                    first_j[e] = first < 0 ? -1 : (first == top ? nd : first);
+                if (nd_out)
+                    nd_out[e] = nd;
+                live = false;
+            }
+        }
+    }
+    evaluated = __reduce_add_sync(0xffffffffu, evaluated);
+    rechecks = __reduce_add_sync(0xffffffffu, rechecks);
+    if (lane == 0)
+    {
+        if (evaluated)
+            atomicAdd(&ctr->evaluated, (unsigned long long)evaluated);
+        if (rechecks)
+            atomicAdd(&ctr->rechecked, (unsigned long long)rechecks);
+    }
+}
+
+static unsigned chain_lane_smem(const SpaceParams &sp, const WorldArgs &wa, bool motion)
+{
+    const int m = sp.dim + 1, n_self = (m - 1) * (m - 2) / 2, n_tests = n_self + m * wa.n;
+    const int n_first = wa.masks.cell ? n_self + wa.n : 0;
+    return wa.bytes32 + 4 * 32 * chain_lane_stride(sp.dim) * 16 + (((n_tests + 3) & ~3) + ((n_first + 3) & ~3)) * 4 +
+           (motion ? 4 * 4 * sp.dim * 32 * 4 : 0);
 }
 
 // Hit bitmaps of n states (SoA FP64, ld = n) for the host's test ordering: one warp per state.
@@ -342,9 +918,36 @@ static int chain_block(const SpaceParams &sp, const WorldArgs &wa, unsigned &sm)
     return 0;
 }
 
+static bool chain_lanes_fit(const SpaceParams &sp, const WorldArgs &wa, bool motion)
+{
+    // dim <= 15: link angles of interpolated states inside sincos_ff's range, two lanes a link in the rounds
+    return sp.dim <= 15 && wa.stage32 && chain_smem_fits(chain_lane_smem(sp, wa, motion));
+}
+
+// Lane per edge once the batch fills every lane the GPU holds (97,280 at 10 links): below that a warp waits for its
+// slowest edge with few others to hide it (65,536 edges between valid states of the benchmark's world: 187 us against
+// 173 us a warp per edge; 100,000: 248 against 245; 400,000: 673 against 871; 100,000 edges that end at their first
+// state: 35 against 92).
+bool chain_motion_lanes(const LaunchCfg &lc, const SpaceParams &sp, const WorldArgs &wa, int64_t n)
+{
+    if (wa.kind != GBO_CHECK_CHAIN_SEGMENTS || n < 32768 || !chain_lanes_fit(sp, wa, true))
+        return false;
+    return n >= 128ll * persistent_grid((const void *)chain_motion_lane_kernel, 128, chain_lane_smem(sp, wa, true), lc,
+                                        INT64_MAX / 2);
+}
+
 bool launch_chain_validity_warp(const LaunchCfg &lc, const SpaceParams &sp, const WorldArgs &wa, StatesView v,
                                 int64_t n, uint8_t *out, RunCounters *ctr)
 {
+    // lanes per state from the batch on that fills them (32,768 states: the same 27 us; 65,536: 41 against 27)
+    if (n >= 32768 && chain_lanes_fit(sp, wa, false))
+    {
+        const unsigned bytes = chain_lane_smem(sp, wa, false);
+        const int grid = persistent_grid((const void *)chain_validity_lane_kernel, 128, bytes, lc, (n + 127) / 128);
+        chain_validity_lane_kernel<<<grid, 128, bytes, lc.stream>>>(sp, wa, v, n, out, ctr);
+        note_launch();
+        return true;
+    }
     unsigned sm = 0;
     const int block = sp.dim > 31 || !wa.stage32 ? 0 : chain_block(sp, wa, sm);
     if (!block)
@@ -359,6 +962,14 @@ bool launch_chain_validity_warp(const LaunchCfg &lc, const SpaceParams &sp, cons
 bool launch_chain_motion_warp(const LaunchCfg &lc, const SpaceParams &sp, const WorldArgs &wa, StatesView v1,
                               StatesView v2, int64_t n, uint8_t *ok, int32_t *fj, int32_t *nd, RunCounters *ctr)
 {
+    if (chain_motion_lanes(lc, sp, wa, n))
+    {
+        const unsigned bytes = chain_lane_smem(sp, wa, true);
+        const int grid = persistent_grid((const void *)chain_motion_lane_kernel, 128, bytes, lc, (n + 127) / 128);
+        chain_motion_lane_kernel<<<grid, 128, bytes, lc.stream>>>(sp, wa, v1, v2, n, ok, fj, nd, ctr);
+        note_launch();
+        return true;
+    }
     unsigned sm = 0;
     // link angles of interpolated states reach |theta| <= 2 dim pi, inside sincos_ff's range for dim <= 15
     const int block = sp.dim > 15 || !wa.stage32 ? 0 : chain_block(sp, wa, sm);
