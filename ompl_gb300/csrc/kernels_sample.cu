@@ -43,75 +43,110 @@ __device__ __forceinline__ double canonical53(unsigned w0, unsigned w1)
     return r;
 }
 
+// The recurrence on the stream's own index: with x_0 .. x_623 the generator's block, the next words are
+// x_n = x_(n-227) ^ f(x_(n-624), x_(n-623)), n >= 624. Thread t < 227 produces n = 624 + t, then every
+// 227th: x_(n-227) is the word it produced last (a register), and the words n and n + 227 of one step need
+// nothing later than x_(n-170), so a step makes 454 words between two barriers. The words live in a ring of
+// four steps in shared memory (word n at slot mt_slot(n)), so each thread's addresses repeat every fourth
+// step and are kept in registers. Bound by the chain barrier, load, f, store, barrier; the recurrence in
+// blocks had three barriers to 624 words (153 segments of 2^17 words: 60 us with tempering, now 25 without).
+constexpr int kMtLag = 227, kMtStep = 2 * kMtLag, kMtRing = 4 * kMtStep;
+static_assert(kMtRing >= 624 + kMtStep, "a step's inputs and outputs fit in the ring");
+
+__device__ __forceinline__ int mt_slot(int64_t n)  // n >= 0; the block's words 0 .. 623 end the ring
+{
+    return (int)((n + kMtRing - 624) % kMtRing);
+}
+
+// Words [624, make) of the stream after the block in the ring (whole steps); those below keep are stored
+// at o + n. Every thread of the CTA (at least 227) calls it; the ring is complete on return.
+template <bool kTemper>
+__device__ __forceinline__ void mt_run(unsigned *ring, int64_t make, int64_t keep, unsigned *o)
+{
+    const int t = threadIdx.x;
+    const bool act = t < kMtLag;
+    int in[4][4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+    {
+        const int at[4] = {624, 623, 397, 396};
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+        {
+            const int r = kMtStep * j + (act ? t : 0) - at[q];
+            in[j][q] = r < 0 ? r + kMtRing : r;
+        }
+    }
+    unsigned v0 = 0u, v1 = act ? ring[mt_slot(397 + t)] : 0u;
+    auto step = [&](int j) {
+        const unsigned a = ring[in[j][0]], b = ring[in[j][1]], c = ring[in[j][2]], d = ring[in[j][3]];
+        v0 = twist_word(a, b, v1);
+        v1 = twist_word(c, d, v0);
+        if (act)
+        {
+            ring[kMtStep * j + t] = v0;
+            ring[kMtStep * j + kMtLag + t] = v1;
+        }
+        __syncthreads();
+    };
+    int64_t n = 624;
+    unsigned *w = o + n + t;
+    // whole rounds without a test; a step's words are stored after its barrier, under the next step's loads
+    for (const int64_t whole = min(make, keep) - kMtRing; n <= whole; n += kMtRing, w += kMtRing)
+    {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+        {
+            step(j);
+            if (act)
+            {
+                w[kMtStep * j] = kTemper ? temper(v0) : v0;
+                w[kMtStep * j + kMtLag] = kTemper ? temper(v1) : v1;
+            }
+        }
+    }
+    for (; n < make; n += kMtRing, w += kMtRing)  // the rest: make may be up to a block beyond keep
+    {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+        {
+            if (n + kMtStep * j >= make)
+                return;
+            step(j);
+            if (act && n + kMtStep * j + t < keep)
+                w[kMtStep * j] = kTemper ? temper(v0) : v0;
+            if (act && n + kMtStep * j + kMtLag + t < keep)
+                w[kMtStep * j + kMtLag] = kTemper ? temper(v1) : v1;
+        }
+    }
+}
+
 // The word stream: one CTA continues the stream at st->pos and writes its next W tempered words to
-// out, then saves the generator. A block's regeneration runs in the three dependency-free chunks
-// [0,227), [227,454), [454,623) and word 623 into a second buffer (4 barriers per block), and each
-// word is tempered and stored as soon as its chunk produces it.
+// out, then saves the generator.
 // kRaw (speculative draws): the words are stored untempered, every new block is stored whole (up to
 // W + 623 words) and the generator is left unchanged, so that any prefix of the stream can later be
 // committed by copying the block that holds its last word (gauss_advance_kernel).
 template <bool kRaw>
 __global__ void __launch_bounds__(256) mt_words_kernel(SamplerState *st, int64_t W, unsigned *out)
 {
-    __shared__ unsigned buf[2][624];
-    unsigned *cur = buf[0], *nxt = buf[1];
+    __shared__ unsigned ring[kMtRing];
     const int t = threadIdx.x;
     for (int i = t; i < 624; i += blockDim.x)
-        cur[i] = st->mt[i];
-    int pos = (int)st->pos;  // next unused word of cur (624: none)
+        ring[mt_slot(i)] = st->mt[i];
+    const int pos = (int)st->pos;  // next unused word of the block (624: none)
     __syncthreads();
-    int64_t w = min((int64_t)(624 - pos), W);  // the rest of the current block
-    for (int i = t; i < (int)w; i += blockDim.x)
-        out[i] = kRaw ? cur[pos + i] : temper(cur[pos + i]);
-    pos += (int)w;
-    while (w < W)
-    {
-        const int m = kRaw ? 624 : (int)min((int64_t)624, W - w);  // words of the new block that are stored
-        unsigned *o = out + w;
-        if (t < 227)
-        {
-            const unsigned v = twist_word(cur[t], cur[t + 1], cur[t + 397]);
-            nxt[t] = v;
-            if (t < m)
-                o[t] = kRaw ? v : temper(v);
-        }
-        __syncthreads();
-        if (t < 227)
-        {
-            const unsigned v = twist_word(cur[t + 227], cur[t + 228], nxt[t]);
-            nxt[t + 227] = v;
-            if (t + 227 < m)
-                o[t + 227] = kRaw ? v : temper(v);
-        }
-        __syncthreads();
-        if (t < 169)
-        {
-            const unsigned v = twist_word(cur[t + 454], cur[t + 455], nxt[t + 227]);
-            nxt[t + 454] = v;
-            if (t + 454 < m)
-                o[t + 454] = kRaw ? v : temper(v);
-        }
-        __syncthreads();
-        if (t == 0)
-        {
-            const unsigned v = twist_word(cur[623], nxt[0], nxt[396]);
-            nxt[623] = v;
-            if (623 < m)
-                o[623] = kRaw ? v : temper(v);
-        }
-        __syncthreads();
-        unsigned *tmp = cur;
-        cur = nxt;
-        nxt = tmp;
-        w += m;
-        pos = m;
-    }
+    const int64_t end = pos + W;            // words [pos, end) of the stream
+    const int64_t block = (end - 1) / 624;  // the block of the last one
+    const int64_t whole = 624 * (block + 1);
+    for (int i = pos + t; i < 624 && i < end; i += blockDim.x)
+        out[i - pos] = kRaw ? ring[mt_slot(i)] : temper(ring[mt_slot(i)]);
+    mt_run<!kRaw>(ring, whole, kRaw ? whole : end, out - pos);
     if (kRaw)
         return;
     for (int i = t; i < 624; i += blockDim.x)
-        st->mt[i] = cur[i];
+        st->mt[i] = ring[mt_slot(624 * block + i)];
     if (t == 0)
-        st->pos = (unsigned)pos;
+        st->pos = (unsigned)(end - 624 * block);
 }
 
 // Values v0 .. v0 + nv - 1 of a sampling call (value v = coordinate v % dim of state v / dim) from the
@@ -191,334 +226,355 @@ void launch_sample_uniform(const LaunchCfg &lc, SamplerState *st, const SpacePar
 // canonical53, including the largest double below 1 for sums that round up to 2^64.
 __device__ __forceinline__ double canonical53_int(unsigned w0, unsigned w1)
 {
-    const unsigned long long w = ((unsigned long long)w1 << 32) | w0;
-    if (w == 0)
-        return 0.0;
-    const int z = __clzll(w);
-    const unsigned long long m = w << z;  // leading one at bit 63
-    unsigned long long mant = m >> 11;    // 53 bits
-    const unsigned rem = (unsigned)(m & 0x7ffu);
-    mant += (rem > 0x400u || (rem == 0x400u && (mant & 1ull))) ? 1ull : 0ull;
-    unsigned long long e = 1022ull - (unsigned long long)z;  // value in [2^(-1-z), 2^-z)
-    if (mant >> 53)
-    {
-        mant >>= 1;
-        e += 1;
-    }
-    if (e >= 1023ull)
-        return 0.99999999999999988897769753748;  // rounded to 1: nextafter(1, 0)
-    return __longlong_as_double((long long)((e << 52) | (mant & 0xFFFFFFFFFFFFFull)));
+    if (w1 == 0u)  // below 2^-32: the sum is exact
+        return __dmul_rn((double)w0, 5.421010862427522170037264e-20);
+    const int z = __clz((int)w1);
+    const unsigned hi = __funnelshift_l(w0, w1, z), lo = w0 << z;  // leading one at bit 63
+    // round to 53 bits, ties to even; value in [2^(-1-z), 2^-z), the leading one added to the exponent (a
+    // carry out of the mantissa makes it a power of two)
+    const unsigned inc = ((lo & 0x7ffu) + 0x3ffu + ((lo >> 11) & 1u)) >> 11;
+    const unsigned long long b = ((unsigned long long)(hi >> 11) << 32 | __funnelshift_r(lo, hi, 11)) +
+                                 ((unsigned long long)((1021u - (unsigned)z) << 20) << 32) + inc;
+    return b == 0x3ff0000000000000ull ? 0.99999999999999988897769753748  // rounded to 1: nextafter(1, 0)
+                                      : __longlong_as_double((long long)b);
 }
 
-// Coordinate d of state i of a call from generate_canonical's U.
-__device__ __forceinline__ void emit_uniform_id(int64_t i, int d, double U, const SpaceParams &sp, const double *span,
-                                                StatesView nearv, int use_near, double distance, MutStatesView out)
+// A factor prepared for span_times_canonical: its 53-bit mantissa with the leading one at bit 63 (0: not
+// a normal number, or too small for every product to be one) and the rest as the bits of a power of two.
+struct SpanFactor
 {
-    double x;
-    if (use_near)
+    unsigned mant_hi, mant_lo;
+    unsigned base;  // sign and exponent: the high word of +-2^e
+    double value;
+};
+
+__device__ __forceinline__ SpanFactor span_factor(double v)
+{
+    const unsigned long long a = (unsigned long long)__double_as_longlong(v);
+    const int e = (int)(a >> 52) & 0x7ff;
+    const bool fits = e >= 66 && e != 0x7ff;  // U is 0 or at least 2^-64
+    const unsigned long long m = fits ? (a << 11) | (1ull << 63) : 0ull;
+    return {(unsigned)(m >> 32), (unsigned)m, (unsigned)(a >> 32) & 0xfff00000u, v};
+}
+
+// RN(span * U), U = generate_canonical's value for the word pair: both roundings to 53 bits on the integer
+// pipe (an FP64 instruction holds an SM's pipe for 16 cycles). Factors that do not fit, a high word 0 and a U
+// that rounds up to a power of two go through the doubles.
+__device__ __forceinline__ double span_times_canonical(const SpanFactor &f, unsigned w0, unsigned w1)
+{
+    const int z = __clz((int)w1);
+    const unsigned mh = __funnelshift_l(w0, w1, z), ml = w0 << (z & 31);  // w1 != 0: leading one at bit 63
+    // U's mantissa: 53 bits at the top, ties to even
+    const unsigned long long u =
+        ((((unsigned long long)mh << 32) | (ml & 0xfffff800u)) +
+         (((ml & 0x7ffu) + 0x3ffu + ((ml >> 11) & 1u)) & 0x800u));
+    const unsigned uh = (unsigned)(u >> 32), ul = (unsigned)u;
+    if (w1 == 0u || uh == 0u || f.mant_hi == 0u)
+        return __dmul_rn(f.value, canonical53_int(w0, w1));
+    // the 128-bit product of the mantissas, in [2^126, 2^128); no partial sum exceeds 64 bits
+    const unsigned long long p0 = (unsigned long long)f.mant_lo * ul;
+    const unsigned long long p1 = (unsigned long long)f.mant_lo * uh + (unsigned)(p0 >> 32);
+    const unsigned long long p2 = (unsigned long long)f.mant_hi * ul + (unsigned)p1;
+    const unsigned long long p3 = (unsigned long long)f.mant_hi * uh + ((p1 >> 32) + (p2 >> 32));
+    unsigned h1 = (unsigned)(p3 >> 32), h0 = (unsigned)p3, l1 = (unsigned)p2;
+    const unsigned down = (~h1) >> 31;  // product of the mantissas below 2: one bit lower
+    h1 = __funnelshift_l(h0, h1, down);
+    h0 = __funnelshift_l(l1, h0, down);
+    l1 <<= down;
+    const unsigned sticky = (l1 | (unsigned)p0) != 0u ? 1u : 0u;
+    const unsigned inc = ((h0 & 0x7ffu) + 0x3ffu + (((h0 >> 11) & 1u) | sticky)) >> 11;
+    // span = +-2^e times its mantissa, U = 2^(-1 - z) times its own: exponent e - z - down, less one because the
+    // mantissa's leading one is added to it (a carry out of the rounded mantissa goes the same way)
+    const unsigned long long m = (((unsigned long long)(h1 >> 11) << 32) | __funnelshift_r(h0, h1, 11)) + inc;
+    const unsigned top = f.base - ((unsigned)(z + 1) << 20) - (down << 20);
+    return __longlong_as_double((long long)(m + ((unsigned long long)top << 32)));
+}
+
+// Coordinate d of state i of a sampleUniformNear call from generate_canonical's U.
+__device__ __forceinline__ double near_value(int64_t i, int d, double U, const SpaceParams &sp, StatesView nearv,
+                                             double distance)
+{
+    const double c = nearv(i, d);
+    double lo, hi;
+    if (sp.kind == GBO_SPACE_SO2)
     {
-        const double c = nearv(i, d);
-        double lo, hi;
-        if (sp.kind == GBO_SPACE_SO2)
-        {
-            lo = __dsub_rn(c, distance);
-            hi = __dadd_rn(c, distance);
-        }
-        else
-        {
-            lo = fmax(sp.low[d], __dsub_rn(c, distance));
-            hi = fmin(sp.high[d], __dadd_rn(c, distance));
-        }
-        x = __dadd_rn(__dmul_rn(__dsub_rn(hi, lo), U), lo);
-        if (sp.kind == GBO_SPACE_SO2)
-        {
-            // SO2StateSpace::enforceBounds (SO2StateSpace.cpp:79-87)
-            double y = fmod(x, 2.0 * kPi);
-            if (y < -kPi)
-                y = __dadd_rn(y, 2.0 * kPi);
-            else if (y >= kPi)
-                y = __dsub_rn(y, 2.0 * kPi);
-            x = y;
-        }
+        lo = __dsub_rn(c, distance);
+        hi = __dadd_rn(c, distance);
     }
     else
-        x = __dadd_rn(__dmul_rn(span[d], U), sp.low[d]);
-    out(i, d) = x;
+    {
+        lo = fmax(sp.low[d], __dsub_rn(c, distance));
+        hi = fmin(sp.high[d], __dadd_rn(c, distance));
+    }
+    double x = __dadd_rn(__dmul_rn(__dsub_rn(hi, lo), U), lo);
+    if (sp.kind == GBO_SPACE_SO2)
+    {
+        // SO2StateSpace::enforceBounds (SO2StateSpace.cpp:79-87)
+        double y = fmod(x, 2.0 * kPi);
+        if (y < -kPi)
+            y = __dadd_rn(y, 2.0 * kPi);
+        else if (y >= kPi)
+            y = __dsub_rn(y, 2.0 * kPi);
+        x = y;
+    }
+    return x;
 }
 
-// The next 624 raw words (nxt) after block cur: the recurrence in its three dependency-free chunks,
-// word 623 with the last one. Every thread of the CTA (at least 227) calls it.
-__device__ __forceinline__ void twist_block(const unsigned *cur, unsigned *nxt)
+// u_t = x_(T0-1+t), t < kJumpU, is what the jumps read: coefficients below 19968 + 32, words below 624
+constexpr int64_t kJumpU = 19968 + 704;
+
+// Windows of a call's nseg segments: the sampler's block and position (625 words), then words w of
+// windows 1 .. nseg - 1 at w * ldw + window - 1 (side by side, so that a warp's 32 windows share a line).
+__host__ __device__ inline int window_stride(int nseg)
 {
-    const int t = threadIdx.x;
-    if (t < 227)
-        nxt[t] = twist_word(cur[t], cur[t + 1], cur[t + 397]);
-    __syncthreads();
-    if (t < 227)
-        nxt[t + 227] = twist_word(cur[t + 227], cur[t + 228], nxt[t]);
-    __syncthreads();
-    if (t < 169)
-        nxt[t + 454] = twist_word(cur[t + 454], cur[t + 455], nxt[t + 227]);
-    else if (t == 169)
-        nxt[623] = twist_word(cur[623], nxt[0], nxt[396]);
-    __syncthreads();
+    return (nseg - 1 + 31) & ~31;
 }
 
-constexpr int64_t kJumpU = 19968 + 704;  // u words the jumps read (coefficients < 19968, words < 640 + 64)
-
-// u_t = x_(T0-1+t) for t < n (one CTA), and states[0] = the sampler's block and position.
-__global__ void __launch_bounds__(256) mt_window_seq_kernel(const SamplerState *st, int64_t n, unsigned *u,
-                                                            unsigned *state0)
+// CTA 0: u and the sampler's block; the others clear the windows that the jumps add to.
+__global__ void __launch_bounds__(256) mt_window_seq_kernel(const SamplerState *st, unsigned *u, unsigned *windows,
+                                                            int cleared)
 {
-    __shared__ unsigned buf[2][624];
-    unsigned *cur = buf[0], *nxt = buf[1];
     const int t = threadIdx.x;
+    if (blockIdx.x > 0)
+    {
+        for (int i = (blockIdx.x - 1) * 256 + t; i < cleared; i += (gridDim.x - 1) * 256)
+            windows[625 + i] = 0u;
+        return;
+    }
+    __shared__ unsigned ring[kMtRing];
+    const int pos = (int)st->pos;  // 1..624
     for (int i = t; i < 624; i += blockDim.x)
     {
-        cur[i] = st->mt[i];
-        state0[i] = cur[i];
+        const unsigned v = st->mt[i];
+        ring[mt_slot(i)] = v;
+        windows[i] = v;
+        if (i >= pos - 1)
+            u[i - (pos - 1)] = v;
     }
-    const int pos = (int)st->pos;  // 1..624
     if (t == 0)
-        state0[624] = (unsigned)pos;
+        windows[624] = (unsigned)pos;
     __syncthreads();
-    int64_t w = 625 - pos;  // u_0 .. u_(624-pos) are cur[pos-1 .. 623]
-    for (int i = t; i < w && i < n; i += blockDim.x)
-        u[i] = cur[pos - 1 + i];
-    while (w < n)
-    {
-        twist_block(cur, nxt);
-        for (int i = t; i < 624 && w + i < n; i += blockDim.x)
-            u[w + i] = nxt[i];
-        unsigned *tmp = cur;
-        cur = nxt;
-        nxt = tmp;
-        w += 624;
-        __syncthreads();
-    }
+    mt_run<false>(ring, kJumpU + pos - 1, kJumpU + pos - 1, u - (pos - 1));
 }
 
 // Windows 1..K by table lookup ("four Russians"): coefficients are taken 5 at a time (group g covers
-// i = 5g .. 5g + 4), and for each window word w the 32 XOR combinations of u[5g + w .. 5g + w + 4] are
-// tabulated once per group and shared by every window: window k adds the entry its 5 coefficient bits
-// select. A CTA of NW warps covers 8 NW window words and one range of groups for up to 32 NW windows
-// (one thread per window, 8 NW accumulators each). Entry (w, h) sits at word 33 w + h: a reader's
-// address is its h plus a constant per w, and the 32 readers of one column hit 32 banks or the same
-// word; lane (c, q) of warp p builds entries 8q .. 8q + 7 of column 8p + c, and a warp's stores of one
-// step cover 32 banks. Partial results go to states[1..K] by atomicXor (zeroed before).
+// i = 5g .. 5g + 4), and for each stream position p the 32 XOR combinations of u[p .. p + 4] are tabulated:
+// word w of a window adds, for group g, the entry of position 5g + w that the window's 5 coefficient bits
+// select. A CTA covers kJW window words, one range of groups in phases of kJGB, and up to 32 NW windows
+// (one thread per window, kJW accumulators each). The phase's groups and words share their positions:
+// 5 (kJGB - 1) + kJW tables serve kJGB kJW lookups per window, so a call of one warp of windows spends 16% of
+// its shared-memory accesses on building and one of five warps 3% (a table per group and word: 1 in 5 at
+// five warps, half of them at one). Entry h of position p sits at word 33 p + h: the 32 lanes of a lookup
+// (one p, any h) hit 32 banks or the same word, and so does a build (lane h). Bound by the lookups' shared-
+// memory wavefronts, K 624 3988 / 32 of them: 1M 10-D states (K = 152) 83 -> 60 us (74% of the
+// wavefront rate), 100,000 7-D Gaussian states (K = 55) 106 -> 28 us. Partial results go to the windows
+// (zeroed before) by atomicXor, 32 windows to a line.
 constexpr int kJG = 5;                                 // coefficients per lookup
 constexpr int kJGroups = (19937 + kJG - 1) / kJG;      // 3988 groups (bits past 19936 are zero)
+constexpr int kJGB = 16;                               // groups per phase: 80 coefficients, 2.5 words
+constexpr int kJPhases = (kJGroups + kJGB - 1) / kJGB; // 250
+constexpr int kJW = 48;                                // window words per CTA (624 = 13 * 48)
+constexpr int kJumpWarps = 20;                         // warps per SM the grid aims at
+constexpr int kJTables = kJG * (kJGB - 1) + kJW;       // positions tabulated per phase
+static_assert(kJG * kJGB * kJPhases + 624 + kJG <= kJumpU, "every position a phase tabulates is in u");
 
-// grid: (window-word chunks, ranges of qper groups, window chunks); dynamic shared memory holds the
-// range's u words (5 qper + 8 NW + 5)
+// grid: (624 / kJW, ranges of per phases, window chunks)
 template <int NW>
-__global__ void __launch_bounds__(32 * NW) mt_jump_kernel(const unsigned *u, const unsigned *polys, int K, int qper,
-                                                          unsigned *states)
+__global__ void __launch_bounds__(32 * NW) mt_jump_kernel(const unsigned *u, const unsigned *polys, int K, int ldw,
+                                                          int per, unsigned *windows)
 {
-    constexpr int TW = 8 * NW, KP = 32 * NW, GB = NW <= 5 ? 4 : 2;  // GB groups tabulated per phase
-    extern __shared__ unsigned us[];
-    __shared__ unsigned tab[2][GB][33 * TW];
-    const int w0 = blockIdx.x * TW;
-    const int g0 = blockIdx.y * qper, g1 = min(g0 + qper, kJGroups);
-    const int k0 = blockIdx.z * KP;
-    const int t = threadIdx.x, nk = min(KP, K - k0);
-    const int sl = kJG * qper + TW + kJG;
-    const int ubase = kJG * g0 + w0;
-    for (int j = t; j < sl; j += blockDim.x)
-        us[j] = ubase + j < kJumpU ? u[ubase + j] : 0u;  // words past kJumpU are never used
-    __syncthreads();
-    const int lane = t & 31, bw = 8 * (t >> 5) + (lane & 7), bq = lane >> 3;
-    // tables of groups ga .. ga + GB - 1 (those below g1) into set (ga / GB) & 1
-    auto build = [&](int ga) {
+    __shared__ unsigned tab[33 * kJTables];
+    constexpr int kPerWarp = (kJTables + NW - 1) / NW;
+    const int w0 = blockIdx.x * kJW;
+    const int p0 = blockIdx.y * per, p1 = min(p0 + per, kJPhases);
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const int k = blockIdx.z * 32 * NW + t;
+    unsigned mask[kJG];
 #pragma unroll
-        for (int e = 0; e < GB; ++e)
-        {
-            const int g = ga + e;
-            if (g >= g1)
-                break;
-            unsigned *T = tab[((ga - g0) / GB) & 1][e] + 33 * bw + 8 * bq;
-            const unsigned *x = us + kJG * (g - g0) + bw;
-            const unsigned x0 = x[0], x1 = x[1], x2 = x[2];
-            const unsigned base = ((bq & 1) ? x[3] : 0u) ^ ((bq & 2) ? x[4] : 0u);
+    for (int j = 0; j < kJG; ++j)
+        mask[j] = 0u - ((unsigned)(lane >> j) & 1u);
+    unsigned acc[kJW];
 #pragma unroll
-            for (int j = 0; j < 8; ++j)
-                T[j] = base ^ ((j & 1) ? x0 : 0u) ^ ((j & 2) ? x1 : 0u) ^ ((j & 4) ? x2 : 0u);
-        }
-    };
-    unsigned acc[TW];
-#pragma unroll
-    for (int w = 0; w < TW; ++w)
+    for (int w = 0; w < kJW; ++w)
         acc[w] = 0u;
-    // this window's coefficient words qa, qa + 1 (zero past word 623), advanced as the groups move on
-    const unsigned *crow = polys + (size_t)(k0 + min(t, nk - 1)) * 624;
-    int qa = (kJG * g0) >> 5;
-    unsigned c_lo = crow[qa], c_hi = qa + 1 < 624 ? crow[qa + 1] : 0u;
-    if (g0 < g1)
-        build(g0);
-    __syncthreads();
+    // the 80 coefficient bits of a phase start at bit 0 or 16 of word 2.5 p (zero past word 623)
+    const unsigned *crow = polys + (size_t)min(k, K - 1) * 624;
+    auto coefficients = [&](int p, unsigned(&c)[4]) {
+        const int q = (kJG * kJGB * p) >> 5;
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            c[j] = q + j < 624 ? crow[q + j] : 0u;
+    };
+    unsigned next[4];
+    coefficients(min(p0, kJPhases - 1), next);
 #pragma unroll 1
-    for (int ga = g0; ga < g1; ga += GB)
+    for (int p = p0; p < p1; ++p)
     {
-        if (ga + GB < g1)
-            build(ga + GB);
-        const unsigned(*set)[33 * TW] = tab[((ga - g0) / GB) & 1];
-#pragma unroll
-        for (int e = 0; e < GB; ++e)
+        const int sh = (p & 1) * 16;
+        const unsigned c[4] = {__funnelshift_r(next[0], next[1], sh), __funnelshift_r(next[1], next[2], sh),
+                               __funnelshift_r(next[2], next[3], sh), 0u};
+        if (p + 1 < p1)
+            coefficients(p + 1, next);
         {
-            const int g = ga + e;
-            if (g >= g1)
-                break;
-            const int b = kJG * g, q = b >> 5, sh = b & 31;
-            if (q != qa)
+            const int first = warp * kPerWarp, last = min(first + kPerWarp, kJTables);
+            const unsigned *x = u + kJG * kJGB * p + w0 + first;
+            unsigned *T = tab + 33 * first + lane;
+            unsigned r0 = x[0], r1 = x[1], r2 = x[2], r3 = x[3];
+#pragma unroll 8
+            for (int i = 0; i < last - first; ++i)
             {
-                qa = q;
-                c_lo = c_hi;
-                c_hi = qa + 1 < 624 ? crow[qa + 1] : 0u;
-            }
-            if (t < nk)
-            {
-                unsigned v = c_lo >> sh;
-                if (sh > 32 - kJG)
-                    v |= c_hi << (32 - sh);
-                const unsigned *T = set[e] + (v & 31u);
-#pragma unroll
-                for (int w = 0; w < TW; ++w)
-                    acc[w] ^= T[33 * w];
+                const unsigned r4 = x[i + 4];
+                T[33 * i] = (r0 & mask[0]) ^ (r1 & mask[1]) ^ (r2 & mask[2]) ^ (r3 & mask[3]) ^ (r4 & mask[4]);
+                r0 = r1;
+                r1 = r2;
+                r2 = r3;
+                r3 = r4;
             }
         }
         __syncthreads();
-    }
-    if (t < nk)
-    {
-        unsigned *o = states + (size_t)(k0 + t + 1) * 625 + w0;
 #pragma unroll
-        for (int w = 0; w < TW; ++w)
-            if (w0 + w < 624)
-                atomicXor(o + w, acc[w]);
+        for (int e = 0; e < kJGB; e += 2)  // two groups to one three-way XOR
+        {
+            const int b0 = kJG * e, b1 = b0 + kJG;
+            const unsigned h0 = __funnelshift_r(c[b0 >> 5], c[(b0 >> 5) + 1], b0 & 31) & 31u;
+            const unsigned h1 = __funnelshift_r(c[b1 >> 5], c[(b1 >> 5) + 1], b1 & 31) & 31u;
+            const unsigned *T0 = tab + 33 * kJG * e + h0, *T1 = tab + 33 * kJG * (e + 1) + h1;
+#pragma unroll
+            for (int w = 0; w < kJW; ++w)
+                acc[w] ^= T0[33 * w] ^ T1[33 * w];
+        }
+        __syncthreads();
+    }
+    if (k < K)
+    {
+        unsigned *o = windows + 625 + (size_t)w0 * ldw + k;
+#pragma unroll
+        for (int w = 0; w < kJW; ++w)
+            atomicXor(o + (size_t)w * ldw, acc[w]);
     }
 }
 
 template <int NW>
-static void launch_jump_t(const LaunchCfg &lc, const unsigned *u, const uint32_t *polys, int K, unsigned *states)
+static void launch_jump_t(const LaunchCfg &lc, const unsigned *u, const uint32_t *polys, int K, int ldw,
+                          unsigned *windows)
 {
-    // two CTAs per SM: the ranges of groups split the rest of the grid over 2 x SM count (four per SM
-    // measured the same: the lookups are bound by shared-memory wavefronts, not by latency)
-    const int wchunks = (624 + 8 * NW - 1) / (8 * NW), kchunks = (K + 32 * NW - 1) / (32 * NW);
-    const int ranges = std::max(1, std::min(kJGroups, (2 * lc.sm_count + wchunks * kchunks / 2) / (wchunks * kchunks)));
-    const int qper = (kJGroups + ranges - 1) / ranges;
-    const size_t smem = (size_t)(kJG * qper + 8 * NW + kJG) * sizeof(unsigned);
-    if (smem > 48 * 1024)
-        cudaFuncSetAttribute(mt_jump_kernel<NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    mt_jump_kernel<NW><<<dim3(wchunks, (kJGroups + qper - 1) / qper, kchunks), 32 * NW, smem, lc.stream>>>(
-        u, polys, K, qper, states);
+    // ranges of phases fill the SMs with up to kJumpWarps warps each (12 warps: 61 us at K = 152, 20: 60)
+    const int chunks = 624 / kJW * ((K + 32 * NW - 1) / (32 * NW));
+    const int ctas = lc.sm_count * std::max(1, kJumpWarps / NW);
+    const int ranges = std::max(1, std::min(kJPhases, ctas / chunks));
+    const int per = (kJPhases + ranges - 1) / ranges;
+    mt_jump_kernel<NW><<<dim3(624 / kJW, (kJPhases + per - 1) / per, (K + 32 * NW - 1) / (32 * NW)), 32 * NW, 0,
+                         lc.stream>>>(u, polys, K, ldw, per, windows);
 }
 
-static void launch_jump(const LaunchCfg &lc, const unsigned *u, const uint32_t *polys, int K, unsigned *states)
+// The windows of nseg segments after the sampler's next word, in scratch; returns their address.
+static const unsigned *launch_windows(const LaunchCfg &lc, const SamplerState *st, const uint32_t *polys, int nseg,
+                                      unsigned *scratch)
 {
-    switch (std::min(8, (K + 31) / 32))
+    const int K = nseg - 1, ldw = window_stride(nseg);
+    unsigned *u = scratch, *windows = scratch + kJumpU;
+    const int cleared = 624 * ldw;
+    mt_window_seq_kernel<<<1 + std::min((cleared + 1023) / 1024, lc.sm_count), 256, 0, lc.stream>>>(st, u, windows,
+                                                                                                    cleared);
+    note_launch();
+    if (K > 0)
     {
-    case 1: launch_jump_t<1>(lc, u, polys, K, states); break;
-    case 2: launch_jump_t<2>(lc, u, polys, K, states); break;
-    case 3: launch_jump_t<3>(lc, u, polys, K, states); break;
-    case 4: launch_jump_t<4>(lc, u, polys, K, states); break;
-    case 5: launch_jump_t<5>(lc, u, polys, K, states); break;
-    case 6: launch_jump_t<6>(lc, u, polys, K, states); break;
-    case 7: launch_jump_t<7>(lc, u, polys, K, states); break;
-    default: launch_jump_t<8>(lc, u, polys, K, states); break;
+        switch (std::min(8, (K + 31) / 32))
+        {
+        case 1: launch_jump_t<1>(lc, u, polys, K, ldw, windows); break;
+        case 2: launch_jump_t<2>(lc, u, polys, K, ldw, windows); break;
+        case 3: launch_jump_t<3>(lc, u, polys, K, ldw, windows); break;
+        case 4: launch_jump_t<4>(lc, u, polys, K, ldw, windows); break;
+        case 5: launch_jump_t<5>(lc, u, polys, K, ldw, windows); break;
+        case 6: launch_jump_t<6>(lc, u, polys, K, ldw, windows); break;
+        case 7: launch_jump_t<7>(lc, u, polys, K, ldw, windows); break;
+        default: launch_jump_t<8>(lc, u, polys, K, ldw, windows); break;
+        }
+        note_launch();
     }
+    return windows;
 }
 
-// One CTA per segment s: words [s L, min((s + 1) L, W)) of the call from window s, tempered and stored
-// as the recurrence produces them (word j of the call at words[j]); the last segment leaves its
-// generator in st. kRaw: the words are stored untempered and st is left unchanged (sampleGaussian's
-// speculative draws, committed afterwards).
-template <bool kRaw>
-__global__ void __launch_bounds__(256) mt_segment_kernel(SamplerState *st, const unsigned *states, int64_t L,
+// One CTA per segment s: words [s L, min((s + 1) L, W)) of the call from window s, untempered, stored as the
+// recurrence produces them (word j of the call at words[j]; tempering here took as long as the recurrence,
+// 42 us against 25 for 153 segments of 2^17 words, and a few instructions where the words are read). kSave: the
+// last segment leaves its generator in st; sampleGaussian's draws are speculative and committed afterwards.
+template <bool kSave>
+__global__ void __launch_bounds__(256) mt_segment_kernel(SamplerState *st, const unsigned *windows, int64_t L,
                                                          int64_t W, int nseg, unsigned *words)
 {
-    __shared__ unsigned buf[2][624];
-    unsigned *cur = buf[0], *nxt = buf[1];
+    __shared__ unsigned ring[kMtRing];
     const int t = threadIdx.x, s = blockIdx.x;
-    const unsigned *src = states + (size_t)s * 625;
+    const unsigned *src = s == 0 ? windows : windows + 625 + (s - 1);
+    const size_t stride = s == 0 ? 1 : (size_t)window_stride(nseg);
     for (int i = t; i < 624; i += blockDim.x)
-        cur[i] = src[i];
-    int pos = s == 0 ? (int)src[624] : 1;
-    const int64_t begin = (int64_t)s * L, len = min(begin + L, W) - begin;
-    unsigned *o = words + begin;
+        ring[mt_slot(i)] = src[i * stride];
+    const int pos = s == 0 ? (int)windows[624] : 1;
     __syncthreads();
-    int64_t w = min((int64_t)(624 - pos), len);  // the rest of the first block
-    for (int i = t; i < (int)w; i += blockDim.x)
-        o[i] = kRaw ? cur[pos + i] : temper(cur[pos + i]);
-    pos += (int)w;
-#pragma unroll 1
-    while (w < len)
-    {
-        const int m = (int)min((int64_t)624, len - w);  // words of the new block that belong to the segment
-        unsigned *ob = o + w;
-        if (t < 227)
-        {
-            const unsigned v = twist_word(cur[t], cur[t + 1], cur[t + 397]);
-            nxt[t] = v;
-            if (t < m)
-                ob[t] = kRaw ? v : temper(v);
-        }
-        __syncthreads();
-        if (t < 227)
-        {
-            const unsigned v = twist_word(cur[t + 227], cur[t + 228], nxt[t]);
-            nxt[t + 227] = v;
-            if (t + 227 < m)
-                ob[t + 227] = kRaw ? v : temper(v);
-        }
-        __syncthreads();
-        if (t < 170)
-        {
-            const unsigned v = t < 169 ? twist_word(cur[t + 454], cur[t + 455], nxt[t + 227])
-                                       : twist_word(cur[623], nxt[0], nxt[396]);
-            nxt[t + 454] = v;
-            if (t + 454 < m)
-                ob[t + 454] = kRaw ? v : temper(v);
-        }
-        __syncthreads();
-        unsigned *tmp = cur;
-        cur = nxt;
-        nxt = tmp;
-        w += m;
-        pos = m;
-    }
-    if (!kRaw && s == nseg - 1)
+    const int64_t begin = (int64_t)s * L, end = pos + min(begin + L, W) - begin;
+    const bool last = kSave && s == nseg - 1;
+    const int64_t block = (end - 1) / 624;  // the block of the segment's last word
+    unsigned *o = words + begin - pos;
+    for (int i = pos + t; i < 624 && i < end; i += blockDim.x)
+        o[i] = ring[mt_slot(i)];
+    mt_run<false>(ring, last ? 624 * (block + 1) : end, end, o);
+    if (last)
     {
         for (int i = t; i < 624; i += blockDim.x)
-            st->mt[i] = cur[i];
+            st->mt[i] = ring[mt_slot(624 * block + i)];
         if (t == 0)
-            st->pos = (unsigned)pos;
+            st->pos = (unsigned)(end - 624 * block);
     }
 }
 
-// Values v0 .. v0 + nv - 1 of the call from the stored word pairs (2m, 2m + 1), m = v - v0:
-// generate_canonical in integer arithmetic, then uniformReal (or the near bounds). state = v / dim by a
-// multiply-high with magic = ceil(2^40 / dim) (exact for v < 2^31 and dim <= 256).
+// The call's values from the stored word pairs (value v = coordinate v % dim of state v / dim from pair v):
+// tempering, generate_canonical in integer arithmetic, then uniformReal (or the near bounds), lanes over
+// consecutive values. Bound by the integer pipe and the FP64 addition; with the product on the FP64 pipe it
+// was bound there (1M 10-D states: 52 us on words already tempered, now 48 with the tempering). (Tiles of 128 states turned in shared memory, for whole
+// lines written to a coordinate-major output, took 58 us: the L2 merges the sectors, the barriers cost more.)
+template <bool kNear>
 __global__ void __launch_bounds__(256) pairs_to_states_kernel(const uint2 *pairs, int64_t nv, SpaceParams sp,
-                                                              unsigned long long magic, StatesView nearv,
-                                                              int use_near, double distance, MutStatesView out)
+                                                              StatesView nearv, double distance,
+                                                              MutStatesView out)
 {
-    __shared__ double span[GBO_MAXD];
+    __shared__ SpanFactor span[GBO_MAXD];
+    __shared__ double low[GBO_MAXD];
     for (int d = threadIdx.x; d < sp.dim; d += blockDim.x)
-        span[d] = __dsub_rn(sp.high[d], sp.low[d]);
-    __syncthreads();
-    for (int64_t m = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; m < nv; m += (int64_t)gridDim.x * blockDim.x)
     {
-        const uint2 w = pairs[m];
-        const unsigned long long v = (unsigned long long)m;
-        const int64_t i = (int64_t)__umul64hi(v << 24, magic);
-        emit_uniform_id(i, (int)(v - (unsigned long long)i * sp.dim), canonical53_int(w.x, w.y), sp, span, nearv,
-                        use_near, distance, out);
+        span[d] = span_factor(__dsub_rn(sp.high[d], sp.low[d]));
+        low[d] = sp.low[d];
+    }
+    __syncthreads();
+    // this thread's values step by the grid: state and coordinate are carried instead of divided out
+    const unsigned step = gridDim.x * blockDim.x, first = blockIdx.x * blockDim.x + threadIdx.x;
+    const int di = (int)(step / (unsigned)sp.dim), dd = (int)(step % (unsigned)sp.dim);
+    int64_t i = first / (unsigned)sp.dim;
+    int d = (int)(first % (unsigned)sp.dim);
+    double *o = &out(i, d);
+    const int64_t hop = di * out.si + dd * out.sd, wrap = out.si - sp.dim * out.sd;
+    uint2 next = first < nv ? pairs[first] : uint2{0u, 0u};
+    for (int64_t m = first; m < nv; m += step)
+    {
+        const unsigned w0 = temper(next.x), w1 = temper(next.y);
+        if (m + step < nv)
+            next = pairs[m + step];
+        *o = kNear ? near_value(i, d, canonical53_int(w0, w1), sp, nearv, distance)
+                   : __dadd_rn(span_times_canonical(span[d], w0, w1), low[d]);
+        i += di;
+        d += dd;
+        o += hop;
+        if (d >= sp.dim)
+        {
+            d -= sp.dim;
+            ++i;
+            o += wrap;
+        }
     }
 }
 
 int64_t sample_jump_words(int64_t nseg, int64_t W)
 {
-    return kJumpU + nseg * 625 + 4 + W;
+    return kJumpU + 625 + 624 * (int64_t)window_stride((int)nseg) + 4 + W;
 }
 
 void launch_sample_uniform_jump(const LaunchCfg &lc, SamplerState *st, const SpaceParams &sp, const double *near,
@@ -526,23 +582,13 @@ void launch_sample_uniform_jump(const LaunchCfg &lc, SamplerState *st, const Spa
                                 const uint32_t *polys, int64_t L, int nseg)
 {
     const int64_t values = n * sp.dim, W = 2 * values;
-    unsigned *u = scratch, *states = scratch + kJumpU, *words = states + (size_t)nseg * 625;
+    const unsigned *windows = launch_windows(lc, st, polys, nseg, scratch);
+    unsigned *words = scratch + kJumpU + 625 + 624 * (int64_t)window_stride(nseg);
     words += (4 - ((uintptr_t)words / 4) % 4) % 4;  // 16-byte aligned
-    const int K = nseg - 1;
-    if (K > 0)
-        cudaMemsetAsync(states + 625, 0, (size_t)K * 625 * sizeof(unsigned), lc.stream);
-    mt_window_seq_kernel<<<1, 256, 0, lc.stream>>>(st, kJumpU, u, states);
-    note_launch();
-    if (K > 0)
-    {
-        launch_jump(lc, u, (const unsigned *)polys, K, states);
-        note_launch();
-    }
-    mt_segment_kernel<false><<<nseg, 256, 0, lc.stream>>>(st, states, L, W, nseg, words);
-    const unsigned long long magic = ((1ull << 40) + (unsigned long long)sp.dim - 1) / (unsigned long long)sp.dim;
+    mt_segment_kernel<true><<<nseg, 256, 0, lc.stream>>>(st, windows, L, W, nseg, words);
     const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((values + 255) / 256, (int64_t)lc.sm_count * 16));
-    pairs_to_states_kernel<<<grid, 256, 0, lc.stream>>>((const uint2 *)words, values, sp, magic, nearv, near != nullptr,
-                                                        distance, out);
+    (near ? pairs_to_states_kernel<true> : pairs_to_states_kernel<false>)<<<grid, 256, 0, lc.stream>>>(
+        (const uint2 *)words, values, sp, nearv, distance, out);
     note_launch();
     note_launch();
 }
@@ -553,18 +599,8 @@ static void launch_raw_words_jump(const LaunchCfg &lc, const SamplerState *st, i
                                   unsigned *scratch, const uint32_t *polys, int64_t L)
 {
     const int nseg = (int)((W + L - 1) / L);
-    unsigned *u = scratch, *states = scratch + kJumpU;
-    const int K = nseg - 1;
-    if (K > 0)
-        cudaMemsetAsync(states + 625, 0, (size_t)K * 625 * sizeof(unsigned), lc.stream);
-    mt_window_seq_kernel<<<1, 256, 0, lc.stream>>>(st, kJumpU, u, states);
-    if (K > 0)
-    {
-        launch_jump(lc, u, polys, K, states);
-        note_launch();
-    }
-    mt_segment_kernel<true><<<nseg, 256, 0, lc.stream>>>(nullptr, states, L, W, nseg, raw);
-    note_launch();
+    const unsigned *windows = launch_windows(lc, st, polys, nseg, scratch);
+    mt_segment_kernel<false><<<nseg, 256, 0, lc.stream>>>(nullptr, windows, L, W, nseg, raw);
     note_launch();
 }
 

@@ -98,3 +98,50 @@ def test_gaussian_calls_on_segments_continue_one_stream(port):
             mi += c
     want = port.sample_script(d, 123, ops, mean, 0.4, log_mode=1)
     assert same_bits(np.vstack(got), want)
+
+
+# segment counts around the widths of the jump's window groups (32 windows a warp, 1 to 8 warps), a last
+# segment of one value, of one value less than whole, and calls just above the switch
+@pytest.mark.parametrize("words", [2 ** 18, 32 * 2 ** 15, 32 * 2 ** 15 + 2, 33 * 2 ** 15 + 2, 64 * 2 ** 15 + 2,
+                                   65 * 2 ** 15 - 2, 97 * 2 ** 15, 129 * 2 ** 15 + 4, 160 * 2 ** 15,
+                                   160 * 2 ** 15 + 2])
+@pytest.mark.parametrize("first", [1, 311, 312])
+def test_segment_counts(port, words, first):
+    d, space = rv(1)
+    smp = B.StateSampler(space, 40 + first)
+    got = [smp.sampleUniform(first), smp.sampleUniform(words // 2, soa=first == 311).reshape(-1, 1),
+           smp.sampleUniform(700)]
+    ref = port.sample_uniform(d, 40 + first, first + words // 2 + 700)
+    assert same_bits(np.vstack(got), ref)
+
+
+@pytest.mark.parametrize("dim", [2, 8, 12, 15, 16])
+@pytest.mark.parametrize("soa", [False, True])
+def test_segment_layouts(port, dim, soa):
+    """Both output orders at dimensions whose strides meet the same shared-memory banks."""
+    d, space = rv(dim)
+    smp = B.StateSampler(space, dim)
+    n = 2 ** 19 // dim + 17
+    a = smp.sampleUniform(n, soa=soa)
+    b = smp.sampleUniform(5)
+    ref = port.sample_uniform(d, dim, n + 5)
+    assert same_bits(a.T if soa else a, ref[:n]) and same_bits(b, ref[n:])
+
+
+@pytest.mark.parametrize("words", [2, 622, 624, 626, 1078, 1530, 2 ** 18 - 2])
+def test_short_calls(port, words):
+    """Calls on one CTA: ends at, before and after a block and a step of the recurrence."""
+    d, space = rv(1)
+    smp = B.StateSampler(space, words)
+    got = [smp.sampleUniform(words // 2) for _ in range(3)]
+    assert same_bits(np.vstack(got), port.sample_uniform(d, words, 3 * (words // 2)))
+
+
+def test_spans_of_every_size(port):
+    """Spans from the smallest to the largest exponents, a power of two and its neighbours."""
+    low = np.array([0.0, -1e-290, 1.0, 0.0, -4e307, -1.0, 0.0, 5.0])
+    high = np.array([1e-300, 1e-290, np.nextafter(1.0, 2.0), 4.0, 4e307, np.nextafter(1.0, 0.0), 3e-305, 1e18])
+    d = SpaceDesc(capi.SPACE_REAL_VECTOR, 8, low, high)
+    n = 2 ** 17
+    got = B.StateSampler(B.RealVectorStateSpace(8, low, high), 9).sampleUniform(n)
+    assert same_bits(got, port.sample_uniform(d, 9, n))
