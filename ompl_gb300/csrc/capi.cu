@@ -1307,9 +1307,8 @@ gbo_status gbo_is_valid(gbo_checker *c, const double *states, int64_t n, int64_t
 }
 
 static gbo_status motion_impl(gbo_checker *c, const double *s1, const double *s2, int64_t n, int64_t ld, int layout,
-                              int schedule, uint8_t *ok, int32_t *first_j, int32_t *nd, cudaStream_t stream)
+                              int schedule, uint8_t *ok, int32_t *first_j, int32_t *nd, const LaunchCfg &lc)
 {
-    LaunchCfg lc = lcfg(stream);
     RunCounters *ctr = c->ctr.take(lc.stream);
     launch_motion(lc, c->precision, schedule, c->sp, c->wa, make_view(s1, ld, layout), make_view(s2, ld, layout), n,
                   ok, first_j, nd, ctr, c->tail ? c->tail + (ctr - c->ctr.dev) * kArmTailRoom : nullptr);
@@ -1317,19 +1316,17 @@ static gbo_status motion_impl(gbo_checker *c, const double *s1, const double *s2
     return GBO_OK;
 }
 
-gbo_status gbo_check_motion(gbo_checker *c, const double *s1, const double *s2, int64_t n, int64_t ld, int layout,
-                            int schedule, uint8_t *ok, int32_t *first_j, int32_t *nd, gbo_stream stream)
+// checkMotion's schedule and launch; host_rows: s1 and s2 are page-locked host memory read in place.
+static gbo_status motion_call(gbo_checker *c, const double *s1, const double *s2, int64_t n, int64_t ld, int layout,
+                              int schedule, uint8_t *ok, int32_t *first_j, int32_t *nd, gbo_stream stream,
+                              bool host_rows)
 {
-    Trace trace("gbo_check_motion");
-    if (!c || n < 0 || (n > 0 && (!s1 || !s2 || !ok)) || !valid_layout(layout, n, ld, c->sp.dim) ||
-        schedule < GBO_SCHEDULE_PLAIN || schedule > GBO_SCHEDULE_AUTO)
-        return fail(GBO_ERR_INVALID_ARGUMENT, "bad checkMotion arguments");
-    if (n == 0)
-        return GBO_OK;
+    LaunchCfg lc = lcfg(stream);
+    lc.host_rows = host_rows;
     if (schedule == GBO_SCHEDULE_AUTO && c->wa.kind == GBO_CHECK_DH_SPHERES)
         schedule = GBO_SCHEDULE_WARP;  // one form for every schedule
     if (schedule == GBO_SCHEDULE_AUTO && c->precision == GBO_PRECISION_FP32_GUARDED &&
-        chain_motion_lanes(lcfg(stream), c->sp, c->wa, n))
+        chain_motion_lanes(lc, c->sp, c->wa, n))
         schedule = GBO_SCHEDULE_WARP;  // a large chain batch: its own form, nothing to tune
     if (schedule == GBO_SCHEDULE_AUTO)
     {
@@ -1347,10 +1344,10 @@ gbo_status gbo_check_motion(gbo_checker *c, const double *s1, const double *s2, 
             {
                 for (int rep = 0; rep < 2; ++rep)
                 {
-                    cudaEventRecord(e0, (cudaStream_t)stream);
-                    if (auto st = motion_impl(c, s1, s2, m, ld, layout, sch, ok, first_j, nd, (cudaStream_t)stream))
+                    cudaEventRecord(e0, lc.stream);
+                    if (auto st = motion_impl(c, s1, s2, m, ld, layout, sch, ok, first_j, nd, lc))
                         return st;
-                    cudaEventRecord(e1, (cudaStream_t)stream);
+                    cudaEventRecord(e1, lc.stream);
                     cudaEventSynchronize(e1);
                     float ms = 0.f;
                     cudaEventElapsedTime(&ms, e0, e1);
@@ -1367,7 +1364,19 @@ gbo_status gbo_check_motion(gbo_checker *c, const double *s1, const double *s2, 
         }
         schedule = c->tuned_schedule;
     }
-    return motion_impl(c, s1, s2, n, ld, layout, schedule, ok, first_j, nd, (cudaStream_t)stream);
+    return motion_impl(c, s1, s2, n, ld, layout, schedule, ok, first_j, nd, lc);
+}
+
+gbo_status gbo_check_motion(gbo_checker *c, const double *s1, const double *s2, int64_t n, int64_t ld, int layout,
+                            int schedule, uint8_t *ok, int32_t *first_j, int32_t *nd, gbo_stream stream)
+{
+    Trace trace("gbo_check_motion");
+    if (!c || n < 0 || (n > 0 && (!s1 || !s2 || !ok)) || !valid_layout(layout, n, ld, c->sp.dim) ||
+        schedule < GBO_SCHEDULE_PLAIN || schedule > GBO_SCHEDULE_AUTO)
+        return fail(GBO_ERR_INVALID_ARGUMENT, "bad checkMotion arguments");
+    if (n == 0)
+        return GBO_OK;
+    return motion_call(c, s1, s2, n, ld, layout, schedule, ok, first_j, nd, stream, false);
 }
 
 gbo_status gbo_last_valid(const gbo_space *s, const double *s1, const double *s2, const int32_t *first_j,
@@ -1434,14 +1443,21 @@ gbo_status gbo_is_valid_host(gbo_checker *c, const double *states, int64_t n, ui
     const size_t bin = (size_t)n * c->sp.dim * sizeof(double);
     const double *din = (const double *)mapped_host(states);
     uint8_t *dout = (uint8_t *)mapped_host(out);
-    if (!din)
+    // a lane per state would read the rows across the host link a few bytes at a time: copied first (400,000
+    // chain states: 391 us; a warp per state in place 518)
+    if (!din || (c->precision == GBO_PRECISION_FP32_GUARDED && chain_validity_lanes(c->sp, c->wa, n)))
     {
-        if (auto st = c->pin_in.reserve(bin))
-            return st;
         if (auto st = c->dev_in.reserve(bin, c->host_stream))
             return st;
-        std::memcpy(c->pin_in.p, states, bin);
-        CUDA_TRY(cudaMemcpyAsync(c->dev_in.p, c->pin_in.p, bin, cudaMemcpyHostToDevice, c->host_stream));
+        const void *src = states;
+        if (!din)
+        {
+            if (auto st = c->pin_in.reserve(bin))
+                return st;
+            std::memcpy(c->pin_in.p, states, bin);
+            src = c->pin_in.p;
+        }
+        CUDA_TRY(cudaMemcpyAsync(c->dev_in.p, src, bin, cudaMemcpyHostToDevice, c->host_stream));
         din = (const double *)c->dev_in.p;
     }
     if (!dout)
@@ -1471,8 +1487,10 @@ gbo_status gbo_check_motion_host(gbo_checker *c, const double *s1, const double 
     const size_t bst = (size_t)n * dim * sizeof(double);
     // page-locked arrays are used in place (mapped_host); the others go through device buffers
     const double *m1 = (const double *)mapped_host(s1), *m2 = (const double *)mapped_host(s2);
-    const bool in_place = m1 && m2;
-    uint8_t *mok = (uint8_t *)mapped_host(ok);
+    // the arm's lanes read their edges' rows, the chain's warps in place (chain_motion_lanes)
+    const bool arm = c->wa.kind == GBO_CHECK_DH_SPHERES;
+    const bool in_place = m1 && m2 && !arm;
+    uint8_t *mok = arm ? nullptr : (uint8_t *)mapped_host(ok);
     double *mlt = (double *)mapped_host(last_t), *mls = (double *)mapped_host(last_state);
     // device layout: [s1 | s2 (copy path)] | first_j | nd | ok | last_t | last_state
     const size_t off_fj = in_place ? 0 : 2 * bst, off_nd = off_fj + 4 * (size_t)n, off_ok = off_nd + 4 * (size_t)n;
@@ -1491,7 +1509,7 @@ gbo_status gbo_check_motion_host(gbo_checker *c, const double *s1, const double 
     uint8_t *okd = mok ? mok : (uint8_t *)(d + off_ok);
     int32_t *fj = (int32_t *)(d + off_fj), *ndv = (int32_t *)(d + off_nd);
     const int sched = c->precision == GBO_PRECISION_FP64 ? GBO_SCHEDULE_PLAIN : GBO_SCHEDULE_AUTO;
-    if (auto st = gbo_check_motion(c, m1, m2, n, dim, GBO_LAYOUT_AOS, sched, okd, fj, ndv, c->host_stream))
+    if (auto st = motion_call(c, m1, m2, n, dim, GBO_LAYOUT_AOS, sched, okd, fj, ndv, c->host_stream, in_place))
         return st;
     double *ltd = mlt ? mlt : (double *)(d + off_lt), *lsd = mls ? mls : (double *)(d + off_ls);
     if (last_t || last_state)

@@ -88,6 +88,7 @@ struct LaunchCfg
 {
     cudaStream_t stream;
     int sm_count;
+    bool host_rows = false;  // the states are read in place from page-locked host memory
 };
 
 int persistent_grid(const void *kernel, int block, unsigned smem, const LaunchCfg &lc, int64_t max_blocks);
@@ -111,6 +112,7 @@ void launch_arm_motion(const LaunchCfg &lc, int precision, const SpaceParams &sp
                        RunCounters *ctr);
 bool launch_chain_validity_warp(const LaunchCfg &lc, const SpaceParams &sp, const WorldArgs &wa, StatesView v,
                                 int64_t n, uint8_t *out, RunCounters *ctr);
+bool chain_validity_lanes(const SpaceParams &sp, const WorldArgs &wa, int64_t n);
 bool chain_motion_lanes(const LaunchCfg &lc, const SpaceParams &sp, const WorldArgs &wa, int64_t n);
 bool launch_chain_motion_warp(const LaunchCfg &lc, const SpaceParams &sp, const WorldArgs &wa, StatesView v1,
                               StatesView v2, int64_t n, uint8_t *ok, int32_t *fj, int32_t *nd, RunCounters *ctr);

@@ -927,20 +927,27 @@ static bool chain_lanes_fit(const SpaceParams &sp, const WorldArgs &wa, bool mot
 // Lane per edge once the batch fills every lane the GPU holds (97,280 at 10 links): below that a warp waits for its
 // slowest edge with few others to hide it (65,536 edges between valid states of the benchmark's world: 187 us against
 // 173 us a warp per edge; 100,000: 248 against 245; 400,000: 673 against 871; 100,000 edges that end at their first
-// state: 35 against 92).
+// state: 35 against 92). Not for rows read across the host link, where a lane's reads come a few bytes at a time
+// (100,000 edges of that world, page-locked: 270 us a warp per edge in place, 660 a lane per edge in place, 350 a
+// lane per edge after a copy to the device).
 bool chain_motion_lanes(const LaunchCfg &lc, const SpaceParams &sp, const WorldArgs &wa, int64_t n)
 {
-    if (wa.kind != GBO_CHECK_CHAIN_SEGMENTS || n < 32768 || !chain_lanes_fit(sp, wa, true))
+    if (lc.host_rows || wa.kind != GBO_CHECK_CHAIN_SEGMENTS || n < 32768 || !chain_lanes_fit(sp, wa, true))
         return false;
     return n >= 128ll * persistent_grid((const void *)chain_motion_lane_kernel, 128, chain_lane_smem(sp, wa, true), lc,
                                         INT64_MAX / 2);
 }
 
+// Lane per state from the batch on that fills them (32,768 states: the same 27 us; 65,536: 41 against 27).
+bool chain_validity_lanes(const SpaceParams &sp, const WorldArgs &wa, int64_t n)
+{
+    return wa.kind == GBO_CHECK_CHAIN_SEGMENTS && n >= 32768 && chain_lanes_fit(sp, wa, false);
+}
+
 bool launch_chain_validity_warp(const LaunchCfg &lc, const SpaceParams &sp, const WorldArgs &wa, StatesView v,
                                 int64_t n, uint8_t *out, RunCounters *ctr)
 {
-    // lanes per state from the batch on that fills them (32,768 states: the same 27 us; 65,536: 41 against 27)
-    if (n >= 32768 && chain_lanes_fit(sp, wa, false))
+    if (chain_validity_lanes(sp, wa, n))
     {
         const unsigned bytes = chain_lane_smem(sp, wa, false);
         const int grid = persistent_grid((const void *)chain_validity_lane_kernel, 128, bytes, lc, (n + 127) / 128);

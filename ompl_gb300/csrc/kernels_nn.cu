@@ -711,10 +711,9 @@ void launch_radius(const LaunchCfg &lc, const NNArgs &nn, const SpaceParams &sp,
 }
 
 // ---------------------------------------------------------------- query order (large batches)
-// A cell key per query from a few quantised features: chain metric, the tip and middle-joint points
+// A cell key per row of the chain metric from a few quantised features: the tip and middle-joint points
 // (X_i, Y_i in units of the link length: roughly mean 0 and variance (i + 1) / 2 for uniform joints,
-// 8 levels over +-2.5 standard deviations each); box and wrapped kinds, the first four coordinates over
-// their bounds (8 levels each). A counting sort by key gives the processing order.
+// 8 levels over +-2.5 standard deviations each). A counting sort by key gives the processing order.
 __device__ __forceinline__ int query_level(float v, float lo, float hi)
 {
     int l = (int)floorf((v - lo) * (8.0f / (hi - lo)));
@@ -725,29 +724,12 @@ __device__ __forceinline__ int query_level(float v, float lo, float hi)
 __device__ __forceinline__ int order_key(const SpaceParams &sp, const float *f, int64_t ld, int64_t i)
 {
     int c = 0;
-    if (sp.kind == GBO_SPACE_KINEMATIC_CHAIN)
+    const int links[2] = {sp.dim - 1, sp.dim / 2 - 1 > 0 ? sp.dim / 2 - 1 : 0};
+    for (int t = 0; t < 2; ++t)
     {
-        const int links[2] = {sp.dim - 1, sp.dim / 2 - 1 > 0 ? sp.dim / 2 - 1 : 0};
-        for (int t = 0; t < 2; ++t)
-        {
-            const float r = 2.5f * sqrtf(0.5f * (float)(links[t] + 1));
-            c = c * 64 + query_level(f[(int64_t)(2 * links[t]) * ld + i], -r, r) * 8 +
-                query_level(f[(int64_t)(2 * links[t] + 1) * ld + i], -r, r);
-        }
-    }
-    else
-    {
-        for (int d = 0; d < 4; ++d)
-        {
-            int l = 0;
-            if (d < sp.dim)
-            {
-                const float lo = sp.kind == GBO_SPACE_REAL_VECTOR ? (float)sp.low[d] : -3.14159265f;
-                const float hi = sp.kind == GBO_SPACE_REAL_VECTOR ? (float)sp.high[d] : 3.14159265f;
-                l = hi > lo ? query_level(f[(int64_t)d * ld + i], lo, hi) : 0;
-            }
-            c = c * 8 + l;
-        }
+        const float r = 2.5f * sqrtf(0.5f * (float)(links[t] + 1));
+        c = c * 64 + query_level(f[(int64_t)(2 * links[t]) * ld + i], -r, r) * 8 +
+            query_level(f[(int64_t)(2 * links[t] + 1) * ld + i], -r, r);
     }
     return c;
 }

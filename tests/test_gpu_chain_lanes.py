@@ -82,3 +82,33 @@ def test_states_and_edges(links, segments, name):
     o = port.check_motion(sd, cd, s1[:20_000], s2[:20_000], want_state=False, want_bisect=False)
     for key in ("ok", "first_j", "nd"):
         assert np.array_equal(r[key][:20_000].cpu().numpy(), o[key]), key
+
+
+@pytest.mark.parametrize("n", [32_767, 32_768, 100_003])
+def test_host_arrays(n):
+    """The host calls with page-locked and pageable arrays give the device calls' results."""
+    import ctypes as C
+
+    rng = np.random.default_rng(n)
+    world = _world(rng, 32, "sparse")
+    space = B.KinematicChainSpace(10, 0.1)
+    space.setLongestValidSegmentFraction(0.02)
+    ck = B.KinematicChainValidityChecker(space, world)
+    ck.setPrecision("fp32_guarded")
+    a, b = (torch.as_tensor(_states(rng, world, n, 10)) for _ in range(2))
+    valid = ck.isValid(a.cuda()).cpu()
+    ok = torch.empty(n, dtype=torch.uint8, device="cuda")
+    fj, nd = (torch.empty(n, dtype=torch.int32, device="cuda") for _ in range(2))
+    da, db = a.cuda(), b.cuda()
+    ptr = lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
+    capi.check(capi.lib().gbo_check_motion(ck._h, ptr(da), ptr(db), n, 10, capi.LAYOUT_AOS, capi.SCHEDULE_AUTO, ptr(ok),
+                                           ptr(fj), ptr(nd), None))
+    torch.cuda.synchronize()
+    for pin in (False, True):
+        out = torch.full((2, n), 7, dtype=torch.uint8)
+        s1, s2 = a, b
+        if pin:
+            s1, s2, out = s1.pin_memory(), s2.pin_memory(), out.pin_memory()
+        capi.check(capi.lib().gbo_is_valid_host(ck._h, ptr(s1), n, ptr(out[0])))
+        capi.check(capi.lib().gbo_check_motion_host(ck._h, ptr(s1), ptr(s2), n, ptr(out[1]), None, None))
+        assert torch.equal(out[0], valid) and torch.equal(out[1], ok.cpu())
