@@ -802,22 +802,26 @@ __device__ __forceinline__ void gauss_listed_pair(const uint4 *cand, const unsig
     pair[base + q] = make_double2(__dmul_rn(y, mult), __dmul_rn(x, mult));
 }
 
-// The pairs gauss_pairs_kernel listed, with log_med; those it cannot round go to crlist.
+// The pairs gauss_pairs_kernel listed, with log_med; those it cannot round go to crlist. Consecutive warps of
+// entries go to different CTAs: the list is a few warps an SM, and each is a serial FP64 chain (100,000 7-D
+// states, about 10,000 entries; with gauss_cr_kernel's order the call takes 199 us instead of 209).
 __global__ void __launch_bounds__(256) gauss_slow_kernel(const uint4 *cand, const unsigned short *kidx,
                                                          const unsigned *slowlist, unsigned *crlist,
                                                          GaussChunk *ctl, double2 *pair)
 {
     const long long n = ctl->slow;
-    for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x)
+    const long long w = (long long)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+    for (long long e = w * 32 + (threadIdx.x & 31); e < n; e += (long long)gridDim.x * blockDim.x)
         gauss_listed_pair(cand, kidx, pair, slowlist[e], false, crlist, ctl);
 }
 
-// The pairs gauss_slow_kernel left, with log_cr.
+// The pairs gauss_slow_kernel left, with log_cr. Consecutive entries go to different CTAs: a couple of hundred of
+// them in five warps of one SM waited for its FP64 pipe (500,000 10-D states: 17 us).
 __global__ void __launch_bounds__(256) gauss_cr_kernel(const uint4 *cand, const unsigned short *kidx,
                                                        const unsigned *crlist, GaussChunk *ctl, double2 *pair)
 {
     const long long n = ctl->slow_cr;
-    for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x)
+    for (long long e = (long long)threadIdx.x * gridDim.x + blockIdx.x; e < n; e += (long long)gridDim.x * blockDim.x)
         gauss_listed_pair(cand, kidx, pair, crlist[e], true, nullptr, ctl);
 }
 
