@@ -49,7 +49,8 @@ __device__ __forceinline__ double canonical53(unsigned w0, unsigned w1)
 // nothing later than x_(n-170), so a step makes 454 words between two barriers. The words live in a ring of
 // four steps in shared memory (word n at slot mt_slot(n)), so each thread's addresses repeat every fourth
 // step and are kept in registers. Bound by the chain barrier, load, f, store, barrier; the recurrence in
-// blocks had three barriers to 624 words (one CTA, 240,000 words: 129 -> 53 us; 153 segments of 2^17 words: 60 us with tempering, now 25 without).
+// blocks had three barriers to 624 words (one CTA, 240,000 words: 129 -> 53 us; 153 segments of 2^17 words:
+// 60 us with tempering, now 25 without).
 constexpr int kMtLag = 227, kMtStep = 2 * kMtLag, kMtRing = 4 * kMtStep;
 static_assert(kMtRing >= 624 + kMtStep, "a step's inputs and outputs fit in the ring");
 
