@@ -29,6 +29,16 @@ namespace gbo
 
 constexpr int kSubMax = 1 << 19;  // cells times sub-cells
 
+// Smallest metric distance of x from a point of [lo, hi] on the circle. The metric folds t = |x - y| to min(t, 2 pi -
+// t), which is negative from 2 pi on (elements outside [-pi, pi], an interval widened past the wrap) and counts by
+// its square: 0 where t = 0 or t = 2 pi lies between the ends, else the nearer end's magnitude.
+__device__ __forceinline__ float wrap_gap(float x, float lo, float hi)
+{
+    const float u = fabsf(x - lo), v = fabsf(x - hi);
+    const float a = fminf(u, 6.28318530717958647692f - u), b = fminf(v, 6.28318530717958647692f - v);
+    return (x >= lo && x <= hi) || a * b <= 0.f ? 0.f : fminf(fabsf(a), fabsf(b));
+}
+
 // distance from query q to the box (lo, hi per coordinate), squared, scaled down by (1 - 1e-5) against
 // the rounding of both sides
 template <int KIND, int MAXF>
@@ -45,12 +55,7 @@ __device__ __forceinline__ float bcell_lb(const float4 *b, const float *q, int d
             const float x = q[i];
             float d;
             if constexpr (KIND == GBO_SPACE_WRAP_L2 || KIND == GBO_SPACE_SO2)
-            {
-                // nearest point of [lo, hi] on the circle: 0 inside, else the nearer end
-                const float a = fabsf(x - lo[i]), c = fabsf(x - hi[i]);
-                const float wa = fminf(a, 6.28318530717958647692f - a), wc = fminf(c, 6.28318530717958647692f - c);
-                d = (x >= lo[i] && x <= hi[i]) ? 0.f : fminf(wa, wc);
-            }
+                d = wrap_gap(x, lo[i], hi[i]);
             else
                 d = fmaxf(fmaxf(lo[i] - x, x - hi[i]), 0.f);
             s = fmaf(d, d, s);
@@ -365,10 +370,7 @@ __global__ void __launch_bounds__(128, 8) knn_cell_kernel(const __grid_constant_
             b = fmaxf(b, ci.extent[2 * d + 1]);
         float s;
         if constexpr (KIND == GBO_SPACE_WRAP_L2)
-        {
-            const float u = fabsf(x - a), v = fabsf(x - b);
-            s = (x >= a && x <= b) ? 0.f : fminf(fminf(u, 6.28318530717958647692f - u), fminf(v, 6.28318530717958647692f - v));
-        }
+            s = wrap_gap(x, a, b);
         else
             s = fmaxf(fmaxf(a - x, x - b), 0.f);
         return s * s;
