@@ -366,7 +366,7 @@ __global__ void __launch_bounds__(128, 8) knn_cell_kernel(const __grid_constant_
         float a = lo + (float)l * w - pad, b = lo + (float)(l + 1) * w + pad;
         if (l == 0)
             a = fminf(a, ci.extent[2 * d]);
-        if (l == L - 1)
+        if (l == L - 1 || !(hi > lo))  // bounds that fix the coordinate: every value is in level 0
             b = fmaxf(b, ci.extent[2 * d + 1]);
         float s;
         if constexpr (KIND == GBO_SPACE_WRAP_L2)
