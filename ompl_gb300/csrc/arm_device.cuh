@@ -167,7 +167,7 @@ __device__ __forceinline__ int arm_spheres(const WorldArgs &wa, const ArmChain &
 }
 
 // The cell of an FP32 sphere centre in the obstacle grid, or -1 outside it (no obstacle near). Cells list the
-// obstacles within rs + r + 1e-3 of their box, which covers the centre's FP32 error.
+// obstacles within rs + r + a margin of their box, which covers the centre's FP32 error.
 __device__ __forceinline__ int arm_cell(const WorldArgs &wa, const float *c)
 {
     const int G = wa.grid_n;

@@ -1103,8 +1103,19 @@ gbo_status gbo_checker_create(const gbo_space *space, int kind, const double *wo
         // obstacle lies within D = rs (+ rmax) + margin + one cell diagonal of the robot sphere centre:
         // |d^2 - d_ref^2| <= 2|d| dc + dc^2 (+ rounding of d^2, rr^2). Boxes: the distance of a point
         // from a box is 1-Lipschitz per axis; each axis adds the roundings of |c - centre| - half
-        // extent and of the FP32 box (<= 40u for coordinates below 4).
-        const double margin = 1e-3;
+        // extent and of the FP32 box (<= 40u for coordinates below 4, 10u of them above).
+        // The margin covers the error of a centre's cell in FP32: dc, and 5u of the coordinates (the box's end
+        // rounded, the subtraction, the product with 64 / width). The same coordinates bound the roundings of a
+        // box.
+        double size = reach;
+        for (int64_t i = 0; i < n_world; ++i)
+            for (int r = 0; r < 3; ++r)
+            {
+                const double x = std::fabs(world[stride * i + r]) + std::fabs(world[stride * i + (boxes ? 3 + r : 3)]);
+                if (std::isfinite(x))
+                    size = std::max(size, x + sphere_radius);
+            }
+        const double margin = std::max(1e-3, 2.0 * (dc + 5.0 * u * 3.0 * size));
         const int G = 64;
         double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
         // world obstacle i: centre o(i, r), half extent h(i, r) (boxes) or radius (spheres), and the
@@ -1133,7 +1144,7 @@ gbo_status gbo_checker_create(const gbo_space *space, int kind, const double *wo
             diag2 += ((hi[r] - lo[r]) / G) * ((hi[r] - lo[r]) / G);
         }
         const double D = 1.01 * (sphere_radius + rmax + margin + std::sqrt(diag2));
-        const double dcx = boxes ? dc + 40.0 * u * std::sqrt(3.0) : dc;
+        const double dcx = boxes ? dc + 10.0 * u * std::max(4.0, size) * std::sqrt(3.0) : dc;
         const double E = 2.0 * D * dcx + dcx * dcx + 8.0 * u * D * D + 4.0 * u * (D * D);
         wa.dh_e = (float)(2.0 * E);
         // uniform 64^3 grid: a sphere is listed in every cell whose box lies within rs + ro + margin of its
