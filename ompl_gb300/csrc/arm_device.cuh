@@ -29,7 +29,7 @@ __device__ __forceinline__ float arm_clearance(const WorldArgs &wa, float x, flo
     const float dx = (gx - (ix + 0.5f)) * wa.clr_cell[0], dy = (gy - (iy + 0.5f)) * wa.clr_cell[1];
     const float dz = (gz - (iz + 0.5f)) * wa.clr_cell[2];
     const float v = __half2float(wa.clr[((int)ix * wa.clr_n + (int)iy) * wa.clr_n + (int)iz]);
-    float c = v - arm_sqrt(fmaf(dx, dx, fmaf(dy, dy, dz * dz)));
+    float c = fmaf(v, wa.clr_unit, -arm_sqrt(fmaf(dx, dx, fmaf(dy, dy, dz * dz))));
     if (fmaxf(fabsf(gx - h), fmaxf(fabsf(gy - h), fabsf(gz - h))) > h && c == c)
     {
         // outside the box: at least the distance to it plus rs

@@ -1227,7 +1227,9 @@ gbo_status gbo_checker_create(const gbo_space *space, int kind, const double *wo
                     ok &= world[6 * i + r] >= 0.0;
             for (int r = 0; r < 3; ++r)
                 scale = std::max(scale, std::max(std::fabs(lo[r]), std::fabs(hi[r])) + (hi[r] - lo[r]));
-            ok &= scale < 1e3;
+            ok &= scale < 1e15;  // its square in FP32
+            // the halves hold up to 65,504: distances are stored in units of a power of two (1 below 1e3)
+            wa.clr_unit = ok && scale >= 1e3 ? (float)std::exp2(std::ceil(std::log2(scale * 1e-3))) : 1.f;
             wa.clr_n = CG;
             for (int r = 0; r < 3; ++r)
             {

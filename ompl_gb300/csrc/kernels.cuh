@@ -79,6 +79,7 @@ struct WorldArgs
     const __half *clr;
     int clr_n;
     float clr_lo[3], clr_inv[3], clr_cell[3];
+    float clr_unit;    // the stored distances' unit
     float clr_margin;  // taken off the stored distances: FP32 error of both sides and of the positions
     float clr_out;     // a point outside the box is clear by its distance to the box plus this
     const unsigned *test_order;  // kinematic chain: segment-test order (likely intersections first)

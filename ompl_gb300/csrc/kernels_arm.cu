@@ -75,7 +75,8 @@ __global__ void __launch_bounds__(256) arm_clearance_kernel(const __grid_constan
     const float cx = lo[0] + (float)(8 * bx + 4) * cell[0], cy = lo[1] + (float)(8 * by + 4) * cell[1];
     const float cz = lo[2] + (float)(4 * bz + 2) * cell[2];
     const float hd = sqrtf(16.f * cell[0] * cell[0] + 16.f * cell[1] * cell[1] + 4.f * cell[2] * cell[2]);
-    float m = 30000.f;
+    const float most = 30000.f * wa.clr_unit;
+    float m = most;
     for (int i = t; i < wa.n; i += 256)
         m = fminf(m, obstacle_distance(wa, i, cx, cy, cz));
 #pragma unroll
@@ -101,14 +102,14 @@ __global__ void __launch_bounds__(256) arm_clearance_kernel(const __grid_constan
     const int ix = 8 * bx + t / 32, iy = 8 * by + t / 4 % 8, iz = 4 * bz + t % 4;
     const float x = lo[0] + ((float)ix + 0.5f) * cell[0], y = lo[1] + ((float)iy + 0.5f) * cell[1];
     const float z = lo[2] + ((float)iz + 0.5f) * cell[2];
-    float best = 30000.f;
+    float best = most;
     if (s_n <= kNearRoom)
         for (int k = 0; k < s_n; ++k)
             best = fminf(best, obstacle_distance(wa, near[k], x, y, z));
     else
         for (int i = 0; i < wa.n; ++i)
             best = fminf(best, obstacle_distance(wa, i, x, y, z));
-    out[(ix * G + iy) * G + iz] = __float2half_rd(fmaxf(best - wa.clr_margin, -30000.f));
+    out[(ix * G + iy) * G + iz] = __float2half_rd(fmaxf(best - wa.clr_margin, -most) / wa.clr_unit);
 }
 
 void launch_arm_clearance(const LaunchCfg &lc, const WorldArgs &wa, __half *out)

@@ -1,5 +1,5 @@
 """DH arm worlds in other units than metres: the oracle's verdicts in both precisions where FP32 positions are coarser
-than a fixed margin."""
+than a fixed margin, and clearance that proves as much as in metres."""
 import math
 
 import numpy as np
@@ -80,3 +80,17 @@ def test_contact_below_the_fp32_spacing(boxes):
         ck.setPrecision(p)
         assert np.array_equal(mv.checkMotions(s, s)["ok"], ref["ok"]), p
         assert not ck.isValid(s).any(), p
+
+
+@pytest.mark.parametrize("scale", [1e3, 1e5])
+@pytest.mark.parametrize("boxes", [False, True])
+def test_clearance_does_not_depend_on_the_unit(scale, boxes):
+    s1, s2 = _edges(3000)
+    evaluated = []
+    for f in (1.0, scale):
+        dh, world = _world(f, boxes)
+        ck = _checker(dh, world, 0.05 * f, boxes, 1.0 / 2500)
+        ck.setPrecision("fp32_guarded")
+        B.DiscreteMotionValidator(ck).checkMotions(s1, s2)
+        evaluated.append(ck.stats()["evaluated"])
+    assert evaluated[1] <= 1.1 * evaluated[0]
