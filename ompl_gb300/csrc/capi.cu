@@ -302,7 +302,7 @@ struct gbo_nn
     unsigned char *alive = nullptr;
     float eps32 = 0.f;
     NNBoxCells cells[kCellLevels];
-    int64_t pairs_seen = 0;  // query-element pairs since the element set last changed
+    int64_t forgone = 0;  // pairs above the cell search's worth that batches took without an index
     DevBuf cwork;  // scratch of the cell builds and query orders
     NNChainCells ccells;
     DevBuf qfeat, fb_list, part, qorder;
@@ -1911,7 +1911,7 @@ gbo_status gbo_nn_add(gbo_nn *nn, const double *states, int64_t n, int64_t ld, i
     nn->alive_count += n;
     for (auto &c : nn->cells)
         c.size = 0;
-    nn->pairs_seen = 0;
+    nn->forgone = 0;
     nn->ccells.valid = false;
     return GBO_OK;
 }
@@ -1925,7 +1925,7 @@ gbo_status gbo_nn_remove(gbo_nn *nn, const int64_t *keys, int64_t n, gbo_stream 
     nn->alive_count = -1;  // recounted on demand
     for (auto &c : nn->cells)
         c.size = 0;
-    nn->pairs_seen = 0;
+    nn->forgone = 0;
     nn->ccells.valid = false;
     return GBO_OK;
 }
@@ -1941,7 +1941,7 @@ gbo_status gbo_nn_clear(gbo_nn *nn)
     nn->alive_count = 0;
     for (auto &c : nn->cells)
         c.size = 0;
-    nn->pairs_seen = 0;
+    nn->forgone = 0;
     nn->ccells.valid = false;
     return GBO_OK;
 }
@@ -2066,23 +2066,29 @@ gbo_status gbo_nn_nearest_k(gbo_nn *nn, const double *q, int64_t nq, int64_t ld,
             return st;
         unsigned long long *fb_n = &ctr->queue;
         // The cell searches take batches that are worth more than their fixed cost (query order, the longest
-        // search), counted in query-element pairs. Measured cells / group kernel: 3-D, 60,000 elements, 500
-        // queries (3e7 pairs) 62 / 70 us, 4,096 queries 69 / 327 us; 5-D wrapped, 60,000 elements, 1,000 queries
-        // 121 / 178 us; 7-D, 200,000 elements, 1,000 queries (2e8) 329 / 314 us, 2,000 queries 362 / 568 us;
-        // chain, 200,000 elements, 4,096 queries (8e8) 2.37 / 2.58 ms. An index that is not built yet (0.1 to
-        // 0.3 ms) waits until the set has seen four times that many pairs.
+        // search), counted in query-element pairs. Measured, cells / group kernel: 3-D, 200,000 elements, 512
+        // queries (1e8 pairs) 102 / 162 us; wrapped 5-D, 100,000, 1,024 (1e8) 155 / 212 us; 6-D, 600,000, 256
+        // (1.5e8) 265 us by the group kernel, 512 (3e8) 249 / 482 us; wrapped 7-D, 200,000, 1,024 (2e8) 446 us by
+        // the group kernel, 2,048 (4e8) 466 / 800 us; chain, 200,000, 4,096 (8e8) 2.1 ms, 2,048 (4e8) 1.5 ms by
+        // the group kernel.
+        // An index that is not built yet costs 50 us (70,000 elements) to 95 us (600,000), what the group kernel
+        // takes for 5e7 pairs: it is built by the batch that exceeds `worth` by as much, or by the batches since
+        // the last change of the set together.
         const bool chain = nn->sp.kind == GBO_SPACE_KINEMATIC_CHAIN;
         const int dim = nn->sp.dim;
+        constexpr int64_t kBuildPairs = 50000000ll;
         const int64_t worth = chain ? 800000000ll
                                     : (dim <= 3 ? 30000000ll
                                                 : dim <= 5 ? 50000000ll
                                                            : dim == 6 ? 120000000ll : dim == 7 ? 250000000ll : 400000000ll);
-        const bool built = chain ? nn->ccells.valid : nn->cells[0].size == nn->size;
         const int64_t pairs = nq * nn->size;
-        nn->pairs_seen = std::min<int64_t>(nn->pairs_seen + pairs, 1ll << 60);
-        const bool cells = nn->size >= (chain ? 65536 : 16384) && nn->size < (1ll << 30) && nq < (1ll << 31) &&
-                           nq >= (chain ? 1024 : 64) && pairs >= worth && (chain || built || nn->pairs_seen >= 4 * worth) &&
-                           !(chain && prefix);
+        bool cells = nn->size >= (chain ? 65536 : 16384) && nn->size < (1ll << 30) && nq < (1ll << 31) &&
+                     nq >= (chain ? 1024 : 64) && pairs >= worth && !(chain && prefix);
+        if (cells && !chain && nn->cells[0].size != nn->size)
+        {
+            nn->forgone += std::min(pairs - worth, kBuildPairs);
+            cells = nn->forgone >= kBuildPairs;
+        }
         // a huge batch over a tiny index: thread per query (100 elements, 20,000 queries: 148 us against
         // 186 us wrapped, 0.62 ms against 0.91 ms on the chain)
         const bool tiny = nq >= 16384 && nn->size <= 256;

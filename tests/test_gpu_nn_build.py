@@ -1,0 +1,38 @@
+"""When nearestK builds its cell index, and a captured call's."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+if not torch.cuda.is_available():
+    pytest.skip("needs a CUDA GPU", allow_module_level=True)
+
+from ompl_gb300 import base as B  # noqa: E402
+
+PI = np.pi
+
+
+def _index(dim, size, wrap=True):
+    rng = np.random.default_rng(dim)
+    nn = B.NearestNeighborsGPU(B.WrapL2StateSpace(dim) if wrap else B.RealVectorStateSpace(dim, -PI, PI),
+                               capacity=size + 100)
+    nn.add(torch.as_tensor(rng.uniform(-PI, PI, size=(size, dim)), device="cuda"))
+    return rng, nn
+
+
+@pytest.mark.parametrize("dim,size,nq", [(2, 100_000, 1024), (3, 200_000, 1024), (5, 100_000, 1024),
+                                         (6, 600_000, 512), (7, 200_000, 4096), (8, 100_000, 8192)])
+def test_first_large_batch(dim, size, nq):
+    """The first batch that is worth an index builds it, after every change of the set."""
+    rng, nn = _index(dim, size)
+    q = torch.as_tensor(rng.uniform(-PI, PI, size=(nq, dim)), device="cuda")
+    for _ in range(2):
+        n0 = B.launch_count()
+        nn.nearestK(q, 10)
+        first = B.launch_count() - n0
+        n0 = B.launch_count()
+        nn.nearestK(q, 10)
+        again = B.launch_count() - n0
+        assert first > again > 3  # a build, then the cell search alone
+        nn.add(q[:1])
