@@ -180,6 +180,15 @@ struct DevBuf
     }
 };
 
+// Whether work enqueued on s is being captured into a graph (and does not run now)
+bool capturing(cudaStream_t s)
+{
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &st) != cudaSuccess)
+        cudaGetLastError();
+    return st != cudaStreamCaptureStatusNone;
+}
+
 size_t pad16(size_t b)
 {
     return (b + 15) & ~size_t(15);
@@ -1979,13 +1988,38 @@ static NNArgs nn_args(const gbo_nn *nn)
     return a;
 }
 
+// Prefix levels of a batch: limits in (size / 2, size] at each; without limits, and below 65,536 elements, all that
+// are left
+static int box_cell_levels(int64_t size, bool prefix)
+{
+    int n = 1;
+    while (prefix && size / 2 >= 32768 && n < kCellLevels)
+    {
+        size /= 2;
+        ++n;
+    }
+    return n;
+}
+
+// Whether the indexes that a batch searches are built
+static bool cells_built(const gbo_nn *nn, bool prefix)
+{
+    if (nn->sp.kind == GBO_SPACE_KINEMATIC_CHAIN)
+        return nn->ccells.valid;
+    int64_t size = nn->size;
+    for (int level = 0, n = box_cell_levels(size, prefix); level < n; ++level, size /= 2)
+        if (nn->cells[level].size != size)
+            return false;
+    return true;
+}
+
 // The cell search of a batch over a RealVector / wrapped gbo_nn, building the indexes it needs in stream order.
 static gbo_status box_cells_call(gbo_nn *nn, const LaunchCfg &lc, const float *qf, int64_t nq, const int64_t *prefix,
                                  int k, const KnnOut &out)
 {
     const cudaStream_t s = lc.stream;
     int64_t size = nn->size;
-    for (int level = 0; level < kCellLevels; ++level, size /= 2)
+    for (int level = 0, n = box_cell_levels(size, prefix); level < n; ++level)
     {
         NNBoxCells &c = nn->cells[level];
         KnnOut o = out;
@@ -2007,13 +2041,11 @@ static gbo_status box_cells_call(gbo_nn *nn, const LaunchCfg &lc, const float *q
             CHECK_LAUNCH();
             c.size = size;
         }
-        // limits in (size / 2, size]; without limits, and below 65,536 elements, all that are left
-        const bool last = !prefix || size / 2 < 32768 || level == kCellLevels - 1;
         launch_knn_cells(lc, c.args(), nn->sp, qf, nq, prefix, size / 2, level == 0, k, key, count, qstart, fill, qorder,
                          bs, o);
         CHECK_LAUNCH();
-        if (last)
-            break;
+        if (level + 1 < n)
+            size /= 2;
     }
     if (prefix && !launch_knn_group(lc, out.nn, nn->sp, out.qv, nq, k, prefix, size / 2, out.idx, out.dist, out.fb_list,
                                     out.fb_n, out.ctr))
@@ -2089,6 +2121,9 @@ gbo_status gbo_nn_nearest_k(gbo_nn *nn, const double *q, int64_t nq, int64_t ld,
             nn->forgone += std::min(pairs - worth, kBuildPairs);
             cells = nn->forgone >= kBuildPairs;
         }
+        // a captured call builds none: the build would run with each replay, and not before later calls
+        if (cells && capturing(lc.stream) && !cells_built(nn, prefix != nullptr))
+            cells = false;
         // a huge batch over a tiny index: thread per query (100 elements, 20,000 queries: 148 us against
         // 186 us wrapped, 0.62 ms against 0.91 ms on the chain)
         const bool tiny = nq >= 16384 && nn->size <= 256;

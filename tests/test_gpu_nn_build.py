@@ -36,3 +36,34 @@ def test_first_large_batch(dim, size, nq):
         again = B.launch_count() - n0
         assert first > again > 3  # a build, then the cell search alone
         nn.add(q[:1])
+
+
+@pytest.mark.parametrize("prefix", [False, True])
+@pytest.mark.parametrize("dim,wrap,nq", [(7, True, 4096), (3, False, 4096)])
+def test_captured_before_any_build(dim, wrap, nq, prefix):
+    """A captured call that would build the index: its replays, and direct calls made before and after them."""
+    size = 200_000
+    rng, nn = _index(dim, 1000, wrap)
+    nn = B.NearestNeighborsGPU(nn.space, capacity=size)
+    pts = torch.as_tensor(rng.uniform(-PI, PI, size=(size, dim)), device="cuda")
+    q = torch.as_tensor(rng.uniform(-PI, PI, size=(nq, dim)), device="cuda")
+    lim = torch.as_tensor(rng.integers(0, size + 1, size=nq), device="cuda") if prefix else None
+    nn.add(pts[:1000])
+    nn.nearestK(q, 10, prefix=lim)  # the call's scratch, on a set that needs no index
+    nn.add(pts[1000:])
+    nn.setPrecision("fp64")
+    want = nn.nearestK(q, 10, prefix=lim)
+    nn.setPrecision("fp32_guarded")
+    x = q.clone()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = nn.nearestK(x, 10, prefix=lim)
+    for _ in range(2):  # the first of them builds
+        got = nn.nearestK(q, 10, prefix=lim)
+        assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+    for _ in range(2):
+        out[0].fill_(-7)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out[0], want[0]) and torch.equal(out[1], want[1])
