@@ -148,9 +148,20 @@ struct Pinned
     }
 };
 
+// Whether work enqueued on s is being captured into a graph (and does not run now)
+bool capturing(cudaStream_t s)
+{
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &st) == cudaSuccess)
+        return st != cudaStreamCaptureStatusNone;
+    cudaGetLastError();  // the legacy stream beside another stream's capture
+    return false;
+}
+
 // Per-object device scratch that grows geometrically with the stream-ordered allocator. Outgrown
 // buffers are kept until the object is destroyed: freeing them during a call would synchronise the
-// whole device (cudaFree) and stall every other stream.
+// whole device (cudaFree) and stall every other stream. Grown in a call that is being captured, a buffer is
+// ordinary memory: a stream-ordered allocation would be the graph's, gone for later calls.
 struct DevBuf
 {
     void *p = nullptr;
@@ -162,7 +173,16 @@ struct DevBuf
             return GBO_OK;
         const size_t want = std::max(b, 2 * bytes);
         void *np = nullptr;
-        CUDA_TRY(cudaMallocAsync(&np, want, stream));
+        if (capturing(stream))
+        {
+            cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+            CUDA_TRY(cudaThreadExchangeStreamCaptureMode(&mode));
+            const cudaError_t e = cudaMalloc(&np, want);
+            cudaThreadExchangeStreamCaptureMode(&mode);
+            CUDA_TRY(e);
+        }
+        else
+            CUDA_TRY(cudaMallocAsync(&np, want, stream));
         if (p)
             outgrown.push_back(p);
         p = np;
@@ -179,15 +199,6 @@ struct DevBuf
             cudaFree(q);
     }
 };
-
-// Whether work enqueued on s is being captured into a graph (and does not run now)
-bool capturing(cudaStream_t s)
-{
-    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(s, &st) != cudaSuccess)
-        cudaGetLastError();
-    return st != cudaStreamCaptureStatusNone;
-}
 
 size_t pad16(size_t b)
 {

@@ -67,3 +67,25 @@ def test_captured_before_any_build(dim, wrap, nq, prefix):
         graph.replay()
         torch.cuda.synchronize()
         assert torch.equal(out[0], want[0]) and torch.equal(out[1], want[1])
+
+
+def test_scratch_grown_in_a_capture():
+    """A captured call that needs more scratch than any call before it: direct calls of its size before its first
+    replay, and replays."""
+    rng, nn = _index(7, 20_000)
+    q = torch.as_tensor(rng.uniform(-PI, PI, size=(1024, 7)), device="cuda")
+    nn.setPrecision("fp64")
+    want = nn.nearestK(q, 10)
+    nn.setPrecision("fp32_guarded")
+    nn.nearestK(q[:8].contiguous(), 10)
+    x = q.clone()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = nn.nearestK(x, 10)
+    for _ in range(2):
+        got = nn.nearestK(q, 10)
+        assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out[0], want[0]) and torch.equal(out[1], want[1])
