@@ -207,7 +207,11 @@ gbo_status gbo_nn_size(const gbo_nn *nn, int64_t *size);
  * than k elements; 1 <= k <= 64 (the FP32-guarded form covers k <= 64 on RealVector / wrapped spaces
  * of dim <= 8 and k <= 20 on the chain space; larger k there runs the FP64 scan).
  * prefix (nullable): query i only sees keys < prefix[i] (PRM insertion order).
- * dist may be NULL. distance is evaluated as distance(element, query), like NearestNeighborsLinear. */
+ * dist may be NULL. distance is evaluated as distance(element, query), like NearestNeighborsLinear.
+ * Calls on different streams and threads may overlap: the scratch belongs to the index, so the work of a
+ * call waits on the device for that of the call before it. The caller orders a search after the add /
+ * remove it is to see, and the replays of a captured call (which builds no cell index and waits for
+ * nothing) with other searches of the index. */
 gbo_status gbo_nn_nearest_k(gbo_nn *nn, const double *q, int64_t nq, int64_t ld, int layout, int k,
                             const int64_t *prefix, int64_t *idx, double *dist, gbo_stream stream);
 /* nearestR (distance <= r): counts per query, then the CSR fill given the exclusive-scan offsets. */

@@ -330,11 +330,17 @@ struct gbo_nn
     CounterRing ctr;
     unsigned long long queries = 0;
     std::mutex mu;
+    std::mutex search_mu;  // the set, its indexes and the scratch, while a call enqueues (SearchOrder)
+    cudaEvent_t searched = nullptr;
+    unsigned long long searched_on = 0;
+    bool in_flight = false;
     cudaStream_t host_stream = nullptr;
     Pinned pin;
     DevBuf dev;
     ~gbo_nn()
     {
+        if (searched)
+            cudaEventDestroy(searched);
         if (host_stream)
             cudaStreamDestroy(host_stream);
         if (pts64)
@@ -1887,7 +1893,8 @@ gbo_status gbo_nn_create(const gbo_space *space, int64_t capacity, gbo_nn **out)
     }
     cudaMemset(nn->alive, 0, capacity);
     cudaMemset(nn->outside, 0, sizeof(int));
-    if (cudaStreamCreateWithFlags(&nn->host_stream, cudaStreamNonBlocking) != cudaSuccess)
+    if (cudaStreamCreateWithFlags(&nn->host_stream, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaEventCreateWithFlags(&nn->searched, cudaEventDisableTiming) != cudaSuccess)
     {
         delete nn;
         return fail(GBO_ERR_CUDA, "stream creation failed");
@@ -1917,6 +1924,7 @@ gbo_status gbo_nn_add(gbo_nn *nn, const double *states, int64_t n, int64_t ld, i
 {
     if (!nn || n < 0 || (n > 0 && !states) || !valid_layout(layout, n, ld, nn->sp.dim))
         return fail(GBO_ERR_INVALID_ARGUMENT, "bad add arguments");
+    std::lock_guard<std::mutex> lk(nn->search_mu);
     if (nn->size + n > nn->cap)
         return fail(GBO_ERR_OUT_OF_MEMORY, "nearest-neighbour index capacity exceeded");
     if (first_key)
@@ -1940,6 +1948,7 @@ gbo_status gbo_nn_remove(gbo_nn *nn, const int64_t *keys, int64_t n, gbo_stream 
 {
     if (!nn || n < 0 || (n > 0 && !keys))
         return fail(GBO_ERR_INVALID_ARGUMENT, "bad remove arguments");
+    std::lock_guard<std::mutex> lk(nn->search_mu);
     launch_remove(lcfg(stream), keys, n, nn->size, nn->alive);
     CHECK_LAUNCH();
     nn->alive_count = -1;  // recounted on demand
@@ -1954,6 +1963,7 @@ gbo_status gbo_nn_clear(gbo_nn *nn)
 {
     if (!nn)
         return fail(GBO_ERR_INVALID_ARGUMENT, "nn is NULL");
+    std::lock_guard<std::mutex> lk(nn->search_mu);
     CUDA_TRY(cudaDeviceSynchronize());
     CUDA_TRY(cudaMemset(nn->alive, 0, nn->cap));
     CUDA_TRY(cudaMemset(nn->outside, 0, sizeof(int)));
@@ -1971,6 +1981,7 @@ gbo_status gbo_nn_size(const gbo_nn *nn, int64_t *size)
     if (!nn || !size)
         return fail(GBO_ERR_INVALID_ARGUMENT, "bad size arguments");
     auto *m = const_cast<gbo_nn *>(nn);
+    std::lock_guard<std::mutex> lk(m->search_mu);
     if (m->alive_count < 0)
     {
         std::vector<unsigned char> h(m->size);
@@ -1985,6 +1996,34 @@ gbo_status gbo_nn_size(const gbo_nn *nn, int64_t *size)
     *size = m->alive_count;
     return GBO_OK;
 }
+
+// One nearestK at a time enqueues its work, and the work of one on another stream waits for it: the cell indexes, which
+// a search may have to build, and the scratch belong to the gbo_nn. A call being captured only takes the lock (an event
+// from outside may not enter a capture): its replays are the caller's to order.
+struct SearchOrder
+{
+    gbo_nn *nn;
+    cudaStream_t s;
+    bool captured;
+    unsigned long long id = 0;
+    std::lock_guard<std::mutex> lk;
+    SearchOrder(gbo_nn *n, cudaStream_t stream) : nn(n), s(stream), captured(capturing(stream)), lk(n->search_mu)
+    {
+        if (captured)
+            return;
+        cudaStreamGetId(s, &id);
+        if (nn->in_flight && id != nn->searched_on)
+            cudaStreamWaitEvent(s, nn->searched, 0);
+    }
+    ~SearchOrder()
+    {
+        if (captured)
+            return;
+        cudaEventRecord(nn->searched, s);
+        nn->searched_on = id;
+        nn->in_flight = true;
+    }
+};
 
 static NNArgs nn_args(const gbo_nn *nn)
 {
@@ -2099,6 +2138,7 @@ gbo_status gbo_nn_nearest_k(gbo_nn *nn, const double *q, int64_t nq, int64_t ld,
     if (nq == 0)
         return GBO_OK;
     LaunchCfg lc = lcfg(stream);
+    const SearchOrder order(nn, lc.stream);
     NNArgs a = nn_args(nn);
     StatesView qv = make_view(q, ld, layout);
     RunCounters *ctr = nn->ctr.take(lc.stream);
@@ -2133,7 +2173,7 @@ gbo_status gbo_nn_nearest_k(gbo_nn *nn, const double *q, int64_t nq, int64_t ld,
             cells = nn->forgone >= kBuildPairs;
         }
         // a captured call builds none: the build would run with each replay, and not before later calls
-        if (cells && capturing(lc.stream) && !cells_built(nn, prefix != nullptr))
+        if (cells && order.captured && !cells_built(nn, prefix != nullptr))
             cells = false;
         // a huge batch over a tiny index: thread per query (100 elements, 20,000 queries: 148 us against
         // 186 us wrapped, 0.62 ms against 0.91 ms on the chain)
@@ -2216,6 +2256,7 @@ gbo_status gbo_nn_nearest_k(gbo_nn *nn, const double *q, int64_t nq, int64_t ld,
 static void radius_call(gbo_nn *nn, StatesView qv, int64_t nq, double r, int64_t *counts, const int64_t *offsets,
                         int64_t *idx, double *dist, gbo_stream stream)
 {
+    std::lock_guard<std::mutex> lk(nn->search_mu);
     NNArgs a = nn_args(nn);
     if (nn->alive_count == nn->size)
         a.alive = nullptr;
