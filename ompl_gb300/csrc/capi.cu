@@ -1568,6 +1568,24 @@ gbo_status gbo_check_motion_host(gbo_checker *c, const double *s1, const double 
     return GBO_OK;
 }
 
+// The buffers of a call below: before they are another call's, what it enqueued on them is done, also where it returns
+// early with an error.
+struct RowsInFlight
+{
+    cudaStream_t s;
+    bool done = false;
+    ~RowsInFlight()
+    {
+        if (!done)
+            cudaStreamSynchronize(s);
+    }
+    cudaError_t wait()
+    {
+        done = true;
+        return cudaStreamSynchronize(s);
+    }
+};
+
 // Small batches in host memory on the caller's stream (ordered after its earlier work, unlike the *_host
 // calls' own stream): one copy in, the kernels, one copy out through the object's page-locked buffer.
 gbo_status gbo_is_valid_rows(gbo_checker *c, const double *states, int64_t n, uint8_t *out, gbo_stream stream)
@@ -1584,12 +1602,13 @@ gbo_status gbo_is_valid_rows(gbo_checker *c, const double *states, int64_t n, ui
     if (auto e = c->dev_in.reserve(bin + (size_t)n, st))
         return e;
     char *h = (char *)c->pin_in.p, *d = (char *)c->dev_in.p;
+    RowsInFlight flight{st};
     std::memcpy(h, states, bin);
     CUDA_TRY(cudaMemcpyAsync(d, h, bin, cudaMemcpyHostToDevice, st));
     if (auto e = gbo_is_valid(c, (const double *)d, n, c->sp.dim, GBO_LAYOUT_AOS, (uint8_t *)d + bin, stream))
         return e;
     CUDA_TRY(cudaMemcpyAsync(h + bin, d + bin, (size_t)n, cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(cudaStreamSynchronize(st));
+    CUDA_TRY(flight.wait());
     std::memcpy(out, h + bin, (size_t)n);
     return GBO_OK;
 }
@@ -1610,6 +1629,7 @@ gbo_status gbo_check_motion_rows(gbo_checker *c, const double *s1, const double 
     if (auto e = c->dev_in.reserve(2 * bst + out, st))
         return e;
     char *h = (char *)c->pin_in.p, *d = (char *)c->dev_in.p;
+    RowsInFlight flight{st};
     std::memcpy(h, s1, bst);
     std::memcpy(h + bst, s2, bst);
     CUDA_TRY(cudaMemcpyAsync(d, h, 2 * bst, cudaMemcpyHostToDevice, st));
@@ -1619,7 +1639,7 @@ gbo_status gbo_check_motion_rows(gbo_checker *c, const double *s1, const double 
                                   okd, fj, ndv, stream))
         return e;
     CUDA_TRY(cudaMemcpyAsync(h + 2 * bst, d + 2 * bst, out, cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(cudaStreamSynchronize(st));
+    CUDA_TRY(flight.wait());
     std::memcpy(first_j, h + 2 * bst, 4 * (size_t)n);
     std::memcpy(nd, h + 2 * bst + 4 * (size_t)n, 4 * (size_t)n);
     std::memcpy(ok, h + 2 * bst + 8 * (size_t)n, (size_t)n);
@@ -2443,6 +2463,8 @@ gbo_status gbo_nn_nearest_k_rows(gbo_nn *nn, const double *q, int64_t nq, int k,
 {
     if (!nn || nq < 0 || k < 1 || (nq > 0 && (!q || !idx || !dist)))
         return fail(GBO_ERR_INVALID_ARGUMENT, "bad nearestK arguments");
+    if (k > 64)
+        return fail(GBO_ERR_UNSUPPORTED, "nearestK supports k <= 64");
     if (nq == 0)
         return GBO_OK;
     const cudaStream_t st = (cudaStream_t)stream;
@@ -2453,13 +2475,14 @@ gbo_status gbo_nn_nearest_k_rows(gbo_nn *nn, const double *q, int64_t nq, int k,
     if (auto e = nn->dev.reserve(bq + 2 * bo, st))
         return e;
     char *h = (char *)nn->pin.p, *d = (char *)nn->dev.p;
+    RowsInFlight flight{st};
     std::memcpy(h, q, bq);
     CUDA_TRY(cudaMemcpyAsync(d, h, bq, cudaMemcpyHostToDevice, st));
     if (auto e = gbo_nn_nearest_k(nn, (const double *)d, nq, nn->sp.dim, GBO_LAYOUT_AOS, k, nullptr,
                                   (int64_t *)(d + bq), (double *)(d + bq + bo), stream))
         return e;
     CUDA_TRY(cudaMemcpyAsync(h + bq, d + bq, 2 * bo, cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(cudaStreamSynchronize(st));
+    CUDA_TRY(flight.wait());
     std::memcpy(idx, h + bq, bo);
     std::memcpy(dist, h + bq + bo, bo);
     return GBO_OK;
