@@ -4,9 +4,11 @@
 #include <atomic>
 #include <cmath>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -200,6 +202,100 @@ struct DevBuf
     }
 };
 
+// Staging of the *_rows calls: buffers per call in flight, so that a thread waiting for its stream holds up no other.
+// As many as calls have overlapped, freed with the object. Page-locked memory is made by a call that overlaps none, and
+// at once as large as a small batch can need: making it waits for all the device's work.
+constexpr size_t kRowBytes = 128 * 1024;
+struct RowBuffers
+{
+    Pinned pin;
+    void *plain = nullptr;
+    size_t plain_bytes = 0;
+    DevBuf dev;
+    bool pinned = false;
+    RowBuffers *next = nullptr;  // idle ones of a pool
+    ~RowBuffers() { std::free(plain); }
+};
+struct RowPool
+{
+    std::mutex mu;
+    RowBuffers *idle = nullptr;
+    int out = 0;
+    ~RowPool()
+    {
+        while (RowBuffers *b = idle)
+        {
+            idle = b->next;
+            delete b;
+        }
+    }
+};
+struct RowCall
+{
+    RowPool &pool;
+    cudaStream_t s;
+    RowBuffers *b;
+    bool enqueued = false;
+    RowCall(RowPool &p, cudaStream_t stream) : pool(p), s(stream)
+    {
+        std::lock_guard<std::mutex> lk(pool.mu);
+        b = pool.idle;
+        if (b)
+            pool.idle = b->next;
+        else if ((b = new (std::nothrow) RowBuffers()))
+            b->pinned = pool.out == 0;
+        ++pool.out;
+    }
+    // before the buffers are another call's, what this one enqueued on them is done, also after an error
+    ~RowCall()
+    {
+        if (enqueued)
+            cudaStreamSynchronize(s);
+        std::lock_guard<std::mutex> lk(pool.mu);
+        if (b)
+        {
+            b->next = pool.idle;
+            pool.idle = b;
+        }
+        --pool.out;
+    }
+    gbo_status reserve(size_t bytes)
+    {
+        bytes = std::max(bytes, kRowBytes);
+        if (!b)
+            return fail(GBO_ERR_OUT_OF_MEMORY, "staging allocation failed");
+        if (b->pinned)
+        {
+            if (auto e = b->pin.reserve(bytes))
+                return e;
+        }
+        else if (b->plain_bytes < bytes)
+        {
+            std::free(b->plain);
+            b->plain = std::malloc(bytes);
+            b->plain_bytes = b->plain ? bytes : 0;
+            if (!b->plain)
+                return fail(GBO_ERR_OUT_OF_MEMORY, "staging allocation failed");
+        }
+        return b->dev.reserve(bytes, s);
+    }
+    char *host() const { return (char *)(b->pinned ? b->pin.p : b->plain); }
+    char *device() const { return (char *)b->dev.p; }
+    gbo_status copy_in(size_t bytes)
+    {
+        enqueued = true;
+        CUDA_TRY(cudaMemcpyAsync(device(), host(), bytes, cudaMemcpyHostToDevice, s));
+        return GBO_OK;
+    }
+    gbo_status copy_out(size_t at, size_t bytes)
+    {
+        CUDA_TRY(cudaMemcpyAsync(host() + at, device() + at, bytes, cudaMemcpyDeviceToHost, s));
+        enqueued = false;
+        CUDA_TRY(cudaStreamSynchronize(s));
+        return GBO_OK;
+    }
+};
+
 size_t pad16(size_t b)
 {
     return (b + 15) & ~size_t(15);
@@ -231,6 +327,7 @@ struct gbo_checker
     cudaStream_t host_stream = nullptr;
     Pinned pin_in, pin_out;
     DevBuf dev_in, dev_out;
+    RowPool rows;
     ~gbo_checker()
     {
         if (d64)
@@ -337,6 +434,7 @@ struct gbo_nn
     cudaStream_t host_stream = nullptr;
     Pinned pin;
     DevBuf dev;
+    RowPool rows;
     ~gbo_nn()
     {
         if (searched)
@@ -1568,47 +1666,26 @@ gbo_status gbo_check_motion_host(gbo_checker *c, const double *s1, const double 
     return GBO_OK;
 }
 
-// The buffers of a call below: before they are another call's, what it enqueued on them is done, also where it returns
-// early with an error.
-struct RowsInFlight
-{
-    cudaStream_t s;
-    bool done = false;
-    ~RowsInFlight()
-    {
-        if (!done)
-            cudaStreamSynchronize(s);
-    }
-    cudaError_t wait()
-    {
-        done = true;
-        return cudaStreamSynchronize(s);
-    }
-};
-
 // Small batches in host memory on the caller's stream (ordered after its earlier work, unlike the *_host
-// calls' own stream): one copy in, the kernels, one copy out through the object's page-locked buffer.
+// calls' own stream): one copy in, the kernels, one copy out through the object's page-locked buffers.
 gbo_status gbo_is_valid_rows(gbo_checker *c, const double *states, int64_t n, uint8_t *out, gbo_stream stream)
 {
     if (!c || n < 0 || (n > 0 && (!states || !out)))
         return fail(GBO_ERR_INVALID_ARGUMENT, "bad isValid arguments");
     if (n == 0)
         return GBO_OK;
-    const cudaStream_t st = (cudaStream_t)stream;
-    std::lock_guard<std::mutex> lk(c->mu);
     const size_t bin = (size_t)n * c->sp.dim * sizeof(double);
-    if (auto e = c->pin_in.reserve(bin + (size_t)n))
+    RowCall call(c->rows, (cudaStream_t)stream);
+    if (auto e = call.reserve(bin + (size_t)n))
         return e;
-    if (auto e = c->dev_in.reserve(bin + (size_t)n, st))
-        return e;
-    char *h = (char *)c->pin_in.p, *d = (char *)c->dev_in.p;
-    RowsInFlight flight{st};
+    char *h = call.host(), *d = call.device();
     std::memcpy(h, states, bin);
-    CUDA_TRY(cudaMemcpyAsync(d, h, bin, cudaMemcpyHostToDevice, st));
+    if (auto e = call.copy_in(bin))
+        return e;
     if (auto e = gbo_is_valid(c, (const double *)d, n, c->sp.dim, GBO_LAYOUT_AOS, (uint8_t *)d + bin, stream))
         return e;
-    CUDA_TRY(cudaMemcpyAsync(h + bin, d + bin, (size_t)n, cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(flight.wait());
+    if (auto e = call.copy_out(bin, (size_t)n))
+        return e;
     std::memcpy(out, h + bin, (size_t)n);
     return GBO_OK;
 }
@@ -1621,25 +1698,22 @@ gbo_status gbo_check_motion_rows(gbo_checker *c, const double *s1, const double 
         return fail(GBO_ERR_INVALID_ARGUMENT, "bad checkMotion arguments");
     if (n == 0)
         return GBO_OK;
-    const cudaStream_t st = (cudaStream_t)stream;
-    std::lock_guard<std::mutex> lk(c->mu);
     const size_t bst = (size_t)n * c->sp.dim * sizeof(double), out = 9 * (size_t)n;
-    if (auto e = c->pin_in.reserve(2 * bst + out))
+    RowCall call(c->rows, (cudaStream_t)stream);
+    if (auto e = call.reserve(2 * bst + out))
         return e;
-    if (auto e = c->dev_in.reserve(2 * bst + out, st))
-        return e;
-    char *h = (char *)c->pin_in.p, *d = (char *)c->dev_in.p;
-    RowsInFlight flight{st};
+    char *h = call.host(), *d = call.device();
     std::memcpy(h, s1, bst);
     std::memcpy(h + bst, s2, bst);
-    CUDA_TRY(cudaMemcpyAsync(d, h, 2 * bst, cudaMemcpyHostToDevice, st));
+    if (auto e = call.copy_in(2 * bst))
+        return e;
     int32_t *fj = (int32_t *)(d + 2 * bst), *ndv = fj + n;
     uint8_t *okd = (uint8_t *)(ndv + n);
     if (auto e = gbo_check_motion(c, (const double *)d, (const double *)(d + bst), n, c->sp.dim, GBO_LAYOUT_AOS, schedule,
                                   okd, fj, ndv, stream))
         return e;
-    CUDA_TRY(cudaMemcpyAsync(h + 2 * bst, d + 2 * bst, out, cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(flight.wait());
+    if (auto e = call.copy_out(2 * bst, out))
+        return e;
     std::memcpy(first_j, h + 2 * bst, 4 * (size_t)n);
     std::memcpy(nd, h + 2 * bst + 4 * (size_t)n, 4 * (size_t)n);
     std::memcpy(ok, h + 2 * bst + 8 * (size_t)n, (size_t)n);
@@ -2467,22 +2541,19 @@ gbo_status gbo_nn_nearest_k_rows(gbo_nn *nn, const double *q, int64_t nq, int k,
         return fail(GBO_ERR_UNSUPPORTED, "nearestK supports k <= 64");
     if (nq == 0)
         return GBO_OK;
-    const cudaStream_t st = (cudaStream_t)stream;
-    std::lock_guard<std::mutex> lk(nn->mu);
     const size_t bq = (size_t)nq * nn->sp.dim * sizeof(double), bo = (size_t)nq * k * 8;
-    if (auto e = nn->pin.reserve(bq + 2 * bo))
+    RowCall call(nn->rows, (cudaStream_t)stream);
+    if (auto e = call.reserve(bq + 2 * bo))
         return e;
-    if (auto e = nn->dev.reserve(bq + 2 * bo, st))
-        return e;
-    char *h = (char *)nn->pin.p, *d = (char *)nn->dev.p;
-    RowsInFlight flight{st};
+    char *h = call.host(), *d = call.device();
     std::memcpy(h, q, bq);
-    CUDA_TRY(cudaMemcpyAsync(d, h, bq, cudaMemcpyHostToDevice, st));
+    if (auto e = call.copy_in(bq))
+        return e;
     if (auto e = gbo_nn_nearest_k(nn, (const double *)d, nq, nn->sp.dim, GBO_LAYOUT_AOS, k, nullptr,
                                   (int64_t *)(d + bq), (double *)(d + bq + bo), stream))
         return e;
-    CUDA_TRY(cudaMemcpyAsync(h + bq, d + bq, 2 * bo, cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(flight.wait());
+    if (auto e = call.copy_out(bq, 2 * bo))
+        return e;
     std::memcpy(idx, h + bq, bo);
     std::memcpy(dist, h + bq + bo, bo);
     return GBO_OK;

@@ -1,4 +1,6 @@
 """Host-array arguments in calls that are refused and from several threads."""
+import threading
+import time
 
 import numpy as np
 import pytest
@@ -40,3 +42,68 @@ def test_a_refused_call_uses_no_buffer():
         for _ in range(300):
             got = nn.nearestK(a, 20)
             assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
+
+
+def test_all_calls_from_threads():
+    """isValid, checkMotions and nearestK from four threads at once, with batches whose sizes differ (the buffers grow
+    meanwhile): the results of the same calls made one after another."""
+    rng, ck, nn = _setup()
+    mv = B.DiscreteMotionValidator(ck)
+    sizes = [1, 3, 17, 64, 120, 290]
+    batches = [(rng.uniform(-PI, PI, size=(n, 7)), rng.uniform(-PI, PI, size=(n, 7)), 1 + n % 9) for n in sizes * 8]
+
+    def calls(b):
+        a, c, k = b
+        m = mv.checkMotions(a, c)
+        i, d = nn.nearestK(a, k)
+        return [ck.isValid(a), m["ok"], m["first_j"], m["nd"], i, d]
+
+    want = [calls(b) for b in batches]
+    rng, ck, nn = _setup()  # buffers of no size yet
+    mv = B.DiscreteMotionValidator(ck)
+    got, bad = {}, []
+
+    def work(t):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                for i in range(t, len(batches), 4):
+                    got[i] = calls(batches[i])
+        except Exception as e:  # reported below
+            bad.append(e)
+
+    ts = [threading.Thread(target=work, args=(t,)) for t in range(4)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert not bad
+    for i, w in enumerate(want):
+        assert all(np.array_equal(x, y) for x, y in zip(got[i], w)), i
+
+
+def test_a_waiting_thread_holds_up_no_other():
+    """A thread whose stream has queued work waits for it in its call; another thread's call on another stream does
+    not."""
+    rng, ck, _ = _setup()
+    mv = B.DiscreteMotionValidator(ck)
+    a = rng.uniform(-PI, PI, size=(4, 7))
+    for _ in range(3):
+        ck.isValid(a), mv.checkMotions(a, a)
+    slow, quick = torch.cuda.Stream(), torch.cuda.Stream()
+    done = []
+
+    def held():
+        with torch.cuda.stream(slow):
+            torch.cuda._sleep(1_500_000_000)  # most of a second of clock cycles
+            ck.isValid(a)
+            done.append(time.perf_counter())
+
+    t = threading.Thread(target=held)
+    t.start()
+    time.sleep(0.1)
+    with torch.cuda.stream(quick):
+        ck.isValid(a)
+        mv.checkMotions(a, a)
+    free = time.perf_counter()
+    t.join()
+    assert done[0] > free
