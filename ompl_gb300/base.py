@@ -9,6 +9,7 @@ from __future__ import annotations
 
 import ctypes as C
 import math
+import operator
 
 import numpy as np
 import torch
@@ -58,7 +59,10 @@ _SMALL_HOST_BYTES = 1 << 16
 
 
 def _rows(x, dim):
-    return np.ascontiguousarray(x, dtype=np.float64).reshape(-1, dim)
+    a = np.ascontiguousarray(x)
+    if a.dtype != np.float64:  # the conversions that a larger batch gets, and their refusals
+        a = torch.as_tensor(a, dtype=torch.float64).numpy()
+    return a.reshape(-1, dim)
 
 
 class StateSpace:
@@ -485,7 +489,7 @@ class NearestNeighborsGPU:
 
     def nearestK(self, queries, k, prefix=None, soa=False, want_dist=True, stream=None):
         if prefix is None and not soa and want_dist and not isinstance(queries, torch.Tensor):
-            a, k = _rows(queries, self.space.dim), int(k)
+            a, k = _rows(queries, self.space.dim), operator.index(k)
             if a.nbytes + 16 * a.shape[0] * max(k, 0) <= _SMALL_HOST_BYTES:
                 idx = np.empty((a.shape[0], max(k, 0)), dtype=np.int64)
                 dist = np.empty((a.shape[0], max(k, 0)))

@@ -1,4 +1,4 @@
-"""Host-array arguments in calls that are refused and from several threads."""
+"""Host-array arguments: what numpy batches are refused whatever their size, and calls from several threads."""
 import threading
 import time
 
@@ -26,6 +26,27 @@ def _setup(n=4000):
     nn.add(torch.as_tensor(rng.uniform(-PI, PI, size=(n, 7)), device="cuda"))
     torch.cuda.synchronize()
     return rng, ck, nn
+
+
+@pytest.mark.parametrize("rows", [2, 3000])  # below and above the size of a small batch
+def test_refused(rows):
+    _, ck, nn = _setup()
+    text = [["0.1"] * 7] * rows
+    with pytest.raises(TypeError):
+        ck.isValid(text)
+    with pytest.raises(TypeError):
+        B.DiscreteMotionValidator(ck).checkMotions(text, text)
+    with pytest.raises(TypeError):
+        nn.nearestK(text, 1)
+    with pytest.raises(TypeError):
+        nn.nearestK(np.zeros((rows, 7)), 2.5)
+    for k in (-1, 0, 65):
+        with pytest.raises((RuntimeError, ValueError)):
+            nn.nearestK(np.zeros((rows, 7)), k)
+    # converted as before
+    a = np.zeros((rows, 7), dtype=np.float32)
+    assert np.array_equal(ck.isValid(a), ck.isValid(a.astype(np.float64)))
+    assert np.array_equal(nn.nearestK(a.astype(np.int32).tolist(), np.int64(3))[0], nn.nearestK(a, 3)[0])
 
 
 def test_a_refused_call_uses_no_buffer():
