@@ -58,8 +58,7 @@ def _host(t):
 _SMALL_HOST_BYTES = 1 << 16
 
 
-def _rows(x, dim):
-    a = np.ascontiguousarray(x)
+def _rows(a, dim):
     if a.dtype != np.float64:  # the conversions that a larger batch gets, and their refusals
         a = torch.as_tensor(a, dtype=torch.float64).numpy()
     return a.reshape(-1, dim)
@@ -230,8 +229,9 @@ class StateValidityChecker:
 
     def isValid(self, states, soa=False, stream=None):
         if not soa and not isinstance(states, torch.Tensor):
-            a = _rows(states, self.space.dim)
-            if a.nbytes <= _SMALL_HOST_BYTES:
+            states = np.ascontiguousarray(states)
+            if 8 * states.size <= _SMALL_HOST_BYTES:
+                a = _rows(states, self.space.dim)
                 out = np.empty(a.shape[0], dtype=np.uint8)
                 check(lib().gbo_is_valid_rows(self._h, a.ctypes.data, a.shape[0], out.ctypes.data, _stream(stream)))
                 return out.astype(bool)
@@ -310,8 +310,9 @@ class DiscreteMotionValidator:
         """Batch checkMotion: dict(ok, first_j, nd[, last_t, last_state]) as tensors or numpy arrays."""
         dim = self.space.dim
         if not soa and not last_valid and not isinstance(s1, torch.Tensor) and not isinstance(s2, torch.Tensor):
-            a, b = _rows(s1, dim), _rows(s2, dim)
-            if a.shape == b.shape and 2 * a.nbytes <= _SMALL_HOST_BYTES:
+            s1, s2 = np.ascontiguousarray(s1), np.ascontiguousarray(s2)
+            if s1.size == s2.size and 16 * s1.size <= _SMALL_HOST_BYTES:
+                a, b = _rows(s1, dim), _rows(s2, dim)
                 n = a.shape[0]
                 res = {"ok": np.empty(n, dtype=np.uint8), "first_j": np.empty(n, dtype=np.int32),
                        "nd": np.empty(n, dtype=np.int32)}
@@ -489,8 +490,9 @@ class NearestNeighborsGPU:
 
     def nearestK(self, queries, k, prefix=None, soa=False, want_dist=True, stream=None):
         if prefix is None and not soa and want_dist and not isinstance(queries, torch.Tensor):
-            a, k = _rows(queries, self.space.dim), operator.index(k)
-            if a.nbytes + 16 * a.shape[0] * max(k, 0) <= _SMALL_HOST_BYTES:
+            queries, k = np.ascontiguousarray(queries), operator.index(k)
+            if 8 * queries.size + 16 * (queries.size // self.space.dim) * max(k, 0) <= _SMALL_HOST_BYTES:
+                a = _rows(queries, self.space.dim)
                 idx = np.empty((a.shape[0], max(k, 0)), dtype=np.int64)
                 dist = np.empty((a.shape[0], max(k, 0)))
                 check(lib().gbo_nn_nearest_k_rows(self._h, a.ctypes.data, a.shape[0], k, idx.ctypes.data,

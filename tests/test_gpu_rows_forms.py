@@ -128,3 +128,24 @@ def test_a_waiting_thread_holds_up_no_other():
     free = time.perf_counter()
     t.join()
     assert done[0] > free
+
+
+def test_large_lists_are_converted_once():
+    """A batch too large for the row buffers goes on as the array that its size was taken from."""
+    rng, ck, nn = _setup()
+    made = []
+
+    class Counted:
+        def __init__(self, a):
+            self.a = a
+
+        def __array__(self, dtype=None, copy=None):
+            made.append(1)
+            return self.a if dtype is None else self.a.astype(dtype)
+
+    a, b = rng.uniform(-PI, PI, size=(3000, 7)), rng.uniform(-PI, PI, size=(3000, 7))
+    assert np.array_equal(ck.isValid(Counted(a)), ck.isValid(a)) and len(made) == 1
+    mv = B.DiscreteMotionValidator(ck)
+    assert np.array_equal(mv.checkMotions(Counted(a), Counted(b))["first_j"], mv.checkMotions(a, b)["first_j"])
+    assert len(made) == 3
+    assert np.array_equal(nn.nearestK(Counted(a), 3)[0], nn.nearestK(a, 3)[0]) and len(made) == 4
