@@ -729,12 +729,18 @@ static gbo_status build_chain_masks(gbo_checker *c, const double *world, int n)
         const double dx = world[4 * j + 2] - world[4 * j], dy = world[4 * j + 3] - world[4 * j + 1];
         const double ax = world[4 * j] - dx / 64.0, ay = world[4 * j + 1] - dy / 64.0;  // lengthened at both ends
         const double bx = dx * (33.0 / 32.0), by = dy * (33.0 / 32.0), B = std::hypot(dx, dy);
-        for (int p = 0; p < G; ++p)
-            for (int q = 0; q < G; ++q)
+        // the cells whose middle lies in the segment's box widened by `reach`
+        const double b2 = bx * bx + by * by, far2 = reach * reach * (1.0 + 1e-12);
+        auto first = [&](double lo) { return std::max(0, (int)std::floor((lo - reach + half) / cell - 0.5)); };
+        auto last = [&](double hi) { return std::min(G - 1, (int)std::ceil((hi + reach + half) / cell - 0.5)); };
+        const int p1 = last(std::max(ax, ax + bx)), q1 = last(std::max(ay, ay + by));
+        for (int p = first(std::min(ax, ax + bx)); p <= p1; ++p)
+            for (int q = first(std::min(ay, ay + by)); q <= q1; ++q)
             {
-                const double x = -half + (p + 0.5) * cell - ax, y = -half + (q + 0.5) * cell - ay, b2 = bx * bx + by * by;
+                const double x = -half + (p + 0.5) * cell - ax, y = -half + (q + 0.5) * cell - ay;
                 const double t = b2 > 0.0 ? std::min(1.0, std::max(0.0, (x * bx + y * by) / b2)) : 0.0;
-                if (std::hypot(x - t * bx, y - t * by) <= reach)
+                const double ex = x - t * bx, ey = y - t * by;
+                if (ex * ex + ey * ey <= far2)
                     m[(size_t)p * G + q] |= 1ull << j;
             }
         // |denom| = L B |sin|, 66 FLT_EPSILON against the rounding of the FP32 direction (and 1e-5 of an angle)
