@@ -791,28 +791,25 @@ static gbo_status build_circle_grid(gbo_checker *c, const double *world, int64_t
     for (int G = 256; G >= 2; G /= 2)
     {
         const double cell[2] = {(hi[0] - lo[0]) / G, (hi[1] - lo[1]) / G};
+        // the cells a thousandth of a cell around circle i: a row's run of cells follows from its distance in x
+        const double inv[2] = {1.0 / cell[0], 1.0 / cell[1]};
         auto visit = [&](int64_t i, auto &&emit) {
-            const double x[2] = {world[3 * i], world[3 * i + 1]}, r = std::fabs(world[3 * i + 2]);
-            int a[2], b[2];
-            for (int d = 0; d < 2; ++d)
+            const double x = world[3 * i] - lo[0], y = world[3 * i + 1] - lo[1], r = std::fabs(world[3 * i + 2]);
+            const double r2 = r * r * (1.0 + 1e-9);
+            auto first = [&](double at) { return std::max(0, (int)std::floor(at - 2e-3)); };
+            auto last = [&](double at) { return std::min(G - 1, (int)std::floor(at + 2e-3)); };
+            const int p1 = last((x + r) * inv[0]);
+            for (int p = first((x - r) * inv[0]); p <= p1; ++p)
             {
-                a[d] = std::max(0, (int)std::floor((x[d] - r - lo[d]) / cell[d]) - 1);
-                b[d] = std::min(G - 1, (int)std::floor((x[d] + r - lo[d]) / cell[d]) + 1);
+                const double b0 = (p - 1e-3) * cell[0], b1 = (p + 1.0 + 1e-3) * cell[0];
+                const double gap = x < b0 ? b0 - x : (x > b1 ? x - b1 : 0.0);
+                if (gap * gap > r2)
+                    continue;
+                const double w = std::sqrt(r2 - gap * gap);
+                const int q1 = last((y + w) * inv[1]);
+                for (int q = first((y - w) * inv[1]); q <= q1; ++q)
+                    emit(p * G + q);
             }
-            for (int p = a[0]; p <= b[0]; ++p)
-                for (int q = a[1]; q <= b[1]; ++q)
-                {
-                    double d2 = 0.0;
-                    const int k[2] = {p, q};
-                    for (int d = 0; d < 2; ++d)
-                    {
-                        const double b0 = lo[d] + (k[d] - 1e-3) * cell[d], b1 = lo[d] + (k[d] + 1.0 + 1e-3) * cell[d];
-                        const double gap = x[d] < b0 ? b0 - x[d] : (x[d] > b1 ? x[d] - b1 : 0.0);
-                        d2 += gap * gap;
-                    }
-                    if (d2 <= r * r * (1.0 + 1e-9))
-                        emit(p * G + q);
-                }
         };
         const size_t most = 4096 + 16 * (size_t)n;
         size_t total = 0;
