@@ -23,12 +23,12 @@ struct RunCounters
     unsigned int deferred;         // edges the arm's motion kernel left to its chunk kernel
 };
 
-// An edge whose states many warps share (kernels_arm.cu): first unchecked state, smallest colliding one found
-// (INT_MAX: none)
-struct ArmTail
+// An edge whose states many warps share (kernels_arm.cu): its number (below 2^32: a row is 8 bytes or more), first
+// unchecked state, smallest colliding one found (INT_MAX: none), segment count
+struct __align__(16) ArmTail
 {
-    long long e;
-    int next, first;
+    unsigned e;
+    int next, first, nd;
 };
 constexpr int kArmTailRoom = 2048;
 

@@ -39,7 +39,8 @@ namespace gbo
 {
 
 constexpr int kLateRounds = 8;   // rounds of a warp after the queue ran empty
-constexpr int kArmChunks = 32;   // runs an edge is cut into
+constexpr int kArmChunks = 32;   // most runs that an edge is cut into, and
+constexpr int kArmRun = 32;      // fewest states of a run
 
 // Signed distance of obstacle i's surface from (x, y, z); the definition compares sphere distances with
 // (rs + r)^2, so a negative radius acts by |rs + r|.
@@ -360,9 +361,7 @@ __global__ void __launch_bounds__(128, 5)
             at = __shfl_sync(0xffffffffu, at, 0) + __popc(L & ((1u << lane) - 1u));
             if (live && at < (unsigned)kArmTailRoom)
             {
-                tail[at].e = e;
-                tail[at].next = next;
-                tail[at].first = INT_MAX;
+                tail[at] = ArmTail{(unsigned)e, next, INT_MAX, nd};
                 live = false;
             }
         }
@@ -370,16 +369,16 @@ __global__ void __launch_bounds__(128, 5)
     arm_counts(ctr, evaluated, rechecks, lane);
 }
 
-// Edges shared by many warps: a batch (tail null, first_j holds the smallest colliding state found) or the
-// list that arm_motion_kernel left. The states left of an edge are cut into `chunks` runs; work item
-// c * count + i is run c of edge i, so that every edge's early runs go first and the later runs of an edge
-// that has already collided before them are passed over. A run's 32 lanes evaluate states a stride apart, as
-// above. arm_finish_kernel then writes the results.
+// Edges shared by many warps: a batch (tail null; first_j holds the smallest colliding state found, nd_out the segment
+// counts) or the list that arm_motion_kernel left. The states left of an edge are cut into at most `chunks` runs of
+// kArmRun states or more; work item c * count + i is run c of edge i, so that every edge's early runs go first and the
+// later runs of an edge that has already collided before them are passed over, as are those that a short edge does not
+// have. A run's 32 lanes evaluate states a stride apart, as above. arm_finish_kernel then writes the results.
 template <int PREC>
 __global__ void __launch_bounds__(128, 5)
     arm_chunk_kernel(const __grid_constant__ SpaceParams sp, const __grid_constant__ WorldArgs wa,
                      const __grid_constant__ StatesView v1, const __grid_constant__ StatesView v2, int n, int chunks,
-                     ArmTail *tail, int32_t *first_j, RunCounters *ctr)
+                     ArmTail *tail, int32_t *first_j, const int32_t *nd_out, RunCounters *ctr)
 {
     __shared__ float tab[4][32][32];
     __shared__ ArmChain chain[4];
@@ -389,16 +388,15 @@ __global__ void __launch_bounds__(128, 5)
     float(*edge)[32] = tab[warp];
     unsigned evaluated = 0, rechecks = 0;
     const int count = tail ? (int)min(ctr->deferred, (unsigned)kArmTailRoom) : n;
-    const int64_t items = (int64_t)count * chunks, warps = (int64_t)gridDim.x * 4;
-    for (int64_t item = (int64_t)blockIdx.x * 4 + warp; item < items; item += warps)
+    const int items = count * chunks, warps = (int)gridDim.x * 4;
+    for (int item = (int)blockIdx.x * 4 + warp; item < items; item += warps)
     {
-        const int c = (int)(item / count), i = (int)(item % count);
+        const int c = item / count, i = item % count;
         const int64_t e = tail ? tail[i].e : i;
-        const int start = tail ? tail[i].next : 1;
+        const int nd = tail ? tail[i].nd : nd_out[i], start = tail ? tail[i].next : 1;
         int *first = tail ? &tail[i].first : first_j + i;
-        double a[8], b[8];
-        const int nd = arm_segments(sp, v1, v2, e, a, b), top = nd > 1 ? nd : 1;
-        const int64_t len = ((int64_t)top - start + chunks) / chunks;
+        const int top = nd > 1 ? nd : 1;
+        const int64_t len = max(((int64_t)top - start + chunks) / chunks, (int64_t)kArmRun);
         int64_t lo = start + c * len;
         const int64_t end = min(lo + len - 1, (int64_t)top);
         // the smallest colliding state found so far, the same in every lane
@@ -409,11 +407,8 @@ __global__ void __launch_bounds__(128, 5)
         if (lo <= end && found() > lo)
         {
             __syncwarp();
-            if (lane == 0)
-#pragma unroll
-                for (int d = 0; d < 8; ++d)
-                    if (d < sp.dim)
-                        arm_store_joint(sp, edge, 0, d, a[d], b[d]);
+            if (lane < sp.dim)
+                arm_store_joint(sp, edge, 0, lane, v1(e, lane), v2(e, lane));
             __syncwarp();
             int64_t stride = 1;
             while (lo <= end && found() > lo)
@@ -460,27 +455,27 @@ __global__ void __launch_bounds__(128, 5)
     arm_counts(ctr, evaluated, rechecks, lane);
 }
 
-__global__ void arm_begin_kernel(int32_t *first_j, int n)
+__global__ void arm_begin_kernel(const __grid_constant__ SpaceParams sp, StatesView v1, StatesView v2, int n,
+                                 int32_t *first_j, int32_t *nd_out)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n)
-        first_j[i] = INT_MAX;
+    if (i >= n)
+        return;
+    double a[8], b[8];
+    nd_out[i] = arm_segments(sp, v1, v2, i, a, b);
+    first_j[i] = INT_MAX;
 }
 
 // results of the edges that the chunk kernel checked
-__global__ void arm_finish_kernel(const __grid_constant__ SpaceParams sp, StatesView v1, StatesView v2, int n,
-                                  const ArmTail *tail, uint8_t *ok, int32_t *first_j, int32_t *nd_out,
+__global__ void arm_finish_kernel(int n, const ArmTail *tail, uint8_t *ok, int32_t *first_j, int32_t *nd_out,
                                   const RunCounters *ctr)
 {
     const int count = tail ? (int)min(ctr->deferred, (unsigned)kArmTailRoom) : n;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count)
         return;
-    const int64_t e = tail ? tail[i].e : i;
-    const int f = tail ? tail[i].first : first_j[i];
-    double a[8], b[8];
-    const int nd = arm_segments(sp, v1, v2, e, a, b);
-    arm_write(e, f == INT_MAX ? -1 : f, nd, nd > 1 ? nd : 1, ok, first_j, nd_out);
+    const ArmTail t = tail ? tail[i] : ArmTail{(unsigned)i, 1, first_j[i], nd_out[i]};
+    arm_write(t.e, t.first == INT_MAX ? -1 : t.first, t.nd, t.nd > 1 ? t.nd : 1, ok, first_j, nd_out);
 }
 
 template <int PREC>
@@ -490,15 +485,17 @@ static void launch_arm_motion_t(const LaunchCfg &lc, const SpaceParams &sp, cons
 {
     // CTAs the GPU holds (the same shared memory and registers in both kernels)
     const int full = persistent_grid((const void *)arm_motion_kernel<PREC>, 128, 0, lc, INT64_MAX / 2);
-    // Few edges: a lane each would leave the GPU empty and wait for the longest edge; cut in runs instead (100
-    // edges of 2..2,000 states: 75 us against 220 us, 2,000 edges 287 us against 238 us).
-    constexpr int kFewEdges = 768;
-    if (fj && n <= kFewEdges)
+    // Few edges: a lane each would leave the GPU empty and wait for the longest edge; cut in runs instead. Runs / lanes,
+    // among 1,500 spheres: 1,500 edges of 120 states 138 / 226 us, of 2..2,000 states 157 / 275 us; 4,000 edges of 12
+    // states 121 / 108 us, of 120 172 / 283 us, of 2..2,000 226 / 353 us; 6,000 of 12 states 177 / 155 us, of 120 222 /
+    // 245 us; 20,000 of 120 451 / 320 us.
+    constexpr int kFewEdges = 4096;
+    if (fj && nd && n <= kFewEdges)
     {
-        arm_begin_kernel<<<(int)((n + 255) / 256), 256, 0, lc.stream>>>(fj, (int)n);
+        arm_begin_kernel<<<(int)((n + 63) / 64), 64, 0, lc.stream>>>(sp, v1, v2, (int)n, fj, nd);
         const int grid = (int)std::min<int64_t>(full, (n * kArmChunks + 3) / 4);
-        arm_chunk_kernel<PREC><<<grid, 128, 0, lc.stream>>>(sp, wa, v1, v2, (int)n, kArmChunks, nullptr, fj, ctr);
-        arm_finish_kernel<<<(int)((n + 127) / 128), 128, 0, lc.stream>>>(sp, v1, v2, (int)n, nullptr, ok, fj, nd, ctr);
+        arm_chunk_kernel<PREC><<<grid, 128, 0, lc.stream>>>(sp, wa, v1, v2, (int)n, kArmChunks, nullptr, fj, nd, ctr);
+        arm_finish_kernel<<<(int)((n + 127) / 128), 128, 0, lc.stream>>>((int)n, nullptr, ok, fj, nd, ctr);
     }
     else
     {
@@ -508,8 +505,8 @@ static void launch_arm_motion_t(const LaunchCfg &lc, const SpaceParams &sp, cons
             per *= 2;
         const int grid = (int)std::min<int64_t>(full, (n + 4 * per - 1) / (4 * per));
         arm_motion_kernel<PREC><<<grid, 128, 0, lc.stream>>>(sp, wa, v1, v2, n, per, tail, ok, fj, nd, ctr);
-        arm_chunk_kernel<PREC><<<full, 128, 0, lc.stream>>>(sp, wa, v1, v2, 0, kArmChunks, tail, nullptr, ctr);
-        arm_finish_kernel<<<kArmTailRoom / 128, 128, 0, lc.stream>>>(sp, v1, v2, 0, tail, ok, fj, nd, ctr);
+        arm_chunk_kernel<PREC><<<full, 128, 0, lc.stream>>>(sp, wa, v1, v2, 0, kArmChunks, tail, nullptr, nullptr, ctr);
+        arm_finish_kernel<<<kArmTailRoom / 128, 128, 0, lc.stream>>>(0, tail, ok, fj, nd, ctr);
     }
     for (int i = 0; i < 3; ++i)
         note_launch();
