@@ -29,14 +29,14 @@ namespace gbo
 
 constexpr int kSubMax = 1 << 19;  // cells times sub-cells
 
-// Smallest metric distance of x from a point of [lo, hi] on the circle. The metric folds t = |x - y| to min(t, 2 pi -
-// t), which is negative from 2 pi on (elements outside [-pi, pi], an interval widened past the wrap) and counts by
-// its square: 0 where t = 0 or t = 2 pi lies between the ends, else the nearer end's magnitude.
+// Lower bound of the metric distance of x from a point of [lo, hi] on the circle. The metric folds t = |x - y| to
+// min(t, 2 pi - t), which is negative from 2 pi on (elements outside [-pi, pi], an interval widened past the wrap) and
+// counts by its square: 0 inside and where an end lies that far, else the nearer end's.
 __device__ __forceinline__ float wrap_gap(float x, float lo, float hi)
 {
     const float u = fabsf(x - lo), v = fabsf(x - hi);
     const float a = fminf(u, 6.28318530717958647692f - u), b = fminf(v, 6.28318530717958647692f - v);
-    return (x >= lo && x <= hi) || a * b <= 0.f ? 0.f : fminf(fabsf(a), fabsf(b));
+    return (x >= lo && x <= hi) ? 0.f : fmaxf(fminf(a, b), 0.f);
 }
 
 // distance from query q to the box (lo, hi per coordinate), squared, scaled down by (1 - 1e-5) against
