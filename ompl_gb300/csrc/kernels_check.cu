@@ -221,8 +221,10 @@ __device__ int segment_count(const SpaceParams &sp, const WorldArgs &wa, const d
     return segment_count_from_distance(sp, distance64<MAXD>(sp, a, b));
 }
 
-// A warp takes `per` consecutive edges at a time: lane i computes the segment count of edge i (FP64, so a warp
-// instruction costs the same for one edge as for 32), then the warp checks the edges one after another.
+// A warp takes `per` edges at a time, `groups` apart: lane i computes the segment count of the i-th (FP64, so a warp
+// instruction costs the same for one edge as for 32), then the warp checks the edges one after another. Edges side by
+// side in the batch are different warps': with the first 64 of 100,000 edges 2,880 states long and the rest short, among
+// three circles, 245 us; with consecutive edges a warp 2,384 us, one edge a warp 549.
 template <int CK, int MAXD>
 __global__ void __launch_bounds__(256) motion_plain_kernel(SpaceParams sp, WorldArgs wa, StatesView v1,
                                                            StatesView v2, int64_t n, int per, uint8_t *ok,
@@ -237,10 +239,11 @@ __global__ void __launch_bounds__(256) motion_plain_kernel(SpaceParams sp, World
     const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     unsigned evaluated = 0, rechecks = 0;
-    for (int64_t e0 = warp * per; e0 < n; e0 += nwarps * per)
+    const int64_t groups = (n + per - 1) / per;
+    for (int64_t w = warp; w < groups; w += nwarps)
     {
         double a[MAXD], b[MAXD];
-        const int64_t mine = e0 + lane;
+        const int64_t mine = w + lane * groups;
         int nds = 0, result = -1;
         if (lane < per && mine < n)
         {
@@ -249,11 +252,12 @@ __global__ void __launch_bounds__(256) motion_plain_kernel(SpaceParams sp, World
             nds = segment_count_from_distance(sp, distance64<MAXD>(sp, a, b));
         }
         __syncwarp();
-        for (int i = 0; i < per && e0 + i < n; ++i)
+        for (int i = 0; i < per && w + i * groups < n; ++i)
         {
+            const int64_t e = w + i * groups;
             const int nd = __shfl_sync(0xffffffffu, nds, i), top = nd > 1 ? nd : 1;
-            load_state<MAXD>(v1, e0 + i, sp.dim, a);
-            load_state<MAXD>(v2, e0 + i, sp.dim, b);
+            load_state<MAXD>(v1, e, sp.dim, a);
+            load_state<MAXD>(v2, e, sp.dim, b);
             int first = -1;
             for (int base = 1; base <= top; base += 32)
             {
@@ -596,8 +600,11 @@ static void launch_motion_t(const LaunchCfg &lc, int schedule, const SpaceParams
     {
         auto k = motion_plain_kernel<CK, MAXD>;
         const unsigned sm = world_smem_bytes(wa, GBO_PRECISION_FP64);
-        // 16 warps an SM already keep the FP64 pipe busy: beyond that, edges per warp
-        const int per = (int)std::max<int64_t>(1, std::min<int64_t>(32, n / ((int64_t)lc.sm_count * 16)));
+        // 16 warps an SM already keep the FP64 pipe busy with segment counts: beyond that, edges per warp. The chain's
+        // states take longer than its counts and want 32 (20,000 edges of one state: 20.7 ms at 16, 17.9 at 32, 18.2
+        // an edge a warp; 100,000 edges of up to 100 states 27.9 ms, an edge a warp 40.6).
+        const int busy = CK == GBO_CHECK_CHAIN_SEGMENTS ? 32 : 16;
+        const int per = (int)std::max<int64_t>(1, std::min<int64_t>(32, n / ((int64_t)lc.sm_count * busy)));
         const int grid = persistent_grid((const void *)k, 256, sm, lc, ((n + per - 1) / per * 32 + 255) / 256);
         k<<<grid, 256, sm, lc.stream>>>(sp, wa, v1, v2, n, per, ok, fj, nd, ctr);
     }
