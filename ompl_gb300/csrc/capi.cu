@@ -2033,7 +2033,8 @@ gbo_status gbo_nn_add(gbo_nn *nn, const double *states, int64_t n, int64_t ld, i
     launch_features(lc, nn->sp, v, n, nn->feat32 + nn->size, nn->cap, nn->feat4 + nn->size);
     CHECK_LAUNCH();
     nn->size += n;
-    nn->alive_count += n;
+    if (nn->alive_count >= 0)  // else recounted on demand
+        nn->alive_count += n;
     for (auto &c : nn->cells)
         c.size = 0;
     nn->forgone = 0;
