@@ -31,12 +31,12 @@ constexpr int kSubMax = 1 << 19;  // cells times sub-cells
 
 // Lower bound of the metric distance of x from a point of [lo, hi] on the circle. The metric folds t = |x - y| to
 // min(t, 2 pi - t), which is negative from 2 pi on (elements outside [-pi, pi], an interval widened past the wrap) and
-// counts by its square: 0 inside and where an end lies that far, else the nearer end's.
+// counts by its square: 0 inside and where an end lies that far, else the nearer end's. (Outside, the nearer end is
+// max(p, r) away, the other max(|p|, |r|).)
 __device__ __forceinline__ float wrap_gap(float x, float lo, float hi)
 {
-    const float u = fabsf(x - lo), v = fabsf(x - hi);
-    const float a = fminf(u, 6.28318530717958647692f - u), b = fminf(v, 6.28318530717958647692f - v);
-    return (x >= lo && x <= hi) ? 0.f : fmaxf(fminf(a, b), 0.f);
+    const float p = lo - x, r = x - hi;
+    return fmaxf(fminf(fmaxf(p, r), 6.28318530717958647692f - fmaxf(fabsf(p), fabsf(r))), 0.f);
 }
 
 // distance from query q to the box (lo, hi per coordinate), squared, scaled down by (1 - 1e-5) against
@@ -420,6 +420,11 @@ __global__ void __launch_bounds__(128, 8) knn_cell_kernel(const __grid_constant_
             T = fminf(T, r * r * (1.0f + 1e-5f));
         }
     };
+    // a query that is not finite has no neighbours, and its bounds are 0: nothing is searched
+    bool finite = true;
+#pragma unroll
+    for (int f = 0; f < MAXF; ++f)
+        finite = finite && fabsf(q[f]) < inf;
     auto scan_chunk = [&](int p0, int s1) {
         const int p = p0 + lane;
         float d = inf;
@@ -479,11 +484,12 @@ __global__ void __launch_bounds__(128, 8) knn_cell_kernel(const __grid_constant_
     for (int d = MAXF - 1; d >= 0; --d)
         if (d < sp.dim)
             own = own * L + cell_level(sp, L, d, q[d], h);
-    scan_cell(own);
+    if (finite)
+        scan_cell(own);
     // rings of a tenth and a third of the threshold's square, then the rest (an infinite T: all at once)
     float from = -1.f;
 #pragma unroll 1
-    for (int ring = 0; ring < 3; ++ring)
+    for (int ring = 0; finite && ring < 3; ++ring)
     {
         const float cut = fminf(T, list.last());
         const float to = ring == 2 || !(cut < inf) ? inf : (ring == 0 ? 0.1f : 0.33f) * cut;

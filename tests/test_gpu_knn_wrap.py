@@ -60,3 +60,22 @@ def test_outside_the_range(dim):
     pts[:500] = 1.2 * PI + rng.normal(0, 1e-3, size=(500, dim))
     q[:200] = -0.8 * PI + rng.normal(0, 1e-3, size=(200, dim))
     _both(dim, pts, q)
+
+
+@pytest.mark.parametrize("space", [B.WrapL2StateSpace(3), B.RealVectorStateSpace(3, -PI, PI)])
+def test_queries_that_are_not_finite(space):
+    """They have no neighbours, the others in the batch theirs."""
+    rng = np.random.default_rng(2)
+    nn = B.NearestNeighborsGPU(space, capacity=N)
+    nn.add(torch.as_tensor(rng.uniform(-PI, PI, size=(N, 3)), device="cuda"))
+    q = torch.as_tensor(rng.uniform(-PI, PI, size=(NQ, 3)), device="cuda")
+    want = nn.nearestK(q, 10)
+    odd = torch.arange(0, NQ, 7, device="cuda")
+    for value in (float("nan"), float("inf"), -float("inf")):
+        x = q.clone()
+        x[odd, 1] = value
+        idx, dist = nn.nearestK(x, 10)
+        assert bool((idx[odd] == -1).all()) and bool(torch.isinf(dist[odd]).all())
+        fine = torch.ones(NQ, dtype=torch.bool, device="cuda")
+        fine[odd] = False
+        assert torch.equal(idx[fine], want[0][fine]) and torch.equal(dist[fine], want[1][fine])
