@@ -795,6 +795,7 @@ def arm_workload(port, n_plain=16_384):
     return {"workload": "dh_arm7: 7-DoF DH arm (8 spheres r 0.05 per link), 4,096 world spheres in a 64^3 grid, "
                         "256k edges of 2..2000 interpolation steps, one launch",
             "edges": n, "edges_per_s": res, "plain_edges_per_s": res["plain_fp64"],
+            "plain_form": "FP64 verdicts; states that FP32 clearance proves free are not evaluated",
             "batched_edges_per_s": res["batched"], "batched_vs_plain": res["batched"] / res["plain_fp64"],
             "plain_sample_edges": n_plain, "checked_states_per_edge": checked / n,
             "valid_fraction": float(r["ok"].float().mean().item()),

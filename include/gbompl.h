@@ -67,13 +67,17 @@ enum {
                                      collision checker of its own), definition in oracle/dh_arm.h */
 };
 
-/* Arithmetic of validity / motion / kNN evaluation. */
+/* Arithmetic of validity / motion / kNN evaluation. Verdicts, neighbours and distances are the FP64
+ * ones in both. FP64: FP64 throughout, reference operation order (the plain form), with one exception:
+ * DH-arm motion skips states that FP32 kinematics and a clearance grid prove free within their error
+ * bounds, and evaluates every state that may touch an obstacle in FP64. FP32_GUARDED also covers
+ * nearestR: FP32 decides elements away from the radius, FP64 those near it and every distance returned. */
 enum {
-    GBO_PRECISION_FP64 = 0,        /* FP64 throughout, reference operation order (the plain form) */
+    GBO_PRECISION_FP64 = 0,        /* FP64, reference operation order */
     GBO_PRECISION_FP32_GUARDED = 1 /* FP32 bulk; anything within the guard band re-evaluated in FP64 */
 };
 
-/* Motion-batch schedules. */
+/* Motion-batch schedules. The DH arm's motion has one form for all of them. */
 enum {
     GBO_SCHEDULE_PLAIN = 0, /* one launch, one warp per edge, 32 steps per ballot, FP64 (drop-in) */
     GBO_SCHEDULE_TILE = 1,  /* persistent: 32 edges per warp, lanes re-spread over live edges */

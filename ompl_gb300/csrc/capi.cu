@@ -717,7 +717,8 @@ static gbo_status build_chain_masks(gbo_checker *c, const double *world, int n)
             return GBO_OK;
     constexpr int G = kChainMaskCells, K = kChainMaskBins;
     std::vector<unsigned long long> m((size_t)G * G + K, 0);
-    const double half = c->sp.dim * L * 1.01, cell = 2.0 * half / G, reach = L * 33.0 / 64.0 + cell * 0.70711 + 1e-3 * L;
+    const double half = c->sp.dim * L * 1.01, cell = 2.0 * half / G;
+    const double reach = L * 33.0 / 64.0 + cell * 0.70711 + 1e-3 * L;
     const double eps = std::ldexp(1.0, -23);
     // position of a direction in [0, 1): 0.5 - 0.5 cos / (|cos| + |sin|) over the half turn [0, pi)
     auto place = [&](double t) {
@@ -1712,8 +1713,8 @@ gbo_status gbo_check_motion_rows(gbo_checker *c, const double *s1, const double 
         return e;
     int32_t *fj = (int32_t *)(d + 2 * bst), *ndv = fj + n;
     uint8_t *okd = (uint8_t *)(ndv + n);
-    if (auto e = gbo_check_motion(c, (const double *)d, (const double *)(d + bst), n, c->sp.dim, GBO_LAYOUT_AOS, schedule,
-                                  okd, fj, ndv, stream))
+    if (auto e = gbo_check_motion(c, (const double *)d, (const double *)(d + bst), n, c->sp.dim, GBO_LAYOUT_AOS,
+                                  schedule, okd, fj, ndv, stream))
         return e;
     if (auto e = call.copy_out(2 * bst, out))
         return e;
@@ -2189,8 +2190,8 @@ static gbo_status box_cells_call(gbo_nn *nn, const LaunchCfg &lc, const float *q
             CHECK_LAUNCH();
             c.size = size;
         }
-        launch_knn_cells(lc, c.args(), nn->sp, qf, nq, prefix, size / 2, level == 0, k, key, count, qstart, fill, qorder,
-                         bs, o);
+        launch_knn_cells(lc, c.args(), nn->sp, qf, nq, prefix, size / 2, level == 0, k, key, count, qstart, fill,
+                         qorder, bs, o);
         CHECK_LAUNCH();
         if (level + 1 < n)
             size /= 2;
@@ -2258,10 +2259,9 @@ gbo_status gbo_nn_nearest_k(gbo_nn *nn, const double *q, int64_t nq, int64_t ld,
         const bool chain = nn->sp.kind == GBO_SPACE_KINEMATIC_CHAIN;
         const int dim = nn->sp.dim;
         constexpr int64_t kBuildPairs = 50000000ll;
-        const int64_t worth = chain ? 800000000ll
-                                    : (dim <= 3 ? 30000000ll
-                                                : dim <= 5 ? 50000000ll
-                                                           : dim == 6 ? 120000000ll : dim == 7 ? 250000000ll : 400000000ll);
+        constexpr int64_t kBoxWorth[9] = {0,        30000000,  30000000,  30000000, 50000000,
+                                          50000000, 120000000, 250000000, 400000000};
+        const int64_t worth = chain ? 800000000ll : kBoxWorth[std::min(dim, 8)];
         const int64_t pairs = nq * nn->size;
         bool cells = nn->size >= (chain ? 65536 : 16384) && nn->size < (1ll << 30) && nq < (1ll << 31) &&
                      nq >= (chain ? 1024 : 64) && pairs >= worth && !(chain && prefix);
@@ -2299,8 +2299,8 @@ gbo_status gbo_nn_nearest_k(gbo_nn *nn, const double *q, int64_t nq, int64_t ld,
             if (auto st = box_cells_call(nn, lc, (const float *)nn->qfeat.p, nq, prefix, k,
                                          KnnOut{a, qv, idx, dist, (unsigned long long *)nn->fb_list.p, fb_n, ctr}))
                 return st;
-            launch_knn_exact(lc, a, nn->sp, qv, nq, k, prefix, idx, dist, (const unsigned long long *)nn->fb_list.p, fb_n,
-                             std::min<int64_t>(nq, 4096));
+            launch_knn_exact(lc, a, nn->sp, qv, nq, k, prefix, idx, dist,
+                             (const unsigned long long *)nn->fb_list.p, fb_n, std::min<int64_t>(nq, 4096));
             CHECK_LAUNCH();
             return GBO_OK;
         }

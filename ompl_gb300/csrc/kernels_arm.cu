@@ -21,11 +21,12 @@
 // them evaluating states a stride apart, and the covered prefix of the strided states counts. Small batches
 // and what is left when the queue has run empty go to arm_chunk_kernel, where many warps share an edge. The
 // undecided states are settled by the whole warp in FP64, one at a time. In the FP64 form these are all
-// states that may touch an obstacle: FP32 proves spheres free there and decides nothing else.
+// states that may touch an obstacle: FP32 proves spheres free there, by bounds on its error, and decides
+// nothing else.
 //
 // 256,000 edges of 2..2,000 states (48 checked in order, 9.6 evaluated) among 4,096 spheres: 3.20 ms for one
-// warp per edge evaluating every state, 1.16 ms; 3,001 edges among 2,048 boxes in the FP64 form: 8.4 ms with
-// every state and sphere in FP64, 0.45 ms. Bound: instruction issue of the FP32 evaluation (about 3,000
+// warp per edge evaluating every state, 1.20 ms; 3,001 edges among 2,048 boxes in the FP64 form: 6.7 to 8.4 ms
+// with every state and sphere in FP64, 0.37 to 0.43 ms. Bound: instruction issue of the FP32 evaluation (about 3,000
 // instructions per 32 states) and the longest edges' rounds. Cells: 64^3 12.1 evaluations per edge, 128^3 9.6,
 // 192^3 8.8 (not taken: 14 MB a world).
 #include <algorithm>
@@ -437,7 +438,8 @@ __global__ void __launch_bounds__(128, 5)
                 const bool gap = work && (verdict == kInvalid || j - free > before + 1);
                 const unsigned bad = __ballot_sync(0xffffffffu, gap);
                 const int stop = bad ? __ffs(bad) - 1 : 31;
-                const int64_t covered = bad ? __shfl_sync(0xffffffffu, before, stop) : __shfl_sync(0xffffffffu, reach, 31);
+                const int64_t covered =
+                    bad ? __shfl_sync(0xffffffffu, before, stop) : __shfl_sync(0xffffffffu, reach, 31);
                 if (bad && __shfl_sync(0xffffffffu, verdict, stop) == kInvalid &&
                     __shfl_sync(0xffffffffu, j, stop) == covered + 1)
                 {

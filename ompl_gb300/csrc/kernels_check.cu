@@ -295,8 +295,8 @@ __global__ void __launch_bounds__(256) motion_plain_kernel(SpaceParams sp, World
 
 template <int CK, int MAXD, int PREC>
 __global__ void __launch_bounds__(256) motion_tile_kernel(SpaceParams sp, WorldArgs wa, StatesView v1,
-                                                          StatesView v2, int64_t n, uint8_t *ok, int32_t *first_j, int32_t *nd_out,
-                                                          RunCounters *ctr)
+                                                          StatesView v2, int64_t n, uint8_t *ok, int32_t *first_j,
+                                                          int32_t *nd_out, RunCounters *ctr)
 {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ uint64_t bar;
@@ -386,8 +386,8 @@ __global__ void __launch_bounds__(256) motion_tile_kernel(SpaceParams sp, WorldA
 
 template <int CK, int MAXD, int PREC>
 __global__ void __launch_bounds__(256) motion_warp_kernel(SpaceParams sp, WorldArgs wa, StatesView v1,
-                                                          StatesView v2, int64_t n, uint8_t *ok, int32_t *first_j, int32_t *nd_out,
-                                                          RunCounters *ctr)
+                                                          StatesView v2, int64_t n, uint8_t *ok, int32_t *first_j,
+                                                          int32_t *nd_out, RunCounters *ctr)
 {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ uint64_t bar;

@@ -141,10 +141,10 @@ __device__ __forceinline__ void element_features(const NNArgs &nn, const SpacePa
 // K: list length that bounds the band (knn_keep(k)); buckets: a multiple of 32, at least 2 K.
 // nn.alive may be null: every element is present.
 template <int KIND, int MAXF, int QG, int kThreads>
-__global__ void __launch_bounds__(kThreads, QG == 4 ? (MAXF <= 8 ? 768 : 512) / kThreads : 2) knn_group_kernel(NNArgs nn, SpaceParams sp, StatesView qv, int64_t nq,
-                                                             int k, int K, int buckets, const int64_t *prefix,
-                                                             int64_t max_limit, int64_t *idx, double *dist, unsigned long long *fb_list,
-                                                             unsigned long long *fb_n, RunCounters *ctr)
+__global__ void __launch_bounds__(kThreads, QG == 4 ? (MAXF <= 8 ? 768 : 512) / kThreads : 2)
+    knn_group_kernel(NNArgs nn, SpaceParams sp, StatesView qv, int64_t nq, int k, int K, int buckets,
+                     const int64_t *prefix, int64_t max_limit, int64_t *idx, double *dist,
+                     unsigned long long *fb_list, unsigned long long *fb_n, RunCounters *ctr)
 {
     constexpr int MAXD = KIND == GBO_SPACE_KINEMATIC_CHAIN ? MAXF / 2 : MAXF;
     constexpr int kWarps = kThreads / 32;
@@ -459,8 +459,8 @@ namespace
 {
 template <int KIND, int MAXF, int QG, int kThreads>
 void launch_group_t(const LaunchCfg &lc, const NNArgs &nn, const SpaceParams &sp, StatesView qv, int64_t nq, int k,
-                    int K, int CS, const int64_t *prefix, int64_t max_limit, int64_t *idx, double *dist, unsigned long long *fb_list,
-                    unsigned long long *fb_n, RunCounters *ctr)
+                    int K, int CS, const int64_t *prefix, int64_t max_limit, int64_t *idx, double *dist,
+                    unsigned long long *fb_list, unsigned long long *fb_n, RunCounters *ctr)
 {
     const int buckets = std::min(kBuckets, (2 * K + 31) / 32 * 32);
     cudaLaunchConfig_t cfg = {};
@@ -473,8 +473,8 @@ void launch_group_t(const LaunchCfg &lc, const NNArgs &nn, const SpaceParams &sp
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, knn_group_kernel<KIND, MAXF, QG, kThreads>, nn, sp, qv, nq, k, K, buckets, prefix, max_limit, idx, dist,
-                       fb_list, fb_n, ctr);
+    cudaLaunchKernelEx(&cfg, knn_group_kernel<KIND, MAXF, QG, kThreads>, nn, sp, qv, nq, k, K, buckets, prefix,
+                       max_limit, idx, dist, fb_list, fb_n, ctr);
     note_launch();
 }
 }  // namespace
@@ -502,13 +502,13 @@ bool launch_knn_group(const LaunchCfg &lc, const NNArgs &nn, const SpaceParams &
     {                                                                                                                 \
         if (QG == 1)                                                                                                  \
             launch_group_t<KIND, MAXF, 1, 256>(lc, nn, sp, qv, nq, k, knn_keep(k), CS, prefix, max_limit, idx, dist,  \
-                                               fb_list, fb_n, ctr);                                                        \
+                                               fb_list, fb_n, ctr);                                                   \
         else if (threads == 256)                                                                                      \
             launch_group_t<KIND, MAXF, 4, 256>(lc, nn, sp, qv, nq, k, knn_keep(k), CS, prefix, max_limit, idx, dist,  \
-                                               fb_list, fb_n, ctr);                                                        \
+                                               fb_list, fb_n, ctr);                                                   \
         else                                                                                                          \
             launch_group_t<KIND, MAXF, 4, 128>(lc, nn, sp, qv, nq, k, knn_keep(k), CS, prefix, max_limit, idx, dist,  \
-                                               fb_list, fb_n, ctr);                                                        \
+                                               fb_list, fb_n, ctr);                                                   \
     } while (0)
     if (sp.kind == GBO_SPACE_KINEMATIC_CHAIN && sp.dim <= 10)
         GBO_GROUP(GBO_SPACE_KINEMATIC_CHAIN, 20);

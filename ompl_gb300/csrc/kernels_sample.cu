@@ -531,8 +531,9 @@ __global__ void __launch_bounds__(256) mt_segment_kernel(SamplerState *st, const
 // The call's values from the stored word pairs (value v = coordinate v % dim of state v / dim from pair v):
 // tempering, generate_canonical in integer arithmetic, then uniformReal (or the near bounds), lanes over
 // consecutive values. Bound by the integer pipe and the FP64 addition; with the product on the FP64 pipe it
-// was bound there (1M 10-D states: 52 us on words already tempered, now 48 with the tempering). (Tiles of 128 states turned in shared memory, for whole
-// lines written to a coordinate-major output, took 58 us: the L2 merges the sectors, the barriers cost more.)
+// was bound there (1M 10-D states: 52 us on words already tempered, now 48 with the tempering). (Tiles of 128
+// states turned in shared memory, for whole lines written to a coordinate-major output, took 58 us: the L2 merges
+// the sectors, the barriers cost more.)
 template <bool kNear>
 __global__ void __launch_bounds__(256) pairs_to_states_kernel(const uint2 *pairs, int64_t nv, SpaceParams sp,
                                                               StatesView nearv, double distance,
