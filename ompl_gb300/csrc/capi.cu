@@ -38,8 +38,11 @@ gbo_status fail(gbo_status s, const std::string &msg)
     {                                                                                                                \
         cudaError_t _e = (expr);                                                                                     \
         if (_e != cudaSuccess)                                                                                       \
+        {                                                                                                            \
+            cudaGetLastError(); /* reported here, not by the next call's launch check */                             \
             return fail(_e == cudaErrorMemoryAllocation ? GBO_ERR_OUT_OF_MEMORY : GBO_ERR_CUDA,                      \
                         std::string(#expr) + ": " + cudaGetErrorString(_e));                                         \
+        }                                                                                                            \
     } while (0)
 
 #define CHECK_LAUNCH()                                                                                               \
@@ -249,8 +252,8 @@ struct RowCall
     // before the buffers are another call's, what this one enqueued on them is done, also after an error
     ~RowCall()
     {
-        if (enqueued)
-            cudaStreamSynchronize(s);
+        if (enqueued && cudaStreamSynchronize(s) != cudaSuccess)
+            cudaGetLastError();
         std::lock_guard<std::mutex> lk(pool.mu);
         if (b)
         {

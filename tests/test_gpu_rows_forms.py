@@ -149,3 +149,17 @@ def test_large_lists_are_converted_once():
     assert np.array_equal(mv.checkMotions(Counted(a), Counted(b))["first_j"], mv.checkMotions(a, b)["first_j"])
     assert len(made) == 3
     assert np.array_equal(nn.nearestK(Counted(a), 3)[0], nn.nearestK(a, 3)[0]) and len(made) == 4
+
+
+def test_a_host_batch_in_a_capture():
+    """It is refused, since it waits for its results, and leaves no error for the calls after it."""
+    rng, ck, nn = _setup()
+    a = rng.uniform(-PI, PI, size=(4, 7))
+    want, near = ck.isValid(a), nn.nearestK(a, 3)[0]
+    for call in (lambda: ck.isValid(a), lambda: nn.nearestK(a, 3)):
+        torch.cuda.synchronize()
+        with pytest.raises(RuntimeError):
+            with torch.cuda.graph(torch.cuda.CUDAGraph()):
+                call()
+        assert np.array_equal(ck.isValid(a), want)
+        assert np.array_equal(nn.nearestK(a, 3)[0], near)
