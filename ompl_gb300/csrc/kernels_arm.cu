@@ -371,7 +371,7 @@ __global__ void __launch_bounds__(128, 5)
 }
 
 // Edges shared by many warps: a batch (tail null; first_j holds the smallest colliding state found, nd_out the segment
-// counts) or the list that arm_motion_kernel left. The states left of an edge are cut into at most `chunks` runs of
+// counts) or a list: what arm_motion_kernel left, or a batch without those outputs. The states left of an edge are cut into at most `chunks` runs of
 // kArmRun states or more; work item c * count + i is run c of edge i, so that every edge's early runs go first and the
 // later runs of an edge that has already collided before them are passed over, as are those that a short edge does not
 // have. A run's 32 lanes evaluate states a stride apart, as above. arm_finish_kernel then writes the results.
@@ -457,14 +457,23 @@ __global__ void __launch_bounds__(128, 5)
     arm_counts(ctr, evaluated, rechecks, lane);
 }
 
+// a batch that the chunk kernel checks, in the outputs or (without them) as a list
 __global__ void arm_begin_kernel(const __grid_constant__ SpaceParams sp, StatesView v1, StatesView v2, int n,
-                                 int32_t *first_j, int32_t *nd_out)
+                                 ArmTail *tail, int32_t *first_j, int32_t *nd_out, RunCounters *ctr)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n)
         return;
     double a[8], b[8];
-    nd_out[i] = arm_segments(sp, v1, v2, i, a, b);
+    const int nd = arm_segments(sp, v1, v2, i, a, b);
+    if (tail)
+    {
+        tail[i] = ArmTail{(unsigned)i, 1, INT_MAX, nd};
+        if (i == 0)
+            ctr->deferred = (unsigned)n;
+        return;
+    }
+    nd_out[i] = nd;
     first_j[i] = INT_MAX;
 }
 
@@ -492,12 +501,13 @@ static void launch_arm_motion_t(const LaunchCfg &lc, const SpaceParams &sp, cons
     // states 121 / 108 us, of 120 172 / 283 us, of 2..2,000 226 / 353 us; 6,000 of 12 states 177 / 155 us, of 120 222 /
     // 245 us; 20,000 of 120 451 / 320 us.
     constexpr int kFewEdges = 4096;
-    if (fj && nd && n <= kFewEdges)
+    if (n <= (fj && nd ? kFewEdges : kArmTailRoom))
     {
-        arm_begin_kernel<<<(int)((n + 63) / 64), 64, 0, lc.stream>>>(sp, v1, v2, (int)n, fj, nd);
+        ArmTail *list = fj && nd ? nullptr : tail;
+        arm_begin_kernel<<<(int)((n + 63) / 64), 64, 0, lc.stream>>>(sp, v1, v2, (int)n, list, fj, nd, ctr);
         const int grid = (int)std::min<int64_t>(full, (n * kArmChunks + 3) / 4);
-        arm_chunk_kernel<PREC><<<grid, 128, 0, lc.stream>>>(sp, wa, v1, v2, (int)n, kArmChunks, nullptr, fj, nd, ctr);
-        arm_finish_kernel<<<(int)((n + 127) / 128), 128, 0, lc.stream>>>((int)n, nullptr, ok, fj, nd, ctr);
+        arm_chunk_kernel<PREC><<<grid, 128, 0, lc.stream>>>(sp, wa, v1, v2, (int)n, kArmChunks, list, fj, nd, ctr);
+        arm_finish_kernel<<<(int)((n + 127) / 128), 128, 0, lc.stream>>>((int)n, list, ok, fj, nd, ctr);
     }
     else
     {
